@@ -553,124 +553,6 @@ void launch_band_solve_df(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cp
 template void launch_band_solve_df<float>(Ctx&, const BandSolveOps&, const float2*, float2*, long long, const int*,
                                           int, float4*);
 
-// ---- coarsest solve as a dense emulated-FP64 product X = A^{-1} B -------------
-// Ainv is column-major N x N in df64 (A^{-1}(i, k) at k*N + i), computed once in
-// FP64.  Thread = one row i and DCB columns; the k range is split KS ways
-// (partials in FP64, folded by k_dense_fold), so every SM has work even for a
-// few columns.  B and X are the cycle's complex FP32 columns.  Both FP32 parts
-// of each A^{-1} entry multiply b; products are summed in FP32 over blocks of
-// kDenseBlk rows and every block sum joins a double-float accumulator, so the
-// rounding error is that of a 32-term FP32 sum per block, far below the FP32
-// rounding of the result the cycle receives.
-static constexpr int DCB = 8;
-static constexpr int kDenseBlk = 32;  // rows per FP32 partial sum
-
-__global__ void __launch_bounds__(256) k_dense_df(long long N, int ncols, int kchunk, const float4* __restrict__ Ainv,
-                                                  const float2* __restrict__ b, long long ldb,
-                                                  const int* __restrict__ cols, double2* __restrict__ part) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int c0 = blockIdx.y * DCB;
-  const int ks = blockIdx.z;
-  if (i >= N) return;
-  const long long k0 = (long long)ks * kchunk, k1 = min(N, k0 + kchunk);
-  DAcc re[DCB], im[DCB];
-  const float2* bc[DCB];
-#pragma unroll
-  for (int c = 0; c < DCB; ++c) {
-    re[c].init(0.f, 0.f);
-    im[c].init(0.f, 0.f);
-    bc[c] = b + (long long)cols[min(c0 + c, ncols - 1)] * ldb;
-  }
-  // blocks of kDenseBlk rows summed in FP32 (hi and lo parts of A^-1 both
-  // applied), each block sum folded into the double-float accumulators
-  for (long long kb = k0; kb < k1; kb += kDenseBlk) {
-    const long long ke = min(k1, kb + kDenseBlk);
-    float sr[DCB], si[DCB];
-#pragma unroll
-    for (int c = 0; c < DCB; ++c) sr[c] = si[c] = 0.f;
-    for (long long k = kb; k < ke; ++k) {
-      const float4 a = Ainv[k * N + i];
-#pragma unroll
-      for (int c = 0; c < DCB; ++c) {
-        const float2 v = bc[c][k];  // same address across the warp: broadcast
-        sr[c] = __fmaf_rn(a.x, v.x, sr[c]);
-        sr[c] = __fmaf_rn(-a.y, v.y, sr[c]);
-        si[c] = __fmaf_rn(a.x, v.y, si[c]);
-        si[c] = __fmaf_rn(a.y, v.x, si[c]);
-        sr[c] = __fmaf_rn(a.z, v.x, sr[c]);
-        sr[c] = __fmaf_rn(-a.w, v.y, sr[c]);
-        si[c] = __fmaf_rn(a.z, v.y, si[c]);
-        si[c] = __fmaf_rn(a.w, v.x, si[c]);
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < DCB; ++c) {
-      re[c].add(sr[c]);
-      im[c].add(si[c]);
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < DCB; ++c)
-    if (c0 + c < ncols) part[((long long)ks * ncols + c0 + c) * N + i] = mk<double>(re[c].to_double(), im[c].to_double());
-}
-
-__global__ void __launch_bounds__(256) k_dense_fold(long long N, int ncols, int KS, const double2* __restrict__ part,
-                                                    float2* __restrict__ x, long long ldx, const int* __restrict__ cols) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int ci = blockIdx.y;
-  if (i >= N) return;
-  double ar = 0.0, ai = 0.0;
-  for (int ks = 0; ks < KS; ++ks) {
-    const double2 v = part[((long long)ks * ncols + ci) * N + i];
-    ar += v.x;
-    ai += v.y;
-  }
-  x[(long long)cols[ci] * ldx + i] = make_float2((float)ar, (float)ai);
-}
-
-int dense_df_splits(long long N, int ncols) {
-  const long long threads = N * ((ncols + DCB - 1) / DCB);
-  long long ks = (8LL * kSMs * 256 + threads - 1) / std::max(threads, 1LL);
-  return (int)std::max(1LL, std::min(ks, std::max(1LL, N / 64)));
-}
-
-void launch_dense_df(Ctx& ctx, long long N, const float4* Ainv, const float2* b, float2* x, long long ld,
-                     const int* cols, int ncols, double2* part) {
-  if (ncols <= 0) return;
-  const int KS = dense_df_splits(N, ncols);
-  const int kchunk = (int)((N + KS - 1) / KS);
-  const dim3 grid((unsigned)((N + 255) / 256), (unsigned)((ncols + DCB - 1) / DCB), (unsigned)KS);
-  const double bytes = (double)N * N * 16.0 * ((ncols + DCB - 1) / DCB) + (double)ncols * N * 16.0;
-  HZ_LAUNCH(ctx, "band_solve", bytes, k_dense_df, grid, 256, 0, N, ncols, kchunk, Ainv, b, ld, cols, part);
-  HZ_LAUNCH(ctx, "dense_fold", (double)KS * ncols * N * 16.0, k_dense_fold,
-            dim3((unsigned)((N + 255) / 256), (unsigned)ncols), 256, 0, N, ncols, KS, part, x, ld, cols);
-}
-
-// identity block (N columns) for computing the inverse with the FP64 band solve
-__global__ void k_identity(long long N, double2* __restrict__ e) {
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < N * N; q += (long long)gridDim.x * blockDim.x)
-    e[q] = mk<double>((q / N) == (q % N) ? 1.0 : 0.0, 0.0);
-}
-void launch_identity(Ctx& ctx, long long N, double2* e) {
-  const long long nb = std::min<long long>((N * N + 255) / 256, 16LL * kSMs);
-  HZ_LAUNCH(ctx, "identity", (double)N * N * 16.0, k_identity, (unsigned)nb, 256, 0, N, e);
-}
-
-// FP64 -> df64 in place (same 16 bytes per complex value)
-__global__ void k_inplace_df(long long n, double2* __restrict__ a) {
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-    const double2 v = a[q];
-    float rh, rl, ih, il;
-    split(v.x, rh, rl);
-    split(v.y, ih, il);
-    reinterpret_cast<float4*>(a)[q] = make_float4(rh, ih, rl, il);
-  }
-}
-void launch_inplace_df(Ctx& ctx, long long n, double2* a) {
-  const long long nb = std::min<long long>((n + 255) / 256, 16LL * kSMs);
-  HZ_LAUNCH(ctx, "cast", (double)n * 32.0, k_inplace_df, (unsigned)nb, 256, 0, n, a);
-}
-
 // ---- solution update x += sum_i y_i Z_i (Z complex FP32, x FP64) -----------------
 __global__ void __launch_bounds__(256, 4) k_update_x_df(long long N, const float2* __restrict__ Z, long long zstride,
                                                      long long ld, const int* __restrict__ kcol,

@@ -132,13 +132,6 @@ void launch_diag_to_df(Ctx& ctx, long long N, const double2* d, float4* out);
 void launch_update_x_df(Ctx& ctx, long long N, const float2* Z, long long zstride, long long ld, const int* kcol,
                         const double2* y, int ystride, double2* x, long long xld, const int* cols, int ncols,
                         long long zcols);
-// Coarsest solve as a dense emulated-FP64 product x = Ainv b (Ainv column-major
-// df64); part holds dense_df_splits(N, ncols) * ncols * N FP64 values.
-int dense_df_splits(long long N, int ncols);
-void launch_dense_df(Ctx& ctx, long long N, const float4* Ainv, const float2* b, float2* x, long long ld,
-                     const int* cols, int ncols, double2* part);
-void launch_identity(Ctx& ctx, long long N, double2* e);
-void launch_inplace_df(Ctx& ctx, long long n, double2* a);
 // Coarsest solve with the block operators stored as df64 (op.T / op.G point to
 // float4 arrays); work holds 3 * ncols * N df64 values.
 template <typename T>

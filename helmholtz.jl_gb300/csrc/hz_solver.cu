@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "../../include/helmgpu.h"
+#include "hz_coarse.h"
 #include "hz_host.h"
 #include "hz_kernels.cuh"
 #include "hz_learn.h"
@@ -127,8 +128,9 @@ struct Hierarchy {
   DBuf bandT, bandG, bandB, bandwork;
   BandSolveOps band;
   bool band_df = false;   // block operators stored as df64
-  bool dense_df = false;  // coarsest solve as a dense df64 product with A^{-1}
-  DBuf dense;             // A^{-1} (column-major, df64)
+  bool dense = false;     // coarsest solve as a product with A^{-1} (digit form)
+  CoarseOp coarse;
+  DBuf cimage, cscale;
 };
 
 }  // namespace
@@ -324,27 +326,14 @@ std::vector<double> restrict_nodal(const std::vector<double>& f, const Grid& gf,
   return c;
 }
 
-// Largest coarsest level solved through a dense inverse in the emulated mode
-// (A^{-1} takes N^2 x 16 bytes: 1 GiB at this size).
-static constexpr long long kDenseCoarseMax = 8192;
-
 // ---- hierarchy setup -------------------------------------------------------
 
-// Stencil offsets per level are all within one node; the banded storage uses
-// kl = ku = nx*ny + nx + 1 (3D) or nx + 1 (2D).
-// Banded LU of one level's operator (host, FP64) and the dense block operators
-// of its blocked solve.
-void band_factor_level(hz_handle* h, const Hierarchy& H, const Level& L, std::vector<BandBlock>& blocks,
-                       std::vector<std::complex<double>>& T, std::vector<std::complex<double>>& G, int& kl_out,
-                       int& ku_out) {
+// Stencil coefficients of a level in FP64 on the host, coef[s * N + p] = A(p, p + offset_s).
+std::vector<std::complex<double>> level_coefficients(hz_handle* h, const Hierarchy& H, const Level& L) {
   const Grid g = L.g;
   const int dim = h->prob.dim;
   const long long N = g.N;
-  const int bw = dim == 3 ? g.nx * g.ny + g.nx + 1 : g.nx + 1;
-  const int kl = bw, ku = bw;
-  const long long ldab = 2LL * kl + ku + 1;
   const int ns = dim == 3 ? 27 : 9;
-  // gather the stencil coefficients of the coarsest level on the host
   std::vector<std::complex<double>> coef((size_t)ns * N, 0.0);
   if (L.fine) {
     // 5/7-point coarsest level (single-level hierarchy or re-discretised levels)
@@ -375,6 +364,24 @@ void band_factor_level(hz_handle* h, const Hierarchy& H, const Level& L, std::ve
   } else {
     ck(cudaMemcpy(coef.data(), L.coef64.p, (size_t)ns * N * 16, cudaMemcpyDeviceToHost), "copy coarse coef");
   }
+  return coef;
+}
+
+// Stencil offsets per level are all within one node; the banded storage uses
+// kl = ku = nx*ny + nx + 1 (3D) or nx + 1 (2D).
+// Banded LU of one level's operator (host, FP64) and the dense block operators
+// of its blocked solve.
+void band_factor_level(hz_handle* h, const Hierarchy& H, const Level& L, std::vector<BandBlock>& blocks,
+                       std::vector<std::complex<double>>& T, std::vector<std::complex<double>>& G, int& kl_out,
+                       int& ku_out) {
+  const Grid g = L.g;
+  const int dim = h->prob.dim;
+  const long long N = g.N;
+  const int bw = dim == 3 ? g.nx * g.ny + g.nx + 1 : g.nx + 1;
+  const int kl = bw, ku = bw;
+  const long long ldab = 2LL * kl + ku + 1;
+  const int ns = dim == 3 ? 27 : 9;
+  const std::vector<std::complex<double>> coef = level_coefficients(h, H, L);
   std::vector<std::complex<double>> ab((size_t)(ldab * N), 0.0);
   const int kv = kl + ku;
   for (long long p = 0; p < N; ++p) {
@@ -399,50 +406,99 @@ void band_factor_level(hz_handle* h, const Hierarchy& H, const Level& L, std::ve
   ku_out = ku;
 }
 
+// The coarsest operator's inverse in digit form (hz_coarse.cu), or false where
+// the level is too large, the memory does not suffice, or the inverse fails its
+// check (A x = b for two random columns, on the host): the slab elimination
+// pivots within a slab only, the band LU across them.
+bool invert_coarsest(hz_handle* h, Hierarchy& H) {
+  Level& L = *H.lv.back();
+  const long long N = L.g.N;
+  const bool fp64 = h->opt.precision != HZ_PREC_MIXED;
+  // BiCGSTAB's short recurrences carry a rounding difference of the cycle into the
+  // iteration count (103 against 112 iterations for one source of a 257 x 129 grid),
+  // where FGMRES contracts it: its native-FP64 cycles keep the band substitution
+  if (h->opt.krylov == HZ_KRYLOV_BICGSTAB && h->opt.outer_arith != HZ_OUTER_EMULATED) return false;
+  if (!coarse_supported(L.g)) return false;
+  CoarseOp& op = H.coarse;
+  op.N = N;
+  op.slices = fp64 ? 8 : 6;
+  const std::vector<std::complex<double>> coef = level_coefficients(h, H, L);
+  cudaStream_t st = h->ctx.stream;
+  try {
+    DBuf scratch, dcoef, bad, vb, vx, vw, vc;
+    H.cimage.alloc(op.image_bytes());
+    H.cscale.alloc((size_t)N * sizeof(int));
+    op.image = H.cimage.p;
+    op.rscale = H.cscale.as<int>();
+    const double2* dc = L.coef64.as<double2>();
+    if (L.fine) {
+      dcoef.alloc(coef.size() * 16);
+      ck(cudaMemcpyAsync(dcoef.p, coef.data(), coef.size() * 16, cudaMemcpyHostToDevice, st), "upload coarse coef");
+      dc = dcoef.as<double2>();
+    }
+    scratch.alloc(coarse_setup_bytes(L.g));
+    bad.alloc(sizeof(int));
+    ck(cudaMemsetAsync(bad.p, 0, sizeof(int), st), "clear pivot flag");
+    ck(cudaMemsetAsync(H.cimage.p, 0, op.image_bytes(), st), "clear coarse image");
+    launch_coarse_setup(h->ctx, L.g, h->prob.dim == 3, dc, op, scratch.as<double2>(), bad.as<int>());
+    const int nv = 2, cols[2] = {0, 1};
+    std::vector<std::complex<double>> b((size_t)nv * N), x((size_t)nv * N);
+    uint64_t s = 0x9e3779b97f4a7c15ull;
+    auto rnd = [&] {
+      s = s * 6364136223846793005ull + 1442695040888963407ull;
+      return (double)(int64_t)s * 0x1p-63;
+    };
+    for (auto& z : b) {
+      const double re = rnd();
+      z = {re, rnd()};
+    }
+    vb.alloc(b.size() * 16);
+    vx.alloc(b.size() * 16);
+    vw.alloc(op.work_bytes(nv));
+    vc.alloc(sizeof(cols));
+    ck(cudaMemcpyAsync(vb.p, b.data(), b.size() * 16, cudaMemcpyHostToDevice, st), "upload check columns");
+    ck(cudaMemcpyAsync(vc.p, cols, sizeof(cols), cudaMemcpyHostToDevice, st), "upload check columns");
+    launch_coarse<double>(h->ctx, op, vb.as<double2>(), vx.as<double2>(), N, vc.as<int>(), nv, vw.p);
+    int nbad = 0;
+    ck(cudaMemcpyAsync(x.data(), vx.p, b.size() * 16, cudaMemcpyDeviceToHost, st), "check columns");
+    ck(cudaMemcpyAsync(&nbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, st), "pivot flag");
+    sync(h);
+    double rr = 0.0, bb = 0.0;
+    const Grid g = L.g;
+    const int ns = h->prob.dim == 3 ? 27 : 9;
+    for (int c = 0; c < nv; ++c)
+      for (long long p = 0; p < N; ++p) {
+        const int i = (int)(p % g.nx), j = (int)((p / g.nx) % g.ny), k = (int)(p / ((long long)g.nx * g.ny));
+        std::complex<double> r = b[(size_t)c * N + p];
+        bb += std::norm(r);
+        for (int t = 0; t < ns; ++t) {
+          const int ii = i + t % 3 - 1, jj = j + (t / 3) % 3 - 1, kk = ns == 27 ? k + t / 9 - 1 : k;
+          if (ii < 0 || ii >= g.nx || jj < 0 || jj >= g.ny || kk < 0 || kk >= g.nz) continue;
+          r -= coef[(size_t)t * N + p] * x[(size_t)c * N + ii + (long long)g.nx * (jj + (long long)g.ny * kk)];
+        }
+        rr += std::norm(r);
+      }
+    if (nbad == 0 && rr <= bb * (fp64 ? 1e-20 : 1e-18)) return true;
+  } catch (const HzError& e) {
+    if (e.code != HZ_ERR_ALLOC) throw;
+  }
+  H.cimage.reset();
+  H.cscale.reset();
+  return false;
+}
+
 void factor_coarsest(hz_handle* h, Hierarchy& H) {
   Level& L = *H.lv.back();
   const long long N = L.g.N;
+  H.nc = N;
+  H.dense = invert_coarsest(h, H);
+  if (H.dense) return;
   int kl = 0, ku = 0;
   std::vector<std::complex<double>> T, G;
   band_factor_level(h, H, L, H.band.blocks, T, G, kl, ku);
-  H.nc = N;
   H.kl = kl;
   H.ku = ku;
   H.band_df = h->opt.precision == HZ_PREC_MIXED && h->opt.outer_arith == HZ_OUTER_EMULATED;
-  H.dense_df = H.band_df && N <= kDenseCoarseMax;
-  if (H.dense_df) {
-    // emulated-FP64 cycles on a small coarsest level: compute A^{-1} once in FP64
-    // (the blocked band solve applied to the identity), store it as df64 and
-    // apply it as one dense product per cycle
-    DBuf dT, dG, dB, E, W, dc;
-    dT.alloc(T.size() * 16);
-    dG.alloc(G.size() * 16);
-    ck(cudaMemcpy(dT.p, T.data(), T.size() * 16, cudaMemcpyHostToDevice), "upload band forward operators");
-    ck(cudaMemcpy(dG.p, G.data(), G.size() * 16, cudaMemcpyHostToDevice), "upload band backward operators");
-    dB.alloc(H.band.blocks.size() * sizeof(BandBlock));
-    ck(cudaMemcpy(dB.p, H.band.blocks.data(), H.band.blocks.size() * sizeof(BandBlock), cudaMemcpyHostToDevice),
-       "upload band blocks");
-    BandSolveOps ops;
-    ops.N = N;
-    ops.blocks = H.band.blocks;
-    ops.dblocks = dB.as<BandBlock>();
-    ops.T = dT.as<double2>();
-    ops.G = dG.as<double2>();
-    std::vector<int> all((size_t)N);
-    for (long long c = 0; c < N; ++c) all[(size_t)c] = (int)c;
-    dc.alloc((size_t)N * sizeof(int));
-    ck(cudaMemcpy(dc.p, all.data(), (size_t)N * sizeof(int), cudaMemcpyHostToDevice), "upload identity columns");
-    E.alloc((size_t)N * N * 16);
-    W.alloc((size_t)3 * N * N * 16);
-    H.dense.alloc((size_t)N * N * 16);
-    launch_identity(h->ctx, N, E.as<double2>());
-    launch_band_solve<double>(h->ctx, ops, E.as<double2>(), H.dense.as<double2>(), N, dc.as<int>(), (int)N,
-                              W.as<double2>());
-    launch_inplace_df(h->ctx, N * N, H.dense.as<double2>());
-    sync(h);
-    H.band.N = N;
-    return;
-  }
   if (H.band_df) {
     // emulated-FP64 solves: each FP64 entry stored as a (hi, lo) float pair
     auto to_df = [](std::vector<std::complex<double>>& v) {
@@ -656,12 +712,8 @@ void ensure_level_buffers(hz_handle* h, Hierarchy& H, int R) {
       L.gp.alloc((size_t)R * 3 * kcycle_nblk(L.g.N) * 16);
     }
   }
-  // band work: 3 vectors per column; the dense product's split-K partials need
-  // splits(ncols) * ncols vectors, largest over the active column counts
-  long long wcols = 3LL * R;
-  if (H.dense_df)
-    for (int nc = 1; nc <= R; ++nc) wcols = std::max(wcols, (long long)dense_df_splits(H.nc, nc) * nc);
-  H.bandwork.alloc((size_t)wcols * H.nc * 16);
+  // digits of the right-hand sides, or 3 vectors per column of the band solve
+  H.bandwork.alloc(H.dense ? H.coarse.work_bytes(R) : (size_t)3 * R * H.nc * 16);
 }
 
 // ---- multigrid cycle -----------------------------------------------------------
@@ -880,9 +932,8 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
   if (h->cap_on && l == h->cap_level) capture_rhs<TB>(h, L, b, cols, nc);
   if (l == last) {
     if (!std::is_same<T, TB>::value) fail(HZ_ERR_STATE, "single-level mixed hierarchy is not supported");
-    if (H.dense_df)
-      launch_dense_df(h->ctx, H.nc, H.dense.as<float4>(), (const float2*)b, (float2*)out, L.ld, cols, nc,
-                      H.bandwork.as<double2>());
+    if (H.dense)
+      launch_coarse<T>(h->ctx, H.coarse, (const cplx<T>*)b, out, L.ld, cols, nc, H.bandwork.p);
     else if (H.band_df)
       launch_band_solve_df<float>(h->ctx, H.band, (const float2*)b, (float2*)out, L.ld, cols, nc,
                                   H.bandwork.as<float4>());
@@ -1937,8 +1988,9 @@ int hz_clear(hz_handle* h) {
       H.bandT.reset();
       H.bandG.reset();
       H.bandB.reset();
-      H.dense.reset();
-      H.dense_df = false;
+      H.cimage.reset();
+      H.cscale.reset();
+      H.dense = false;
       H.band_df = false;
       H.bandwork.reset();
       H.band = BandSolveOps();

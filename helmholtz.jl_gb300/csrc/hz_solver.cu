@@ -1475,6 +1475,10 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
   return std::min(outer, std::max(1, h->opt.max_outer));
 }
 
+// Graph keys of BiCGSTAB's two preconditioner applications (FGMRES uses its basis
+// index, below the restart limit of 64); the handle runs one Krylov method.
+static constexpr int kBicgKey = 64;
+
 // Right-preconditioned BiCGSTAB on H (or H^H), one multigrid cycle per
 // preconditioner application (solveBiCGSTAB_MG, src/ShiftedLaplacianMultigridSolver.jl:91-93).
 // Returns the iterations of the slowest column.
@@ -1552,7 +1556,7 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
     if (it == maxit) break;
     launch_bicg_scalars(h->ctx, 0, dc, na, red, HS, sc);
     launch_bicg_vec(h->ctx, 0, N, r, p, v, nullptr, sc, dc, na);
-    precondition(h, H, p, ph, dc, na);
+    cycle_graph(h, adj, kBicgKey, na, mixed ? 1 : 0, [&] { precondition(h, H, p, ph, dc, na); });
     if (emu)
       launch_fine_df64<double2>(h->ctx, fopa, h->diagHdf.as<float4>(), (const float2*)ph, v, N, dc, na);
     else if (mixed)
@@ -1563,7 +1567,7 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
     launch_reduce(h->ctx, part, dc, na, 1, nblk, red, HS, 0);
     launch_bicg_scalars(h->ctx, 1, dc, na, red, HS, sc);
     launch_bicg_vec(h->ctx, 1, N, r, nullptr, v, sv, sc, dc, na);
-    precondition(h, H, sv, sh, dc, na);
+    cycle_graph(h, adj, kBicgKey + 1, na, mixed ? 1 : 0, [&] { precondition(h, H, sv, sh, dc, na); });
     if (emu)
       launch_fine_df64<double2>(h->ctx, fopa, h->diagHdf.as<float4>(), (const float2*)sh, t, N, dc, na);
     else if (mixed)

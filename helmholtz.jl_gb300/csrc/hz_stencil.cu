@@ -692,6 +692,141 @@ __global__ void __launch_bounds__(256) k_band_coop(long long N, int nbk, const B
   }
 }
 
+// The same block steps, one cluster of CTAs per column: the columns are
+// independent, so a step ends with a cluster barrier instead of a grid barrier.
+// Every CTA holds the column's vectors in its shared memory; a row's result is
+// written into all of them.  The entries of the next step's operator row are
+// loaded before the barrier.  A warp-wide FP64 instruction occupies its quarter of
+// the SM for 64 clocks, so rows go to the CTAs in turn (one row per quarter up to
+// four rows per CTA), the real and imaginary sums share the reduction's
+// instructions, and stretches of 32 zero entries are skipped.  Every row sum is
+// k_band_coop's, in its order: the results are equal bit for bit.
+static constexpr int kBandWarps = 8;
+
+template <int PF, typename V>
+__device__ __forceinline__ double2 band_row_sum(const double2* Mr, int W, int lane, const double2 (&m)[PF], bool pre,
+                                                V&& value) {
+  double ar = 0.0, ai = 0.0;
+  auto add = [&](double2 a, int k) {
+    if (__any_sync(0xffffffffu, a.x != 0.0 || a.y != 0.0)) {
+      const double2 v = k < W ? value(k) : mk<double>(0, 0);
+      ar = fma(a.x, v.x, ar);
+      ar = fma(-a.y, v.y, ar);
+      ai = fma(a.x, v.y, ai);
+      ai = fma(a.y, v.x, ai);
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < PF; ++q)
+    if (32 * q < W) add(pre ? m[q] : (lane + 32 * q < W ? Mr[lane + 32 * q] : mk<double>(0, 0)), lane + 32 * q);
+  for (int k = lane + 32 * PF; k - lane < W; k += 32) add(k < W ? Mr[k] : mk<double>(0, 0), k);
+  // lanes 0-15 reduce the real sums, lanes 16-31 the imaginary ones, each in the
+  // tree of a full exchange
+  const bool lower = lane < 16;
+  double s = (lower ? ar : ai) + __shfl_xor_sync(0xffffffffu, lower ? ai : ar, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return mk<double>(__shfl_sync(0xffffffffu, s, 0), __shfl_sync(0xffffffffu, s, 16));
+}
+
+template <int PF>
+__device__ __forceinline__ void band_row_prefetch(const double2* Mr, int W, int lane, double2 (&m)[PF]) {
+#pragma unroll
+  for (int q = 0; q < PF; ++q) m[q] = lane + 32 * q < W ? Mr[lane + 32 * q] : mk<double>(0, 0);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(32 * kBandWarps) k_band_cluster(int N, int nbk, const BandBlock* __restrict__ blocks,
+                                                                  const double2* __restrict__ Tops,
+                                                                  const double2* __restrict__ Gops,
+                                                                  const cplx<T>* b, long long ldb,
+                                                                  const int* __restrict__ cols, cplx<T>* x,
+                                                                  long long ldx) {
+  extern __shared__ __align__(16) double2 band_sm[];
+  double2* const bx = band_sm;  // b, then x from the back
+  double2* const Y0 = band_sm + N;
+  double2* const Y1 = band_sm + 2 * N;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int lane = threadIdx.x & 31;
+  const int ctas = (int)cluster.num_blocks();
+  const int gw = (threadIdx.x >> 5) * ctas + (int)cluster.block_rank(), nw = ctas * kBandWarps;
+  constexpr int PF = 4;
+  const int col = cols[blockIdx.x / ctas];
+  const cplx<T>* bc = b + (long long)col * ldb;
+  cplx<T>* xc = x + (long long)col * ldx;
+  for (int k = threadIdx.x; k < N; k += 32 * kBandWarps) {
+    const cplx<T> v = bc[k];
+    bx[k] = mk<double>((double)v.x, (double)v.y);
+  }
+  double2 m[PF];
+  BandBlock B = blocks[0];
+  if (gw < B.W) band_row_prefetch<PF>(Tops + B.toff + (long long)gw * B.W, B.W, lane, m);
+  cluster.sync();
+  long long prev_end = 0;
+  for (int I = 0; I < nbk; ++I) {
+    const int split = (I == 0) ? 0 : (int)(prev_end - B.s);
+    const double2* src0 = ((I & 1) ? Y0 : Y1) + B.s;  // output of block I-1
+    const double2* srcb = bx + B.s;
+    double2* dst = ((I & 1) ? Y1 : Y0) + B.s;
+    for (int i = gw; i < B.W; i += nw) {
+      const double2 r = band_row_sum<PF>(Tops + B.toff + (long long)i * B.W, B.W, lane, m, i == gw,
+                                         [&](int k) { return k < split ? src0[k] : srcb[k]; });
+      if (lane < ctas) cluster.map_shared_rank(dst, lane)[i] = r;
+    }
+    prev_end = B.s + B.W;
+    if (I + 1 < nbk) {
+      B = blocks[I + 1];
+      if (gw < B.W) band_row_prefetch<PF>(Tops + B.toff + (long long)gw * B.W, B.W, lane, m);
+    } else if (gw < B.nb) {
+      band_row_prefetch<PF>(Gops + B.goff + (long long)gw * B.Wb, B.Wb, lane, m);
+    }
+    cluster.sync();
+  }
+  for (int I = nbk - 1; I >= 0; --I) {
+    const double2* yb = ((I & 1) ? Y1 : Y0) + B.s;
+    double2* xb = bx + B.s;
+    for (int i = gw; i < B.nb; i += nw) {
+      const double2 r = band_row_sum<PF>(Gops + B.goff + (long long)i * B.Wb, B.Wb, lane, m, i == gw,
+                                         [&](int k) { return k < B.nb ? yb[k] : xb[k]; });
+      if (lane < ctas) cluster.map_shared_rank(xb, lane)[i] = r;
+      if (lane == 0) xc[B.s + i] = mk<T>((T)r.x, (T)r.y);
+    }
+    if (I > 0) {
+      B = blocks[I - 1];
+      if (gw < B.nb) band_row_prefetch<PF>(Gops + B.goff + (long long)gw * B.Wb, B.Wb, lane, m);
+    }
+    cluster.sync();
+  }
+}
+
+// Clusters of 16 CTAs (8 where the GPU takes no larger ones) with the given shared
+// memory that can be resident at once, per device; 0: not available.
+template <typename T>
+void band_cluster_shape(cudaStream_t st, size_t smem, int& ctas, int& resident) {
+  for (ctas = 16; ctas >= 8; ctas /= 2) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(32 * kBandWarps);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    resident = 0;
+    if (cudaFuncSetAttribute(k_band_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
+            cudaSuccess &&
+        (ctas <= 8 || cudaFuncSetAttribute(k_band_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                          cudaSuccess) &&
+        cudaOccupancyMaxActiveClusters(&resident, k_band_cluster<T>, &cfg) == cudaSuccess && resident > 0)
+      return;
+    cudaGetLastError();
+  }
+  ctas = resident = 0;
+}
+
 template <typename T>
 void launch_band_solve(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cplx<T>* x, long long ld, const int* cols,
                        int ncols, double2* work) {
@@ -713,12 +848,49 @@ void launch_band_solve(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cplx<
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       capacity[dev] = std::max(1, std::min(per_sm, 4)) * std::max(1, sms);
     }
-    const int grid = (dev >= 0 && dev < kMaxDevices) ? capacity[dev] : kSMs;
+    // Clocks of both schedules: a cluster per column (as many at once as fit) and a
+    // cluster barrier per step, or the columns over the whole GPU and a grid barrier
+    // over as many CTAs as the widest step fills; two FP64 FMA lanes per SM and clock.
+    const size_t smem = (size_t)N * 3 * sizeof(double2);
+    int ctas = 0, resident = 0;
+    if (smem <= 220 * 1024) band_cluster_shape<T>(ctx.stream, smem, ctas, resident);
+    double cl = 0.0, gr = 0.0;
+    long long rows = 1;
+    for (const BandBlock& B : op.blocks) {
+      const double fma = 4.0 * ((double)B.W * B.W + (double)B.nb * B.Wb);
+      if (resident) cl += (ncols + resident - 1) / resident * (fma / (2.0 * ctas) + 2 * 2000.0);
+      gr += fma * ncols / (2.0 * kSMs) + 2 * 6000.0;
+      rows = std::max(rows, (long long)B.W);
+    }
+    const bool clustered = resident && cl < gr;
+    const int full = (dev >= 0 && dev < kMaxDevices) ? capacity[dev] : kSMs;
+    const int grid = (int)std::min<long long>(full, (rows * ncols + 7) / 8);
     static thread_local int id = -1;
     if (id < 0 || (size_t)id >= ctx.names.size() || ctx.names[id] != "band_solve") id = ctx.name_id("band_solve");
     cudaEvent_t ev = nullptr;
     ctx.before(id, &ev);
     const BandBlock* blk = op.dblocks;
+    if (clustered) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)(ctas * ncols));
+      cfg.blockDim = dim3(32 * kBandWarps);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = ctx.stream;
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = (unsigned)ctas;
+      at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      const cudaError_t e = cudaLaunchKernelEx(&cfg, k_band_cluster<T>, (int)N, nbk, blk, op.T, op.G, b, ld, cols, x,
+                                               ld);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        throw std::runtime_error(std::string("band_solve cluster launch failed: ") + cudaGetErrorString(e));
+      }
+      ctx.after(id, ev, bytes);
+      return;
+    }
     const double2* Tp = op.T;
     const double2* Gp = op.G;
     long long ldb = ld, ldx = ld;

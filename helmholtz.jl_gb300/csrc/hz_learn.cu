@@ -251,107 +251,6 @@ __global__ void k_wflip(int Cout, int Cin, int K, const bf16* __restrict__ w, bf
   wt[idx] = (co < Cout) ? w[((long long)co * 9 + (8 - t)) * Cin + ci] : __float2bfloat16_rn(0.f);
 }
 
-// Weight gradient on the tensor cores: dw[co][t][ci] += sum_n dout[n][co] * in[n + off_t][ci],
-// a GEMM with M = Cout, N = Cin and K = the nodes.  One CTA (4 warps) owns one
-// tap t (blockIdx.z) and a range of kc nodes (blockIdx.y); it stages KS-node
-// slices of the input rows (zeroed where the tap leaves the grid, so the
-// zero padding is exact) and of the output-gradient rows in shared memory,
-// runs m16n8k16 MMAs over 16-node K-steps (warp w owns the 16x8 output tiles
-// w, w+4, ...), and adds its partial sums to dw with one atomic per weight.
-// Row strides in shared memory are padded by 8 bf16 so the four node rows a
-// fragment load touches fall in different banks.
-constexpr int kWgKS = 64;        // nodes per staged slice
-constexpr int kWgMaxTiles = 16;  // 16x8 tiles per warp (Cout <= 64, Cin <= 128)
-
-__device__ __forceinline__ unsigned pack2(bf16 lo, bf16 hi) {
-  return (unsigned)__bfloat16_as_ushort(lo) | ((unsigned)__bfloat16_as_ushort(hi) << 16);
-}
-
-__global__ void __launch_bounds__(128) k_wgrad_mma(int nx, int ny, int total, int Cin, int Cout,
-                                                   const bf16* __restrict__ in, int ldi, const bf16* __restrict__ dout,
-                                                   int ldd, int d_off, float* __restrict__ dw, int kc) {
-  extern __shared__ __align__(16) unsigned char wg_smem[];
-  const int N = nx * ny;
-  const int t = blockIdx.z;
-  const int dx = t % 3 - 1, dy = t / 3 - 1;
-  const int C16 = (Cout + 15) / 16 * 16;
-  const int sIn = Cin + 8, sD = C16 + 8;
-  bf16* s_in = reinterpret_cast<bf16*>(wg_smem);
-  bf16* s_d = s_in + kWgKS * sIn;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, tq = lane & 3;
-  const int NTn = Cin / 8, T = (C16 / 16) * NTn;
-  float acc[kWgMaxTiles][4];
-#pragma unroll
-  for (int k = 0; k < kWgMaxTiles; ++k) acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.f;
-  const int q0 = blockIdx.y * kc;
-  const int q1 = min(total, q0 + kc);
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  for (int qs = q0; qs < q1; qs += kWgKS) {
-    __syncthreads();
-    const int cin8 = Cin / 8, cd8 = C16 / 8;
-    for (int e = threadIdx.x; e < kWgKS * cin8; e += blockDim.x) {
-      const int r = e / cin8, c8 = e % cin8;
-      const int q = qs + r;
-      uint4 v = zero;
-      if (q < q1) {
-        const int p = q % N;
-        const int i = p % nx + dx, j = p / nx + dy;
-        if (i >= 0 && i < nx && j >= 0 && j < ny)
-          v = *reinterpret_cast<const uint4*>(in + (long long)(q + dx + dy * nx) * ldi + c8 * 8);
-      }
-      *reinterpret_cast<uint4*>(s_in + r * sIn + c8 * 8) = v;
-    }
-    for (int e = threadIdx.x; e < kWgKS * cd8; e += blockDim.x) {
-      const int r = e / cd8, c8 = e % cd8;
-      const int q = qs + r;
-      uint4 v = zero;
-      if (q < q1 && c8 * 8 < Cout) v = *reinterpret_cast<const uint4*>(dout + (long long)q * ldd + d_off + c8 * 8);
-      *reinterpret_cast<uint4*>(s_d + r * sD + c8 * 8) = v;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int kb = 0; kb < kWgKS; kb += 16) {
-      const bf16* d0 = s_d + (kb + tq * 2) * sD;
-      const bf16* i0 = s_in + (kb + tq * 2) * sIn;
-#pragma unroll
-      for (int k = 0; k < kWgMaxTiles; ++k) {
-        const int tile = warp + 4 * k;
-        if (tile < T) {
-          const int co = (tile / NTn) * 16 + g;
-          const int ci = (tile % NTn) * 8 + g;
-          const unsigned a0 = pack2(d0[co], d0[sD + co]);
-          const unsigned a1 = pack2(d0[co + 8], d0[sD + co + 8]);
-          const unsigned a2 = pack2(d0[8 * sD + co], d0[9 * sD + co]);
-          const unsigned a3 = pack2(d0[8 * sD + co + 8], d0[9 * sD + co + 8]);
-          const unsigned b0 = pack2(i0[ci], i0[sIn + ci]);
-          const unsigned b1 = pack2(i0[8 * sIn + ci], i0[9 * sIn + ci]);
-          asm volatile(
-              "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-              "{%0,%1,%2,%3};\n"
-              : "+f"(acc[k][0]), "+f"(acc[k][1]), "+f"(acc[k][2]), "+f"(acc[k][3])
-              : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kWgMaxTiles; ++k) {
-    const int tile = warp + 4 * k;
-    if (tile >= T) break;
-    const int co = (tile / NTn) * 16 + g;
-    const int ci = (tile % NTn) * 8 + tq * 2;
-    if (co < Cout) {
-      atomicAdd(&dw[((long long)co * 9 + t) * Cin + ci], acc[k][0]);
-      atomicAdd(&dw[((long long)co * 9 + t) * Cin + ci + 1], acc[k][1]);
-    }
-    if (co + 8 < Cout) {
-      atomicAdd(&dw[((long long)(co + 8) * 9 + t) * Cin + ci], acc[k][2]);
-      atomicAdd(&dw[((long long)(co + 8) * 9 + t) * Cin + ci + 1], acc[k][3]);
-    }
-  }
-}
-
 // Per-channel resampling between grid levels (NHWC bf16, FP32 arithmetic).
 // mode 0, restriction (fine -> coarse): full weighting with weights 1, 1/2 per
 // axis, normalised by the weights that fall inside the grid.
@@ -494,45 +393,83 @@ __global__ void k_pack_in(long long BN, const float4* __restrict__ x4, bf16* __r
 
 // loss_b = ||y_b - t_b||^2 / ||t_b||^2 (channels 0, 1 of y) accumulated as the
 // batch mean into *loss, and the output gradient dy = 2 (y - t) / ||t_b||^2 / B
-// as bf16 into 16-channel rows (channels 2..15 zero).
-__global__ void __launch_bounds__(256) k_loss(int N, int B, const float* __restrict__ y, const float* __restrict__ t,
-                                              bf16* __restrict__ dy, double* __restrict__ loss) {
-  const int b = blockIdx.x;
-  __shared__ double sh_e[256], sh_t[256];
+// as bf16 into 16-channel rows (channels 2..15 zero).  Two passes of
+// gridDim.y CTAs per sample: the sums of each CTA's nodes into part, then every CTA
+// folds its sample's sums in the same order and writes its nodes.  The FP64 steps
+// (18 per node) bound one CTA per sample: 112 us at 129^2 x 32 and 229 us at 33^3 x
+// 8, now 37 and 29 us.
+__device__ __forceinline__ void loss_diff(const float* y, const float* t, long long r, int c, double& d, double& tv) {
+  tv = widen_f32(t[r * 2 + c]);
+  d = widen_f32(y[r * 8 + c]) - tv;
+}
+
+__global__ void __launch_bounds__(256) k_loss_sums(int N, const float* __restrict__ y, const float* __restrict__ t,
+                                                   double* __restrict__ part) {
+  __shared__ double sh[2][8];
   double e = 0.0, tt = 0.0;
-  for (int p = threadIdx.x; p < N; p += blockDim.x) {
-    const long long r = (long long)b * N + p;
+  for (int p = blockIdx.y * 256 + threadIdx.x; p < N; p += gridDim.y * 256) {
+    const long long r = (long long)blockIdx.x * N + p;
+#pragma unroll
     for (int c = 0; c < 2; ++c) {
-      const double tv = t[r * 2 + c];
-      const double d = (double)y[r * 8 + c] - tv;
-      e += d * d;
-      tt += tv * tv;
+      double d, tv;
+      loss_diff(y, t, r, c, d, tv);
+      e = fma(d, d, e);
+      tt = fma(tv, tv, tt);
     }
   }
-  sh_e[threadIdx.x] = e;
-  sh_t[threadIdx.x] = tt;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    e += __shfl_xor_sync(0xffffffffu, e, o);
+    tt += __shfl_xor_sync(0xffffffffu, tt, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sh[0][threadIdx.x >> 5] = e;
+    sh[1][threadIdx.x >> 5] = tt;
+  }
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      sh_e[threadIdx.x] += sh_e[threadIdx.x + s];
-      sh_t[threadIdx.x] += sh_t[threadIdx.x + s];
-    }
-    __syncthreads();
+  if (threadIdx.x < 2) {
+    double v = 0.0;
+    for (int w = 0; w < 8; ++w) v += sh[threadIdx.x][w];
+    part[((long long)blockIdx.x * gridDim.y + blockIdx.y) * 2 + threadIdx.x] = v;
   }
-  const double tn = sh_t[0] > 0.0 ? sh_t[0] : 1.0;
-  if (threadIdx.x == 0) atomicAdd(loss, sh_e[0] / tn / B);
+}
+
+__global__ void __launch_bounds__(256) k_loss_grad(int N, int B, const float* __restrict__ y,
+                                                   const float* __restrict__ t, const double* __restrict__ part,
+                                                   bf16* __restrict__ dy, double* __restrict__ loss) {
+  __shared__ double tot[2];
+  if (threadIdx.x < 2) {
+    double v = 0.0;
+    for (int k = 0; k < (int)gridDim.y; ++k)
+      v += part[((long long)blockIdx.x * gridDim.y + k) * 2 + threadIdx.x];
+    tot[threadIdx.x] = v;
+  }
+  __syncthreads();
+  const double tn = tot[1] > 0.0 ? tot[1] : 1.0;
+  if (threadIdx.x == 0 && blockIdx.y == 0) atomicAdd(loss, tot[0] / tn / B);
   const double sc = 2.0 / tn / B;
-  for (int p = threadIdx.x; p < N; p += blockDim.x) {
-    const long long r = (long long)b * N + p;
+  for (int p = blockIdx.y * 256 + threadIdx.x; p < N; p += gridDim.y * 256) {
+    const long long r = (long long)blockIdx.x * N + p;
+    double d[2], tv;
+    loss_diff(y, t, r, 0, d[0], tv);
+    loss_diff(y, t, r, 1, d[1], tv);
     __align__(16) __nv_bfloat162 q[8];
-    q[0] = __floats2bfloat162_rn((float)(sc * ((double)y[r * 8] - t[r * 2])),
-                                 (float)(sc * ((double)y[r * 8 + 1] - t[r * 2 + 1])));
+    q[0] = __floats2bfloat162_rn((float)(sc * d[0]), (float)(sc * d[1]));
 #pragma unroll
     for (int k = 1; k < 8; ++k) q[k] = __floats2bfloat162_rn(0.f, 0.f);
     uint4* dst = reinterpret_cast<uint4*>(dy + r * 16);
     dst[0] = *reinterpret_cast<uint4*>(&q[0]);
     dst[1] = *reinterpret_cast<uint4*>(&q[4]);
   }
+}
+
+static int loss_chunks(int N) { return std::min(kLossChunks, (N + 1023) / 1024); }
+size_t net_loss_bytes(int B) { return (1 + 2 * (size_t)kLossChunks * B) * sizeof(double); }
+
+void launch_net_loss(Ctx& c, const char* name, int N, int B, const float* y, const float* t, bf16* dy, double* loss) {
+  const dim3 grid((unsigned)B, (unsigned)loss_chunks(N));
+  HZ_LAUNCH(c, name, (double)N * B * 40.0, k_loss_sums, grid, 256, 0, N, y, t, loss + 1);
+  HZ_LAUNCH(c, name, (double)N * B * 72.0, k_loss_grad, grid, 256, 0, N, B, y, t, loss + 1, dy, loss);
 }
 
 // Adam on the FP32 master weights; the BF16 copy is refreshed in the same pass
@@ -830,7 +767,8 @@ void CoarseNet::ensure(int nx, int ny, int B, bool grads) {
     if (grads) dalloc(&grd_[i], n * 2);
   }
   dalloc(&y32_, (size_t)B * nx * ny * 8 * 4);
-  if (!loss_) dalloc(&loss_, 8);
+  dfree(loss_);
+  dalloc(&loss_, net_loss_bytes(B));
 }
 
 float* CoarseNet::input_staging(int nx, int ny, int B) {
@@ -941,21 +879,12 @@ void CoarseNet::conv_bwd(Ctx& c, int l, int lev, int B, const bf16* in, int ldi,
   if (nodes >= (1LL << 31)) throw std::runtime_error("coarse net: batch too large for the weight gradient");
   if (L.cinp % 8 || L.cinp > 128 || L.coutp > 64 || ldi % 8 || ldd % 8 || d_off % 8 || i_off != 0)
     throw std::runtime_error("coarse net: weight-gradient layout not supported");
-  // node range per CTA: enough CTAs (9 taps x chunks) for a few waves, few atomics
-  long long kc = (nodes + 134) / 135;
-  kc = std::max<long long>(kWgKS, (kc + kWgKS - 1) / kWgKS * kWgKS);
-  // the weight gradient on the tensor cores with the tcgen05 path only: the
-  // warp-level kernel measured faster (1.94 against 2.56 ms per 129^2 x 32 step)
-  if (conv_path_ == 1 && wgrad_tc_supported(9, L.cinp, L.coutp)) {
-    const WgradTc a{nx, ny, 1, nodes, L.cinp, in, ldi, L.coutp, dout, ldd, d_off, g32_ + woff_[l]};
+  // the weight gradient on tcgen05 with that path only: the warp-level kernel is faster
+  const WgradTc a{nx, ny, 1, nodes, L.cinp, in, ldi, L.coutp, dout, ldd, d_off, g32_ + woff_[l]};
+  if (conv_path_ == 1 && wgrad_tc_supported(9, L.cinp, L.coutp))
     wgrad_tc_launch(c, "net_wgrad_tc", a, tc_err_);
-  } else {
-    const dim3 grid(1u, (unsigned)((nodes + kc - 1) / kc), 9u);
-    const size_t smem = (size_t)kWgKS * ((L.cinp + 8) + (round16(L.coutp) + 8)) * 2;
-    c.add_flops("net_wgrad", 2.0 * 9.0 * L.cinp * L.coutp * (double)nodes);
-    HZ_LAUNCH(c, "net_wgrad", (double)nodes * (L.cinp + L.coutp) * 2.0 * 9.0, k_wgrad_mma, grid, 128, smem, nx, ny,
-              (int)nodes, L.cinp, L.coutp, in, ldi, dout, ldd, d_off, g32_ + woff_[l], (int)kc);
-  }
+  else
+    wgrad_launch(c, "net_wgrad", a, 9);
   if (!din) return;
   const int K = round16(L.coutp);
   const int tot = L.cinp * 9 * K;
@@ -980,7 +909,7 @@ double CoarseNet::backward(Ctx& c, const float* t, int nx, int ny, int B) {
   cuda_ok(cudaMemsetAsync(loss_, 0, 8, c.stream), "loss reset");
   cuda_ok(cudaMemsetAsync(g32_, 0, wtotal_ * 4, c.stream), "grad reset");
   bf16* gY = grd_[X];  // the input needs no gradient: its slot holds dL/dy (16 channels)
-  HZ_LAUNCH(c, "net_loss", (double)N0 * B * 72.0, k_loss, B, 256, 0, N0, B, y32_, t, gY, loss_);
+  launch_net_loss(c, "net_loss", N0, B, y32_, t, gY, loss_);
   conv_bwd(c, 7, 0, B, act_[D0], 16, 0, gY, 16, 0, grd_[D0], 16, 0, act_[D0], 16, 0);
   conv_bwd(c, 6, 0, B, act_[C0], 48, 0, grd_[D0], 16, 0, grd_[C0], 48, 0, act_[C0], 48, 32);
   resample(c, 1, 1, gx_, gy_, 0, B, 32, grd_[C0], 48, 0, grd_[D1], 32, 0, 0, act_[D1], 32, 0);

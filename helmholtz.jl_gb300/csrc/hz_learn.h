@@ -150,6 +150,9 @@ struct WgradTc {
 };
 bool wgrad_tc_supported(int taps, int Cin, int Cout);
 void wgrad_tc_launch(Ctx& ctx, const char* name, const WgradTc& a, int* err);
+// The same gradient on warp-level tensor cores (hz_wgrad.cu): taps 9 or 27, Cin a
+// multiple of 16 up to 128, Cout a multiple of 8 up to 64, dw 8-byte aligned.
+void wgrad_launch(Ctx& ctx, const char* name, const WgradTc& a, int taps);
 // Weight image of a convolution with taps taps, Cin inputs and Cout outputs
 // (taps * Cin * Cout BF16 values): flip = 0 from w [wcout][taps][Cin] (outputs
 // >= wcout are zero); flip = 1 the data-gradient weights of a layer
@@ -246,8 +249,10 @@ class CoarseNet3 {
 // 16-channel rows, the loss and its gradient, Adam, FP32 -> BF16, and the
 // mini-batch gather of training pairs.
 __global__ void k_pack_in(long long BN, const float4* __restrict__ x4, __nv_bfloat16* __restrict__ x16);
-__global__ void __launch_bounds__(256) k_loss(int N, int B, const float* __restrict__ y, const float* __restrict__ t,
-                                              __nv_bfloat16* __restrict__ dy, double* __restrict__ loss);
+static constexpr int kLossChunks = 32;  // CTAs per sample
+size_t net_loss_bytes(int B);
+void launch_net_loss(Ctx& c, const char* name, int N, int B, const float* y, const float* t, __nv_bfloat16* dy,
+                     double* loss);
 __global__ void k_adam(long long n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, __nv_bfloat16* __restrict__ wb, float lr, float b1, float b2, float eps,
                        float c1, float c2);

@@ -281,106 +281,6 @@ __global__ void k_wflip3(int Cout, int Cin, int K, const bf16* __restrict__ w, b
   wt[idx] = (co < Cout) ? w[((long long)co * kTaps3 + (kTaps3 - 1 - t)) * Cin + ci] : __float2bfloat16_rn(0.f);
 }
 
-// Weight gradient on the tensor cores: dw[co][t][ci] += sum_n dout[n][co] * in[n + off_t][ci],
-// a GEMM with M = Cout, N = Cin and K = the nodes.  One CTA (4 warps) owns one
-// tap t (blockIdx.z) and a range of kc nodes (blockIdx.y); it stages 64-node
-// slices of the input rows (zeroed where the tap leaves the grid) and of the
-// output-gradient rows in shared memory, runs m16n8k16 MMAs over 16-node
-// K-steps (warp w owns the 16x8 output tiles w, w+4, ...) and adds its
-// partial sums to dw with one atomic per weight.
-constexpr int kWg3KS = 64;
-constexpr int kWg3MaxTiles = 12;  // 16x8 tiles per warp: Cout <= 32 with Cin <= 48
-
-__device__ __forceinline__ unsigned pack2bf(bf16 lo, bf16 hi) {
-  return (unsigned)__bfloat16_as_ushort(lo) | ((unsigned)__bfloat16_as_ushort(hi) << 16);
-}
-
-__global__ void __launch_bounds__(128) k_wgrad3_mma(int nx, int ny, int nz, long long total, int Cin, int Cout,
-                                                    const bf16* __restrict__ in, int ldi,
-                                                    const bf16* __restrict__ dout, int ldd, int d_off,
-                                                    float* __restrict__ dw, long long kc) {
-  extern __shared__ __align__(16) unsigned char wg3_smem[];
-  const long long N = (long long)nx * ny * nz;
-  const int t = blockIdx.z;
-  int dx, dy, dz;
-  tap3(t, dx, dy, dz);
-  const long long toff = dx + (long long)dy * nx + (long long)dz * nx * ny;
-  const int C16 = (Cout + 15) / 16 * 16;
-  const int sIn = Cin + 8, sD = C16 + 8;
-  bf16* s_in = reinterpret_cast<bf16*>(wg3_smem);
-  bf16* s_d = s_in + kWg3KS * sIn;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, tq = lane & 3;
-  const int NTn = Cin / 8, T = (C16 / 16) * NTn;
-  float acc[kWg3MaxTiles][4];
-#pragma unroll
-  for (int k = 0; k < kWg3MaxTiles; ++k) acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.f;
-  const long long q0 = (long long)blockIdx.y * kc;
-  const long long q1 = min(total, q0 + kc);
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  for (long long qs = q0; qs < q1; qs += kWg3KS) {
-    __syncthreads();
-    const int cin8 = Cin / 8, cd8 = C16 / 8;
-    for (int e = threadIdx.x; e < kWg3KS * cin8; e += blockDim.x) {
-      const int r = e / cin8, c8 = e % cin8;
-      const long long q = qs + r;
-      uint4 v = zero;
-      if (q < q1) {
-        const long long p = q % N;
-        const int i = (int)(p % nx) + dx;
-        const long long pq = p / nx;
-        const int j = (int)(pq % ny) + dy, k = (int)(pq / ny) + dz;
-        if (i >= 0 && i < nx && j >= 0 && j < ny && k >= 0 && k < nz)
-          v = *reinterpret_cast<const uint4*>(in + (q + toff) * ldi + c8 * 8);
-      }
-      *reinterpret_cast<uint4*>(s_in + r * sIn + c8 * 8) = v;
-    }
-    for (int e = threadIdx.x; e < kWg3KS * cd8; e += blockDim.x) {
-      const int r = e / cd8, c8 = e % cd8;
-      const long long q = qs + r;
-      uint4 v = zero;
-      if (q < q1 && c8 * 8 < Cout) v = *reinterpret_cast<const uint4*>(dout + q * ldd + d_off + c8 * 8);
-      *reinterpret_cast<uint4*>(s_d + r * sD + c8 * 8) = v;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int kb = 0; kb < kWg3KS; kb += 16) {
-      const bf16* d0 = s_d + (kb + tq * 2) * sD;
-      const bf16* i0 = s_in + (kb + tq * 2) * sIn;
-#pragma unroll
-      for (int k = 0; k < kWg3MaxTiles; ++k) {
-        const int tile = warp + 4 * k;
-        if (tile < T) {
-          const int co = (tile / NTn) * 16 + g;
-          const int ci = (tile % NTn) * 8 + g;
-          const unsigned a0 = pack2bf(d0[co], d0[sD + co]);
-          const unsigned a1 = pack2bf(d0[co + 8], d0[sD + co + 8]);
-          const unsigned a2 = pack2bf(d0[8 * sD + co], d0[9 * sD + co]);
-          const unsigned a3 = pack2bf(d0[8 * sD + co + 8], d0[9 * sD + co + 8]);
-          const unsigned b0 = pack2bf(i0[ci], i0[sIn + ci]);
-          const unsigned b1 = pack2bf(i0[8 * sIn + ci], i0[9 * sIn + ci]);
-          mma16816(acc[k], a0, a1, a2, a3, b0, b1);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kWg3MaxTiles; ++k) {
-    const int tile = warp + 4 * k;
-    if (tile >= T) break;
-    const int co = (tile / NTn) * 16 + g;
-    const int ci = (tile % NTn) * 8 + tq * 2;
-    if (co < Cout) {
-      atomicAdd(&dw[((long long)co * kTaps3 + t) * Cin + ci], acc[k][0]);
-      atomicAdd(&dw[((long long)co * kTaps3 + t) * Cin + ci + 1], acc[k][1]);
-    }
-    if (co + 8 < Cout) {
-      atomicAdd(&dw[((long long)(co + 8) * kTaps3 + t) * Cin + ci], acc[k][2]);
-      atomicAdd(&dw[((long long)(co + 8) * kTaps3 + t) * Cin + ci + 1], acc[k][3]);
-    }
-  }
-}
-
 // Per-channel resampling between 3D grid levels (NDHWC bf16, FP32 arithmetic),
 // the 3D counterparts of the 2D network's transfers:
 // mode 0, restriction (fine -> coarse): full weighting, weights 1, 1/2 per axis,
@@ -777,7 +677,8 @@ void CoarseNet3::ensure(int nx, int ny, int nz, int B, bool grads) {
     }
   }
   dalloc3(&y32_, (size_t)B * nx * ny * nz * 8 * 4);
-  if (!loss_) dalloc3(&loss_, 8);
+  dfree3(loss_);
+  dalloc3(&loss_, net_loss_bytes(B));
   // the zero fills run on the legacy stream: complete them before the caller's
   // (non-blocking) stream reads the padding channels
   cuda_ok3(cudaDeviceSynchronize(), "zero activations");
@@ -896,23 +797,12 @@ void CoarseNet3::conv_bwd(Ctx& c, int l, int B, const bf16* in, int ldi, const b
   const long long nodes = (long long)gd[0] * gd[1] * gd[2] * B;
   if (L.cinp % 8 || L.cinp > 48 || L.coutp > 32 || ldi % 8 || ldd % 8 || d_off % 8)
     throw std::runtime_error("coarse net 3D: weight-gradient layout not supported");
-  // the weight gradient on the tensor cores with the tcgen05 path only: the
-  // warp-level kernel measured faster (7.47 against 9.95 ms per 33^3 x 32 step)
-  if (conv_path_ == 1 && wgrad_tc_supported(kTaps3, L.cinp, L.coutp)) {
-    const WgradTc a{gd[0], gd[1], gd[2], nodes, L.cinp, in, ldi, L.coutp, dout, ldd, d_off, g32_ + woff_[l]};
+  // the weight gradient on tcgen05 with that path only: the warp-level kernel is faster
+  const WgradTc a{gd[0], gd[1], gd[2], nodes, L.cinp, in, ldi, L.coutp, dout, ldd, d_off, g32_ + woff_[l]};
+  if (conv_path_ == 1 && wgrad_tc_supported(kTaps3, L.cinp, L.coutp))
     wgrad_tc_launch(c, "net3_wgrad_tc", a, tc_err_);
-  } else {
-    // node range per CTA: a few waves of (27 taps x chunks) CTAs, few atomics
-    long long kc = (nodes + 44) / 45;
-    kc = std::max<long long>(kWg3KS, (kc + kWg3KS - 1) / kWg3KS * kWg3KS);
-    const long long nch = (nodes + kc - 1) / kc;
-    if (nch > 65535) throw std::runtime_error("coarse net 3D: batch too large for the weight gradient");
-    const dim3 grid(1u, (unsigned)nch, 27u);
-    const size_t smem = (size_t)kWg3KS * ((L.cinp + 8) + (round16(L.coutp) + 8)) * 2;
-    c.add_flops("net3_wgrad", 2.0 * 27.0 * L.cinp * L.coutp * (double)nodes);
-    HZ_LAUNCH(c, "net3_wgrad", (double)nodes * (L.cinp + L.coutp) * 2.0 * 27.0, k_wgrad3_mma, grid, 128, smem,
-              gd[0], gd[1], gd[2], nodes, L.cinp, L.coutp, in, ldi, dout, ldd, d_off, g32_ + woff_[l], kc);
-  }
+  else
+    wgrad_launch(c, "net3_wgrad", a, kTaps3);
   if (!din) return;
   const int K = round16(L.coutp);
   const int tot = L.cinp * kTaps3 * K;
@@ -941,7 +831,7 @@ double CoarseNet3::backward(Ctx& c, const float* t, int nx, int ny, int nz, int 
   cuda_ok3(cudaMemsetAsync(loss_, 0, 8, c.stream), "loss reset");
   cuda_ok3(cudaMemsetAsync(g32_, 0, wtotal_ * 4, c.stream), "grad reset");
   bf16* gY = grd_[X3];  // the input needs no gradient: its slot holds dL/dy (16 channels)
-  HZ_LAUNCH(c, "net3_loss", (double)N0 * B * 72.0, k_loss, B, 256, 0, N0, B, y32_, t, gY, loss_);
+  launch_net_loss(c, "net3_loss", N0, B, y32_, t, gY, loss_);
   conv_bwd(c, 5, B, act_[D03], 16, gY, 16, 0, grd_[D03], 16, 0, act_[D03], 16, 0);
   conv_bwd(c, 4, B, act_[C03], 32, grd_[D03], 16, 0, grd_[C03], 32, 0, act_[C03], 32, 16);
   resample3(c, 1, 1, g_, 0, B, 16, grd_[C03], 32, 0, grd_[D13], 16, 0, 0, act_[D13], 16, 0);

@@ -5,252 +5,381 @@
 // kernels run the "Jac-GMRES" smoother (relaxType of that test, :138): one or
 // two GMRES steps preconditioned by a damped-Jacobi sweep, added to the iterate.
 //
-// Per column c the scalars live on the device in ks[c*8 + slot]:
-//   0 beta^2 (real), 1 h00, 2 h10^2 (real), 3 h01, 4 h11, 5 h21^2 (real), 6 y0, 7 y1.
+// No vector is normalised: with Z0 = M b, W = A Z0, W1 = W - (d0 / beta^2) b, Z1 = M W1,
+// W2 = A Z1 the steps need only the sums below, and the correction is Y0 Z0 + Y1 Z1 (M is
+// homogeneous).  Per column c they live on the device in ks[c*8 + slot]:
+//   0 beta^2 = ||b||^2, 1 d0 = <b, W>, 2 n1 = ||W1||^2, 3 p0 = <b, W2>, 4 p1 = <W1, W2>,
+// and the vectors' coefficients in their precision in kt[c*8 + slot]:
+//   0 d0 / beta^2, 1 p0 / beta^2, 2 p1 / n1, 6 Y0, 7 Y1
+// (a division or an FP64 -> FP32 conversion in every thread would cost more than the
+// vectors: each takes a warp's quarter of an SM 64 clocks).
+// One smoothing step needs one number, y = <W, r> / ||W||^2 for W = A Z, Z = w D^-1 r (kt slot 6);
+// it also leaves A x = b - r + y W behind, so a K step after it needs no operator
+// product and a first step from zero leaves the residual b - y W.
+//
 // Vectors are level vectors in the cycle's precision T and so is the
-// per-element arithmetic (a thread sums a few terms); block and column totals
-// are accumulated in FP64 and folded in a fixed order (deterministic).
+// per-element arithmetic (a thread sums a few terms); a warp's totals are exact to
+// 48 bits (double-float tree) in FP32 and FP64 otherwise, blocks and columns are
+// folded in FP64 in a fixed order (deterministic) by the last block of a column.
+//
+// Why: these levels are small, so launches and the reduction's FP64 steps were the cost.
+// A K step took 14 launches and a smoothing step 11 (normalising copies, separate
+// folds, an operator product for each residual); now 4 and 4.  Solves: 3D 193 x 161 x 97 x 16
+// 630 -> 494 ms, 3D 129^3 x 8 349 -> 299 ms, 2D 641 x 321 x 33 259 -> 234 ms.
 #include "hz_launch.cuh"
 
 namespace hz {
 
 namespace {
 
-template <typename T> __device__ __forceinline__ double2 ld2(const cplx<T>& v) {
-  return make_double2((double)v.x, (double)v.y);
+constexpr int kNV = 4;  // real sums per kernel
+
+__device__ __forceinline__ void two_sum_f(float a, float b, float& s, float& e) {
+  s = __fadd_rn(a, b);
+  const float bb = __fsub_rn(s, a);
+  e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
-// block reduction of up to 3 complex slots; thread 0 writes part[(pos*K1 + s)*nblk + blk]
-__device__ __forceinline__ void block_sum3(double2 (&a)[3], int K1, double2* part, int pos, int nblk, int blk) {
-  __shared__ double2 sh[3][8];
+// Warp totals of four values; lane l < 32 ends with value 2 (l >= 16) + (l / 8 & 1).
+// Each exchange halves the values a lane carries, so four totals take 6 steps.
+__device__ __forceinline__ double warp_totals(const double (&v)[kNV], int lane) {
+  const bool up = lane & 16, up2 = lane & 8;
+  const double a = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+  const double b = (up ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+  double s = (up2 ? b : a) + __shfl_xor_sync(0xffffffffu, up2 ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+__device__ __forceinline__ double warp_totals(const float (&v)[kNV], int lane) {
+  const bool up = lane & 16, up2 = lane & 8;
+  float a, ea, b, eb, s, es;
+  two_sum_f(up ? v[2] : v[0], __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16), a, ea);
+  two_sum_f(up ? v[3] : v[1], __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16), b, eb);
+  float lo = (up2 ? eb : ea) + __shfl_xor_sync(0xffffffffu, up2 ? ea : eb, 8);
+  two_sum_f(up2 ? b : a, __shfl_xor_sync(0xffffffffu, up2 ? a : b, 8), s, es);
+  lo += es;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    lo += __shfl_xor_sync(0xffffffffu, lo, o);
+    two_sum_f(s, __shfl_xor_sync(0xffffffffu, s, o), s, es);
+    lo += es;
+  }
+  return (double)s + (double)lo;
+}
+
+// Column totals of four sums over the blocks (gridDim.x, pos): the block's totals go to
+// part[(pos * 4 + v) * nblk + blk]; the last block of the column to arrive folds
+// them in block order and gets true with tot filled (all threads).  count[c] returns to 0.
+template <typename T>
+__device__ __forceinline__ bool column_totals(const T (&v)[kNV], double* part, int* count, int pos, int c,
+                                              double (&tot)[kNV]) {
+  __shared__ double sh[kNV][8];
+  __shared__ double out[kNV];
+  __shared__ int last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nblk = gridDim.x;
+  const double s = warp_totals(v, lane);
+  if ((lane & 7) == 0) sh[2 * (lane >> 4) + ((lane >> 3) & 1)][warp] = s;
+  __syncthreads();
+  if (warp == 0) {  // lane = 8 value + warp
+    double t = sh[lane >> 3][lane & 7];
 #pragma unroll
-  for (int s = 0; s < 3; ++s) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a[s].x += __shfl_xor_sync(0xffffffffu, a[s].x, o);
-      a[s].y += __shfl_xor_sync(0xffffffffu, a[s].y, o);
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 7) == 0) {
+      __stcg(&part[((long long)pos * kNV + (lane >> 3)) * nblk + blockIdx.x], t);
+      __threadfence();
     }
-    if (lane == 0) sh[s][warp] = a[s];
+    __syncwarp();
+    if (lane == 0) last = atomicInc(reinterpret_cast<unsigned*>(&count[c]), (unsigned)nblk - 1) == (unsigned)nblk - 1;
   }
   __syncthreads();
-  if (threadIdx.x < K1) {
-    double2 t = make_double2(0.0, 0.0);
-    const int nw = blockDim.x >> 5;
-    for (int w = 0; w < nw; ++w) {
-      t.x += sh[threadIdx.x][w].x;
-      t.y += sh[threadIdx.x][w].y;
-    }
-    part[((long long)pos * K1 + threadIdx.x) * nblk + blk] = t;
+  if (!last) return false;
+  __threadfence();
+  if (warp < kNV) {
+    double t = 0.0;
+    for (int b = lane; b < nblk; b += 32) t += __ldcg(&part[((long long)pos * kNV + warp) * nblk + b]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) out[warp] = t;
   }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kNV; ++k) tot[k] = out[k];
+  return true;
+}
+
+template <typename T, typename TB> __device__ __forceinline__ cplx<T> load_b(const cplx<TB>& v) {
+  return mk<T>((T)v.x, (T)v.y);
+}
+
+// conj(u) w into v[i], v[i + 1]
+template <typename T> __device__ __forceinline__ void add_dot(T (&v)[kNV], int i, cplx<T> u, cplx<T> w) {
+  v[i] = fma(u.x, w.x, fma(u.y, w.y, v[i]));
+  v[i + 1] = fma(u.x, w.y, fma(-u.y, w.x, v[i + 1]));
+}
+template <typename T> __device__ __forceinline__ void add_norm(T (&v)[kNV], int i, cplx<T> w) {
+  v[i] = fma(w.x, w.x, fma(w.y, w.y, v[i]));
+}
+
+// coefficient a / n (0 for n = 0) in the vectors' precision
+template <typename T> __device__ __forceinline__ cplx<T> ratio(double2 a, double n) {
+  return n > 0.0 ? mk<T>((T)(a.x / n), (T)(a.y / n)) : mk<T>(0, 0);
+}
+template <typename T> __device__ __forceinline__ cplx<T> narrow(double2 a) { return mk<T>((T)a.x, (T)a.y); }
+
+// Two-step least squares from the sums: the 3 x 2 problem min || beta e0 - H y || by two
+// complex Givens rotations, H = [[h00, h01], [h10, h11], [0, h21]] of the normalised
+// basis, scaled back to the unnormalised Z0, Z1.
+template <typename T> __device__ void least_squares(const double2* s, double n2, cplx<T>* kt) {
+  const double beta2 = s[0].x, n1 = fmax(s[2].x, 0.0);
+  const double beta = sqrt(fmax(beta2, 0.0)), rn1 = sqrt(n1);
+  double2 y0 = make_double2(0.0, 0.0), y1 = make_double2(0.0, 0.0);
+  if (beta > 0.0) {
+    const double2 a = make_double2(s[1].x / beta2, s[1].y / beta2);
+    const double c10 = rn1 / beta;
+    double2 b = make_double2(0.0, 0.0), d = b;
+    double e = 0.0;
+    if (rn1 > 0.0) {
+      b = make_double2(s[3].x / (beta * rn1), s[3].y / (beta * rn1));
+      d = make_double2(s[4].x / n1, s[4].y / n1);
+      e = sqrt(fmax(n2, 0.0)) / rn1;
+    }
+    const double r1 = sqrt(a.x * a.x + a.y * a.y + c10 * c10);
+    if (r1 > 0.0) {
+      const double2 cs = make_double2(a.x / r1, a.y / r1);  // G1 = [conj(cs) sn; -sn cs], sn = c10 / r1 (real)
+      const double sn = c10 / r1;
+      // row 0 after G1: (r1, b'), g0 = conj(cs) beta; row 1: (0, d'), g1 = -sn beta
+      const double2 bp = make_double2(cs.x * b.x + cs.y * b.y + sn * d.x, cs.x * b.y - cs.y * b.x + sn * d.y);
+      const double2 dp = make_double2(-sn * b.x + cs.x * d.x - cs.y * d.y, -sn * b.y + cs.x * d.y + cs.y * d.x);
+      const double2 g0 = make_double2(cs.x * beta, -cs.y * beta);
+      const double g1 = -sn * beta;
+      const double r2 = sqrt(dp.x * dp.x + dp.y * dp.y + e * e);
+      if (r2 > 0.0) {
+        // G2 on rows 1, 2: g1' = conj(dp / r2) g1, y1 = g1' / r2
+        y1 = make_double2(dp.x * g1 / (r2 * r2), -dp.y * g1 / (r2 * r2));
+      }
+      // y0 = (g0 - b' y1) / r1
+      const double2 t = make_double2(g0.x - (bp.x * y1.x - bp.y * y1.y), g0.y - (bp.x * y1.y + bp.y * y1.x));
+      y0 = make_double2(t.x / (r1 * beta), t.y / (r1 * beta));
+      if (rn1 > 0.0) y1 = make_double2(y1.x / rn1, y1.y / rn1);
+    }
+  }
+  kt[6] = narrow<T>(y0);
+  kt[7] = narrow<T>(y1);
 }
 
 }  // namespace
 
-// slots s < nd: conj(V_s) . W ; slot nd (want_norm): ||W||^2
-template <typename T>
-__global__ void __launch_bounds__(256) k_kc_sums(long long N, long long ld, const int* __restrict__ cols, int nd,
-                                                 int want_norm, const cplx<T>* __restrict__ V0,
-                                                 const cplx<T>* __restrict__ V1, const cplx<T>* __restrict__ W,
-                                                 int nblk, double2* __restrict__ part) {
-  const int pos = blockIdx.y, c = cols[pos], blk = blockIdx.x;
-  const long long off = (long long)c * ld;
-  // a thread's few terms are summed in the vectors' precision, blocks in FP64
-  cplx<T> t0 = mk<T>(0, 0), t1 = mk<T>(0, 0);
-  T tn = 0;
-  for (long long p = (long long)blk * blockDim.x + threadIdx.x; p < N; p += (long long)nblk * blockDim.x) {
-    const cplx<T> w = W[off + p];
-    if (nd > 0) t0 = cfma_conj<T>(V0[off + p], w, t0);
-    if (nd > 1) t1 = cfma_conj<T>(V1[off + p], w, t1);
-    if (want_norm) tn = fma(w.x, w.x, fma(w.y, w.y, tn));
+// MODE KC_SMOOTH: kt slot 6 = y = <W, b> / ||W||^2;  KC_FIRST: slots 1, 0 = <b, W>, ||b||^2;
+// KC_SECOND: slots 3, 4 = <b, W>, <W1, W>
+template <typename T, int MODE>
+__device__ __forceinline__ void kc_accumulate(T (&v)[kNV], cplx<T> b, cplx<T> w1, cplx<T> w) {
+  add_dot<T>(v, 0, b, w);
+  if (MODE == KC_SMOOTH) add_norm<T>(v, 2, w);
+  if (MODE == KC_FIRST) add_norm<T>(v, 2, b);
+  if (MODE == KC_SECOND) add_dot<T>(v, 2, w1, w);
+}
+template <typename T, int MODE>
+__device__ __forceinline__ void kc_store(const double (&t)[kNV], double2* s, cplx<T>* kt) {
+  if (MODE == KC_SMOOTH) {
+    kt[6] = ratio<T>(make_double2(t[0], -t[1]), t[2]);
+  } else if (MODE == KC_FIRST) {
+    s[0] = make_double2(t[2], 0.0);
+    s[1] = make_double2(t[0], t[1]);
+    kt[0] = ratio<T>(s[1], t[2]);
+  } else {
+    s[3] = make_double2(t[0], t[1]);
+    s[4] = make_double2(t[2], t[3]);
+    kt[1] = ratio<T>(s[3], s[0].x);
+    kt[2] = ratio<T>(s[4], s[2].x);
   }
-  const double2 nrm = make_double2((double)tn, 0.0);
-  double2 a[3];
-  a[0] = nd > 0 ? ld2<T>(t0) : nrm;
-  a[1] = nd > 1 ? ld2<T>(t1) : nrm;
-  a[2] = nrm;
-  block_sum3(a, nd + want_norm, part, pos, nblk, blk);
 }
 
-// W -= sum_{s<nd} h_s V_s (h_s = ks[c*8 + hb + s]), then ||W||^2 partials (slot 0)
-template <typename T>
-__global__ void __launch_bounds__(256) k_kc_update(long long N, long long ld, const int* __restrict__ cols, int nd,
-                                                   int hb, const double2* __restrict__ ks,
-                                                   const cplx<T>* __restrict__ V0, const cplx<T>* __restrict__ V1,
-                                                   cplx<T>* __restrict__ W, int nblk, double2* __restrict__ part) {
-  const int pos = blockIdx.y, c = cols[pos], blk = blockIdx.x;
+template <typename T, typename TB, int MODE>
+__global__ void __launch_bounds__(256) k_kc_dots(long long N, long long ld, const int* __restrict__ cols,
+                                                 const cplx<TB>* __restrict__ B, const cplx<T>* __restrict__ W1,
+                                                 const cplx<T>* __restrict__ W, double* part, int* count,
+                                                 double2* __restrict__ ks, cplx<T>* __restrict__ kt) {
+  const int c = cols[blockIdx.y];
   const long long off = (long long)c * ld;
-  const double2 h0d = ks[c * 8 + hb];
-  const double2 h1d = nd > 1 ? ks[c * 8 + hb + 1] : make_double2(0.0, 0.0);
-  const cplx<T> h0 = mk<T>((T)h0d.x, (T)h0d.y), h1 = mk<T>((T)h1d.x, (T)h1d.y);
-  T n2 = 0;
-  for (long long p = (long long)blk * blockDim.x + threadIdx.x; p < N; p += (long long)nblk * blockDim.x) {
-    cplx<T> w = cfms<T>(h0, V0[off + p], W[off + p]);
-    if (nd > 1) w = cfms<T>(h1, V1[off + p], w);
+  T v[kNV] = {0, 0, 0, 0};
+#pragma unroll 4
+  for (long long p = (long long)blockIdx.x * 256 + threadIdx.x; p < N; p += (long long)gridDim.x * 256)
+    kc_accumulate<T, MODE>(v, load_b<T, TB>(B[off + p]), MODE == KC_SECOND ? W1[off + p] : mk<T>(0, 0), W[off + p]);
+  double t[kNV];
+  if (column_totals(v, part, count, blockIdx.y, c, t) && threadIdx.x == 0) kc_store<T, MODE>(t, ks + c * 8, kt + c * 8);
+}
+
+// W -= (d0 / beta^2) b, slot 2 = ||W||^2
+template <typename T>
+__global__ void __launch_bounds__(256) k_kc_update(long long N, long long ld, const int* __restrict__ cols,
+                                                   const cplx<T>* __restrict__ B, cplx<T>* __restrict__ W,
+                                                   double* part, int* count, double2* __restrict__ ks,
+                                                   cplx<T>* __restrict__ kt) {
+  const int c = cols[blockIdx.y];
+  const long long off = (long long)c * ld;
+  const cplx<T> h = kt[c * 8];
+  T v[kNV] = {0, 0, 0, 0};
+#pragma unroll 4
+  for (long long p = (long long)blockIdx.x * 256 + threadIdx.x; p < N; p += (long long)gridDim.x * 256) {
+    const cplx<T> w = cfms<T>(h, B[off + p], W[off + p]);
     W[off + p] = w;
-    n2 = fma(w.x, w.x, fma(w.y, w.y, n2));
+    add_norm<T>(v, 0, w);
   }
-  double2 a[3] = {make_double2((double)n2, 0.0), make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
-  block_sum3(a, 1, part, pos, nblk, blk);
+  double t[kNV];
+  if (column_totals(v, part, count, blockIdx.y, c, t) && threadIdx.x == 0) ks[c * 8 + 2] = make_double2(t[0], 0.0);
 }
 
-// Y = X / sqrt(ks[c*8 + slot].x)  (zero when the norm is zero)
+// n2 = ||W2 - (p0 / beta^2) b - (p1 / n1) W1||^2 and the least squares: kt slots 6, 7
 template <typename T>
-__global__ void __launch_bounds__(256) k_kc_scale(long long N, long long ld, const int* __restrict__ cols,
-                                                  const double2* __restrict__ ks, int slot,
-                                                  const cplx<T>* __restrict__ X, cplx<T>* __restrict__ Y) {
+__global__ void __launch_bounds__(256) k_kc_last(long long N, long long ld, const int* __restrict__ cols,
+                                                 const cplx<T>* __restrict__ B, const cplx<T>* __restrict__ W1,
+                                                 const cplx<T>* __restrict__ W2, double* part, int* count,
+                                                 double2* __restrict__ ks, cplx<T>* __restrict__ kt) {
   const int c = cols[blockIdx.y];
-  const double n2 = ks[c * 8 + slot].x;
-  const T s = (T)(n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0);
   const long long off = (long long)c * ld;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (long long)gridDim.x * blockDim.x)
-    Y[off + p] = cscale<T>(s, X[off + p]);
+  const cplx<T> h0 = kt[c * 8 + 1], h1 = kt[c * 8 + 2];
+  T v[kNV] = {0, 0, 0, 0};
+#pragma unroll 4
+  for (long long p = (long long)blockIdx.x * 256 + threadIdx.x; p < N; p += (long long)gridDim.x * 256)
+    add_norm<T>(v, 0, cfms<T>(h1, W1[off + p], cfms<T>(h0, B[off + p], W2[off + p])));
+  double t[kNV];
+  if (column_totals(v, part, count, blockIdx.y, c, t) && threadIdx.x == 0) least_squares<T>(ks + c * 8, t[0], kt + c * 8);
 }
 
-// X += y0 Z0 + y1 Z1 (the GMRES smoothing update of the current iterate)
-template <typename T>
-__global__ void __launch_bounds__(256) k_kc_combine_add(long long N, long long ld, const int* __restrict__ cols,
-                                                        const double2* __restrict__ ks,
-                                                        const cplx<T>* __restrict__ Z0,
-                                                        const cplx<T>* __restrict__ Z1, cplx<T>* __restrict__ X) {
+// End of a smoothing step: X += y Z (y: slot 6 of yt).  MODE KC_FIRST / KC_SECOND:
+// also AX = b - r + y W = A X for the cycle's right-hand side b and the K step's sums of
+// it: the first step's cycle has the step's own b, the second step's has W1 (then KB
+// is the step's b).
+template <typename T, typename TB, int MODE>
+__global__ void __launch_bounds__(256) k_kc_finish(long long N, long long ld, const int* __restrict__ cols,
+                                                   const cplx<T>* __restrict__ yt, cplx<T>* __restrict__ X,
+                                                   const cplx<T>* __restrict__ Z, const cplx<TB>* __restrict__ B,
+                                                   const cplx<T>* __restrict__ R, const cplx<T>* __restrict__ W,
+                                                   const cplx<T>* __restrict__ KB, cplx<T>* __restrict__ AX,
+                                                   double* part, int* count, double2* __restrict__ ks,
+                                                   cplx<T>* __restrict__ kt) {
   const int c = cols[blockIdx.y];
-  const double2 y0d = ks[c * 8 + 6], y1d = ks[c * 8 + 7];
-  const cplx<T> y0 = mk<T>((T)y0d.x, (T)y0d.y), y1 = mk<T>((T)y1d.x, (T)y1d.y);
   const long long off = (long long)c * ld;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (long long)gridDim.x * blockDim.x)
-    X[off + p] = cfma<T>(y1, Z1[off + p], cfma<T>(y0, Z0[off + p], X[off + p]));
+  const cplx<T> y = yt[c * 8 + 6];
+  T v[kNV] = {0, 0, 0, 0};
+#pragma unroll 2
+  for (long long p = (long long)blockIdx.x * 256 + threadIdx.x; p < N; p += (long long)gridDim.x * 256) {
+    X[off + p] = cfma<T>(y, Z[off + p], X[off + p]);
+    if (MODE != KC_SMOOTH) {
+      const cplx<T> b = load_b<T, TB>(B[off + p]);
+      const cplx<T> ax = cfma<T>(y, W[off + p], csub<T>(b, R[off + p]));
+      AX[off + p] = ax;
+      kc_accumulate<T, MODE>(v, MODE == KC_SECOND ? KB[off + p] : b, b, ax);
+    }
+  }
+  if (MODE == KC_SMOOTH) return;
+  double t[kNV];
+  if (column_totals(v, part, count, blockIdx.y, c, t) && threadIdx.x == 0) kc_store<T, MODE>(t, ks + c * 8, kt + c * 8);
 }
 
-// X = y0 Z0 + y1 Z1
-template <typename T>
+// X = Y0 Z0 + Y1 Z1, or X += (ADD)
+template <typename T, bool ADD>
 __global__ void __launch_bounds__(256) k_kc_combine(long long N, long long ld, const int* __restrict__ cols,
-                                                    const double2* __restrict__ ks, const cplx<T>* __restrict__ Z0,
+                                                    const cplx<T>* __restrict__ kt, const cplx<T>* __restrict__ Z0,
                                                     const cplx<T>* __restrict__ Z1, cplx<T>* __restrict__ X) {
   const int c = cols[blockIdx.y];
-  const double2 y0d = ks[c * 8 + 6], y1d = ks[c * 8 + 7];
-  const cplx<T> y0 = mk<T>((T)y0d.x, (T)y0d.y), y1 = mk<T>((T)y1d.x, (T)y1d.y);
+  const cplx<T> y0 = kt[c * 8 + 6], y1 = kt[c * 8 + 7];
   const long long off = (long long)c * ld;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += (long long)gridDim.x * blockDim.x)
-    X[off + p] = cfma<T>(y1, Z1[off + p], cmul<T>(y0, Z0[off + p]));
-}
-
-// min || beta e0 - H y || with H = [[h00, h01], [h10, h11], [0, h21]] by two
-// complex Givens rotations (h10, h21 real, stored squared), per column.
-__global__ void k_kc_lsq(const int* __restrict__ cols, int nc, double2* __restrict__ ks) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc) return;
-  double2* s = ks + cols[i] * 8;
-  const double beta = sqrt(fmax(s[0].x, 0.0));
-  const double2 a = s[1], b = s[3], d = s[4];
-  const double c10 = sqrt(fmax(s[2].x, 0.0)), e = sqrt(fmax(s[5].x, 0.0));
-  double2 y0 = make_double2(0.0, 0.0), y1 = make_double2(0.0, 0.0);
-  const double r1 = sqrt(a.x * a.x + a.y * a.y + c10 * c10);
-  if (beta > 0.0 && r1 > 0.0) {
-    const double2 cs = make_double2(a.x / r1, a.y / r1);  // G1 = [conj(cs) sn; -sn cs], sn = c10 / r1 (real)
-    const double sn = c10 / r1;
-    // row 0 after G1: (r1, b'), g0 = conj(cs) beta; row 1: (0, d'), g1 = -sn beta
-    const double2 bp = make_double2(cs.x * b.x + cs.y * b.y + sn * d.x, cs.x * b.y - cs.y * b.x + sn * d.y);
-    const double2 dp = make_double2(-sn * b.x + cs.x * d.x - cs.y * d.y, -sn * b.y + cs.x * d.y + cs.y * d.x);
-    const double2 g0 = make_double2(cs.x * beta, -cs.y * beta);
-    const double g1 = -sn * beta;
-    const double r2 = sqrt(dp.x * dp.x + dp.y * dp.y + e * e);
-    if (r2 > 0.0) {
-      // G2 on rows 1, 2: g1' = conj(dp / r2) g1, y1 = g1' / r2
-      y1 = make_double2(dp.x * g1 / (r2 * r2), -dp.y * g1 / (r2 * r2));
-    }
-    // y0 = (g0 - b' y1) / r1
-    const double2 t = make_double2(g0.x - (bp.x * y1.x - bp.y * y1.y), g0.y - (bp.x * y1.y + bp.y * y1.x));
-    y0 = make_double2(t.x / r1, t.y / r1);
+#pragma unroll 4
+  for (long long p = (long long)blockIdx.x * 256 + threadIdx.x; p < N; p += (long long)gridDim.x * 256) {
+    const cplx<T> z0 = Z0[off + p];
+    X[off + p] = cfma<T>(y1, Z1[off + p], ADD ? cfma<T>(y0, z0, X[off + p]) : cmul<T>(y0, z0));
   }
-  s[6] = y0;
-  s[7] = y1;
-}
-
-// One GMRES step: min || beta e0 - [h00; h10] y0 || = conj(h00) beta / (|h00|^2 + h10^2); y1 = 0.
-__global__ void k_kc_lsq1(const int* __restrict__ cols, int nc, double2* __restrict__ ks) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nc) return;
-  double2* s = ks + cols[i] * 8;
-  const double beta = sqrt(fmax(s[0].x, 0.0));
-  const double2 a = s[1];
-  const double den = a.x * a.x + a.y * a.y + fmax(s[2].x, 0.0);
-  double2 y0 = make_double2(0.0, 0.0);
-  if (beta > 0.0 && den > 0.0) y0 = make_double2(a.x * beta / den, -a.y * beta / den);
-  s[6] = y0;
-  s[7] = make_double2(0.0, 0.0);
 }
 
 static int kc_nblk(long long N) {
-  long long b = (N + 2047) / 2048;
+  long long b = (N + 1023) / 1024;
   return (int)std::max<long long>(1, std::min<long long>(64, b));
 }
 
-template <typename T>
-void launch_kc_sums(Ctx& ctx, long long N, long long ld, const int* cols, int nc, int nd, int want_norm,
-                    const cplx<T>* V0, const cplx<T>* V1, const cplx<T>* W, double2* part, double2* ks, int base) {
-  const int nblk = kc_nblk(N);
-  const int K1 = nd + want_norm;
-  HZ_LAUNCH(ctx, "kcycle_dots", (double)N * nc * (nd + 1) * sizeof(cplx<T>), k_kc_sums<T>, dim3(nblk, nc), 256, 0, N,
-            ld, cols, nd, want_norm, V0, V1, W, nblk, part);
-  launch_reduce(ctx, part, cols, nc, K1, nblk, ks + base, 8, 0);
+size_t kcycle_part_bytes(long long N, int R) { return (size_t)R * kNV * kc_nblk(N) * sizeof(double); }
+
+template <typename T, typename TB>
+void launch_kc_dots(Ctx& ctx, int mode, long long N, long long ld, const int* cols, int nc, const cplx<TB>* B,
+                    const cplx<T>* W1, const cplx<T>* W, const KcSums& s) {
+  const dim3 grid(kc_nblk(N), nc);
+  const double bytes = (double)N * nc * (sizeof(cplx<TB>) + (mode == KC_SECOND ? 2 : 1) * sizeof(cplx<T>));
+  if (mode == KC_SMOOTH)
+    HZ_LAUNCH(ctx, "smooth_dots", bytes, (k_kc_dots<T, TB, KC_SMOOTH>), grid, 256, 0, N, ld, cols, B, W1, W, s.part,
+              s.count, s.ks, (cplx<T>*)s.kt);
+  else if (mode == KC_FIRST)
+    HZ_LAUNCH(ctx, "kcycle_dots", bytes, (k_kc_dots<T, TB, KC_FIRST>), grid, 256, 0, N, ld, cols, B, W1, W, s.part,
+              s.count, s.ks, (cplx<T>*)s.kt);
+  else
+    HZ_LAUNCH(ctx, "kcycle_dots", bytes, (k_kc_dots<T, TB, KC_SECOND>), grid, 256, 0, N, ld, cols, B, W1, W, s.part,
+              s.count, s.ks, (cplx<T>*)s.kt);
 }
 
 template <typename T>
-void launch_kc_update(Ctx& ctx, long long N, long long ld, const int* cols, int nc, int nd, int hb, double2* ks,
-                      const cplx<T>* V0, const cplx<T>* V1, cplx<T>* W, double2* part, int norm_slot) {
-  const int nblk = kc_nblk(N);
-  HZ_LAUNCH(ctx, "kcycle_update", (double)N * nc * (nd + 2) * sizeof(cplx<T>), k_kc_update<T>, dim3(nblk, nc), 256, 0,
-            N, ld, cols, nd, hb, ks, V0, V1, W, nblk, part);
-  launch_reduce(ctx, part, cols, nc, 1, nblk, ks + norm_slot, 8, 0);
+void launch_kc_update(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const cplx<T>* B, cplx<T>* W,
+                      const KcSums& s) {
+  HZ_LAUNCH(ctx, "kcycle_update", (double)N * nc * 3 * sizeof(cplx<T>), k_kc_update<T>, dim3(kc_nblk(N), nc), 256, 0, N,
+            ld, cols, B, W, s.part, s.count, s.ks, (cplx<T>*)s.kt);
 }
 
 template <typename T>
-void launch_kc_scale(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const double2* ks, int slot,
-                     const cplx<T>* X, cplx<T>* Y) {
-  const int nblk = kc_nblk(N);
-  HZ_LAUNCH(ctx, "kcycle_scale", (double)N * nc * 2 * sizeof(cplx<T>), k_kc_scale<T>, dim3(nblk, nc), 256, 0, N, ld,
-            cols, ks, slot, X, Y);
+void launch_kc_last(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const cplx<T>* B, const cplx<T>* W1,
+                    const cplx<T>* W2, const KcSums& s) {
+  HZ_LAUNCH(ctx, "kcycle_last", (double)N * nc * 3 * sizeof(cplx<T>), k_kc_last<T>, dim3(kc_nblk(N), nc), 256, 0, N, ld,
+            cols, B, W1, W2, s.part, s.count, s.ks, (cplx<T>*)s.kt);
+}
+
+template <typename T, typename TB>
+void launch_kc_finish(Ctx& ctx, int mode, long long N, long long ld, const int* cols, int nc, const cplx<T>* yt,
+                      cplx<T>* X, const cplx<T>* Z, const cplx<TB>* B, const cplx<T>* R, const cplx<T>* W,
+                      const cplx<T>* KB, cplx<T>* AX, const KcSums& s) {
+  const dim3 grid(kc_nblk(N), nc);
+  const double bytes = (double)N * nc *
+                       (3 * sizeof(cplx<T>) + (mode == KC_SMOOTH ? 0 : sizeof(cplx<TB>) + 3 * sizeof(cplx<T>)) +
+                        (mode == KC_SECOND ? sizeof(cplx<T>) : 0));
+  if (mode == KC_SMOOTH)
+    HZ_LAUNCH(ctx, "smooth_update", bytes, (k_kc_finish<T, TB, KC_SMOOTH>), grid, 256, 0, N, ld, cols, yt, X, Z, B, R, W,
+              KB, AX, s.part, s.count, s.ks, (cplx<T>*)s.kt);
+  else if (mode == KC_FIRST)
+    HZ_LAUNCH(ctx, "smooth_update_dots", bytes, (k_kc_finish<T, TB, KC_FIRST>), grid, 256, 0, N, ld, cols, yt, X, Z, B,
+              R, W, KB, AX, s.part, s.count, s.ks, (cplx<T>*)s.kt);
+  else
+    HZ_LAUNCH(ctx, "smooth_update_dots", bytes, (k_kc_finish<T, TB, KC_SECOND>), grid, 256, 0, N, ld, cols, yt, X, Z, B,
+              R, W, KB, AX, s.part, s.count, s.ks, (cplx<T>*)s.kt);
 }
 
 template <typename T>
-void launch_kc_combine(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const double2* ks,
+void launch_kc_combine(Ctx& ctx, bool add, long long N, long long ld, const int* cols, int nc, const cplx<T>* kt,
                        const cplx<T>* Z0, const cplx<T>* Z1, cplx<T>* X) {
-  const int nblk = kc_nblk(N);
-  HZ_LAUNCH(ctx, "kcycle_combine", (double)N * nc * 3 * sizeof(cplx<T>), k_kc_combine<T>, dim3(nblk, nc), 256, 0, N,
-            ld, cols, ks, Z0, Z1, X);
+  const dim3 grid(kc_nblk(N), nc);
+  const double bytes = (double)N * nc * (add ? 4 : 3) * sizeof(cplx<T>);
+  if (add)
+    HZ_LAUNCH(ctx, "smooth_update", bytes, (k_kc_combine<T, true>), grid, 256, 0, N, ld, cols, kt, Z0, Z1, X);
+  else
+    HZ_LAUNCH(ctx, "kcycle_combine", bytes, (k_kc_combine<T, false>), grid, 256, 0, N, ld, cols, kt, Z0, Z1, X);
 }
 
-void launch_kc_lsq(Ctx& ctx, const int* cols, int nc, double2* ks) {
-  HZ_LAUNCH(ctx, "kcycle_lsq", (double)nc * 8 * 16, k_kc_lsq, (nc + 127) / 128, 128, 0, cols, nc, ks);
-}
-
-void launch_kc_lsq1(Ctx& ctx, const int* cols, int nc, double2* ks) {
-  HZ_LAUNCH(ctx, "smooth_lsq", (double)nc * 8 * 16, k_kc_lsq1, (nc + 127) / 128, 128, 0, cols, nc, ks);
-}
-
-template <typename T>
-void launch_kc_combine_add(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const double2* ks,
-                           const cplx<T>* Z0, const cplx<T>* Z1, cplx<T>* X) {
-  const int nblk = kc_nblk(N);
-  HZ_LAUNCH(ctx, "smooth_update", (double)N * nc * 4 * sizeof(cplx<T>), k_kc_combine_add<T>, dim3(nblk, nc), 256, 0,
-            N, ld, cols, ks, Z0, Z1, X);
-}
-
-int kcycle_nblk(long long N) { return kc_nblk(N); }
-
-#define HZ_KC_INST(T)                                                                                                \
-  template void launch_kc_sums<T>(Ctx&, long long, long long, const int*, int, int, int, const cplx<T>*,            \
-                                  const cplx<T>*, const cplx<T>*, double2*, double2*, int);                          \
-  template void launch_kc_update<T>(Ctx&, long long, long long, const int*, int, int, int, double2*, const cplx<T>*, \
-                                    const cplx<T>*, cplx<T>*, double2*, int);                                        \
-  template void launch_kc_scale<T>(Ctx&, long long, long long, const int*, int, const double2*, int, const cplx<T>*, \
-                                   cplx<T>*);                                                                        \
-  template void launch_kc_combine<T>(Ctx&, long long, long long, const int*, int, const double2*, const cplx<T>*,    \
-                                     const cplx<T>*, cplx<T>*);                                                      \
-  template void launch_kc_combine_add<T>(Ctx&, long long, long long, const int*, int, const double2*,                \
-                                         const cplx<T>*, const cplx<T>*, cplx<T>*);
+#define HZ_KC_INST_TB(T, TB)                                                                                           \
+  template void launch_kc_dots<T, TB>(Ctx&, int, long long, long long, const int*, int, const cplx<TB>*,               \
+                                      const cplx<T>*, const cplx<T>*, const KcSums&);                                  \
+  template void launch_kc_finish<T, TB>(Ctx&, int, long long, long long, const int*, int, const cplx<T>*, cplx<T>*,    \
+                                        const cplx<T>*, const cplx<TB>*, const cplx<T>*, const cplx<T>*,               \
+                                        const cplx<T>*, cplx<T>*, const KcSums&);
+#define HZ_KC_INST(T)                                                                                                  \
+  HZ_KC_INST_TB(T, T)                                                                                                  \
+  template void launch_kc_update<T>(Ctx&, long long, long long, const int*, int, const cplx<T>*, cplx<T>*,             \
+                                    const KcSums&);                                                                    \
+  template void launch_kc_last<T>(Ctx&, long long, long long, const int*, int, const cplx<T>*, const cplx<T>*,         \
+                                  const cplx<T>*, const KcSums&);                                                      \
+  template void launch_kc_combine<T>(Ctx&, bool, long long, long long, const int*, int, const cplx<T>*,                \
+                                     const cplx<T>*, const cplx<T>*, cplx<T>*);
 HZ_KC_INST(float)
 HZ_KC_INST(double)
+HZ_KC_INST_TB(float, double)
+HZ_KC_INST_TB(float, df64_tag)
 #undef HZ_KC_INST
+#undef HZ_KC_INST_TB
 
 }  // namespace hz

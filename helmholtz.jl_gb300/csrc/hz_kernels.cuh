@@ -84,11 +84,22 @@ void launch_jacobi0(Ctx& ctx, const Grid& g, const cplx<T>* dinv, int adj, const
 template <typename T>
 void launch_restrict(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<T>* rf, long long ldf, cplx<T>* rc,
                      long long ldc, const int* cols, int ncols);
+// The same of b - y W, y = yt[c*8 + 6].
+template <typename T, typename TB>
+void launch_restrict_diff(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<TB>* b, const cplx<T>* W,
+                          const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols);
 
-// xout = xin + P ec (bi/trilinear nodal prolongation); xin may be null (xout = P ec).
+// A coarse-grid correction: z0, or Y0 z0 + Y1 z1 with the K-cycle's coefficients kt (slots 6, 7).
+template <typename T> struct Correction {
+  const cplx<T>* z0 = nullptr;
+  const cplx<T>* z1 = nullptr;
+  const cplx<T>* kt = nullptr;
+};
+// xout = base + P e (bi/trilinear nodal prolongation); base: nothing (xin null), xin, or
+// y xin with y = yt[c*8 + 6] (yt not null).
 template <typename T>
-void launch_prolong(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<T>* ec, long long ldc, const cplx<T>* xin,
-                    cplx<T>* xout, long long ldf, const int* cols, int ncols);
+void launch_prolong(Ctx& ctx, const Grid& gf, const Grid& gc, const Correction<T>& e, long long ldc,
+                    const cplx<T>* xin, const cplx<T>* yt, cplx<T>* xout, long long ldf, const int* cols, int ncols);
 
 // Coarsest-level direct solve: blocked banded LU (see band_block_operators);
 // T / G are the device copies of the forward / backward block operators.
@@ -139,33 +150,40 @@ void launch_band_solve_df(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cp
                           const int* cols, int ncols, float4* work);
 
 // ---- K-cycle (hz_kcycle.cu) ------------------------------------------------------
-// Two-step FGMRES on a coarse level, per-column scalars ks[c*8 + slot] on the
-// device (0 beta^2, 1 h00, 2 h10^2, 3 h01, 4 h11, 5 h21^2, 6 y0, 7 y1); part
-// holds 3 * ncols * kcycle_nblk(N) partial sums.
-int kcycle_nblk(long long N);
-// slots base.. : conj(V_s) . W for s < nd, then ||W||^2 when want_norm
+// Two-step FGMRES and one-step smoothing on a coarse level; per-column scalars
+// ks[c*8 + slot] (FP64 sums) and kt[c*8 + slot] (cplx<T> coefficients) on the device, partial
+// sums (kcycle_part_bytes) and block counters (one int per column, zeroed once).
+struct KcSums {
+  double2* ks = nullptr;
+  void* kt = nullptr;
+  double* part = nullptr;
+  int* count = nullptr;
+};
+enum KcMode { KC_SMOOTH = 0, KC_FIRST = 1, KC_SECOND = 2 };
+size_t kcycle_part_bytes(long long N, int R);
+// the sums of a mode: KC_SMOOTH y = <W, b> / ||W||^2; KC_FIRST <b, W>, ||b||^2;
+// KC_SECOND <b, W>, <W1, W>
+template <typename T, typename TB>
+void launch_kc_dots(Ctx& ctx, int mode, long long N, long long ld, const int* cols, int nc, const cplx<TB>* B,
+                    const cplx<T>* W1, const cplx<T>* W, const KcSums& s);
+// W -= (<b, W> / ||b||^2) b and its norm
 template <typename T>
-void launch_kc_sums(Ctx& ctx, long long N, long long ld, const int* cols, int nc, int nd, int want_norm,
-                    const cplx<T>* V0, const cplx<T>* V1, const cplx<T>* W, double2* part, double2* ks, int base);
-// W -= sum_{s<nd} ks[hb+s] V_s, ||W||^2 into slot norm_slot
+void launch_kc_update(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const cplx<T>* B, cplx<T>* W,
+                      const KcSums& s);
+// the norm of W2 orthogonalised against b and W1, and the 3x2 least squares -> Y0, Y1
 template <typename T>
-void launch_kc_update(Ctx& ctx, long long N, long long ld, const int* cols, int nc, int nd, int hb, double2* ks,
-                      const cplx<T>* V0, const cplx<T>* V1, cplx<T>* W, double2* part, int norm_slot);
-// Y = X / sqrt(ks[slot])
+void launch_kc_last(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const cplx<T>* B, const cplx<T>* W1,
+                    const cplx<T>* W2, const KcSums& s);
+// X += y Z with y = yt[c*8 + 6]; KC_FIRST / KC_SECOND: also AX = b - R + y W and its sums (KC_SECOND:
+// b is the step's W1 and KB its b)
+template <typename T, typename TB>
+void launch_kc_finish(Ctx& ctx, int mode, long long N, long long ld, const int* cols, int nc, const cplx<T>* yt,
+                      cplx<T>* X, const cplx<T>* Z, const cplx<TB>* B, const cplx<T>* R, const cplx<T>* W,
+                      const cplx<T>* KB, cplx<T>* AX, const KcSums& s);
+// X = Y0 Z0 + Y1 Z1 (add: X +=)
 template <typename T>
-void launch_kc_scale(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const double2* ks, int slot,
-                     const cplx<T>* X, cplx<T>* Y);
-// X = y0 Z0 + y1 Z1
-template <typename T>
-void launch_kc_combine(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const double2* ks,
+void launch_kc_combine(Ctx& ctx, bool add, long long N, long long ld, const int* cols, int nc, const cplx<T>* kt,
                        const cplx<T>* Z0, const cplx<T>* Z1, cplx<T>* X);
-// the 3x2 least-squares problem of each column -> y0, y1
-void launch_kc_lsq(Ctx& ctx, const int* cols, int nc, double2* ks);
-// one-step least squares (y0 from slots 0-2, y1 = 0) and X += y0 Z0 + y1 Z1 (GMRES smoothing)
-void launch_kc_lsq1(Ctx& ctx, const int* cols, int nc, double2* ks);
-template <typename T>
-void launch_kc_combine_add(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const double2* ks,
-                           const cplx<T>* Z0, const cplx<T>* Z1, cplx<T>* X);
 
 // ---- setup kernels ---------------------------------------------------------
 // Fine-level diagonals on the device from nodal m and gamma (device arrays):

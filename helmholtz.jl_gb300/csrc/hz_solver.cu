@@ -111,11 +111,11 @@ struct Level {
   std::vector<double> m, gamma;              // restricted nodal m and shifted gamma (host)
   // work buffers (precision of the cycle): x/t ping-pong, r residual, b right-hand side
   DBuf x, t, r, b;
-  // K-cycle on this level: V0, V1, Z0, Z1, W blocks, per-column scalars, partial sums
-  DBuf kv, ks, kp;
-  // GMRES smoothing ("Jac-GMRES") on this level: the same layout, own storage (the
-  // smoother runs inside the K-cycle's cycles on the same level)
-  DBuf gv, gs, gp;
+  // K-cycle on this level: W1, W2, Z0, Z1 blocks, per-column scalars, partial sums, block counters
+  DBuf kv, ks, kp, kn;
+  // GMRES smoothing ("Jac-GMRES") on this level: R, Z0, W (and Z1, W2 for two steps) and
+  // own scalars (the smoother runs inside the K-cycle's cycles on the same level)
+  DBuf gv, gs, gp, gn;
 };
 
 struct Hierarchy {
@@ -610,7 +610,8 @@ void build_hierarchy(hz_handle* h, int adj) {
     pf.alloc((size_t)ns * Nf * 16);
     pg.alloc((size_t)ns * Nf * 16);
     launch_probe_init(h->ctx, C->g, dim, pin.as<double2>(), Nc);
-    launch_prolong<double>(h->ctx, F.g, C->g, pin.as<double2>(), Nc, nullptr, pf.as<double2>(), Nf, pc, ns);
+    launch_prolong<double>(h->ctx, F.g, C->g, Correction<double>{pin.as<double2>()}, Nc, nullptr, nullptr,
+                           pf.as<double2>(), Nf, pc, ns);
     if (l == 0)
       launch_fine<double, double, double>(h->ctx, MODE_APPLY, fop, h->diagSH.as<double2>(), nullptr,
                                           pf.as<double2>(), (const double2*)nullptr, pg.as<double2>(), Nf, pc, ns,
@@ -687,6 +688,20 @@ void ensure_workspace(hz_handle* h, int nrhs) {
   h->mcap = m;
 }
 
+// Scalars, partial sums and (zeroed) block counters of a level's K-cycle or smoother.
+void alloc_sums(hz_handle* h, long long N, int R, DBuf& ks, DBuf& part, DBuf& count) {
+  ks.alloc((size_t)R * 8 * 16 * 2);  // sums and coefficients
+  part.alloc(kcycle_part_bytes(N, R));
+  const size_t b = (size_t)R * sizeof(int);
+  if (b > count.bytes) {
+    count.alloc(b);
+    ck(cudaMemsetAsync(count.p, 0, b, h->ctx.stream), "zero block counters");
+  }
+}
+KcSums sums_of(const DBuf& ks, const DBuf& part, const DBuf& count) {
+  return KcSums{ks.as<double2>(), (char*)ks.p + ks.bytes / 2, part.as<double>(), count.as<int>()};
+}
+
 template <typename T>
 void ensure_level_buffers(hz_handle* h, Hierarchy& H, int R) {
   const size_t es = sizeof(cplx<T>);
@@ -702,14 +717,12 @@ void ensure_level_buffers(hz_handle* h, Hierarchy& H, int R) {
       L.r.alloc(bytes);
     }
     if (h->opt.cycle == 'K' && l > 0 && l + 1 < H.lv.size()) {
-      L.kv.alloc(5 * bytes);
-      L.ks.alloc((size_t)R * 8 * 16);
-      L.kp.alloc((size_t)R * 3 * kcycle_nblk(L.g.N) * 16);
+      L.kv.alloc(4 * bytes);
+      alloc_sums(h, L.g.N, R, L.ks, L.kp, L.kn);
     }
     if (h->opt.relax_type == HZ_RELAX_JAC_GMRES && (int)l >= h->opt.relax_from && l + 1 < H.lv.size()) {
-      L.gv.alloc(5 * bytes);
-      L.gs.alloc((size_t)R * 8 * 16);
-      L.gp.alloc((size_t)R * 3 * kcycle_nblk(L.g.N) * 16);
+      L.gv.alloc((std::max(h->opt.relax_pre, h->opt.relax_post) > 1 ? 5 : 3) * bytes);
+      alloc_sums(h, L.g.N, R, L.gs, L.gp, L.gn);
     }
   }
   // digits of the right-hand sides, or 3 vectors per column of the band solve
@@ -808,51 +821,57 @@ void learned_correction(hz_handle* h, Hierarchy& H, int l, const cplx<T>* b, cpl
   h->net_calls += 1;
 }
 
-template <typename T, typename TB>
-void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out, const int* cols, int nc);
+// The product A Z a K step needs after its cycle, and its sums: a cycle that ends with a
+// one-step GMRES smoothing has A Z at hand and provides both (done).
+template <typename T> struct KStep {
+  int mode;           // KC_FIRST or KC_SECOND
+  const cplx<T>* b;   // the K-cycle's right-hand side
+  const cplx<T>* W1;  // the second step's
+  cplx<T>* W;         // A Z
+  KcSums sums;
+  bool done = false;
+};
 
-// The preconditioner of a K-cycle step on level k: the level's own cycle, or
-// the network when it is attached to level k (it then stands for everything
-// below level k - 1 that the cycle would do: smoothing on level k and the
-// recursion to the coarsest LU).
+template <typename T, typename TB>
+void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out, const int* cols, int nc,
+              KStep<T>* step = nullptr);
+
+// The preconditioner of a K-cycle step on level k (the level's own cycle, or
+// the network when it is attached to level k: it then stands for everything
+// below level k - 1 that the cycle would do, smoothing on level k and the
+// recursion to the coarsest LU), the operator product and its sums.
 template <typename T>
-void kcycle_precondition(hz_handle* h, Hierarchy& H, int k, const cplx<T>* v, cplx<T>* z, const int* cols, int nc) {
+void kcycle_precondition(hz_handle* h, Hierarchy& H, int k, const cplx<T>* v, cplx<T>* z, KStep<T>& step,
+                         const int* cols, int nc) {
+  Level& L = *H.lv[k];
+  const cplx<T>* none = nullptr;
   if (h->net_active && k == h->net_level)
     learned_correction<T>(h, H, k, v, z, cols, nc);
   else
-    mg_cycle<T, T>(h, H, k, v, z, cols, nc);
+    mg_cycle<T, T>(h, H, k, v, z, cols, nc, &step);
+  if (step.done) return;
+  lev_op<T, T>(h, H, k, MODE_APPLY, z, none, step.W, cols, nc);
+  launch_kc_dots<T, T>(h->ctx, step.mode, L.g.N, L.ld, cols, nc, step.b, step.W1, step.W, step.sums);
 }
 
-// out = e_k for the active columns of b_k by the K-cycle: two FGMRES steps on
+// The K-cycle on level k for the active columns of b_k: two FGMRES steps on
 // level k's operator, right-preconditioned by level k's own cycle (zero
-// initial guess; Multigrid.jl cycleType 'K').
+// initial guess; Multigrid.jl cycleType 'K').  The correction is Y0 Z0 + Y1 Z1.
 template <typename T>
-void kcycle_correction(hz_handle* h, Hierarchy& H, int k, const cplx<T>* b, cplx<T>* out, const int* cols, int nc) {
+Correction<T> kcycle_steps(hz_handle* h, Hierarchy& H, int k, const cplx<T>* b, const int* cols, int nc) {
   Level& L = *H.lv[k];
-  Ctx& c = h->ctx;
   const long long N = L.g.N, ld = L.ld, vs = (long long)h->rcap * ld;
-  cplx<T>* base = L.kv.as<cplx<T>>();
-  cplx<T>* V0 = base;
-  cplx<T>* V1 = base + vs;
-  cplx<T>* Z0 = base + 2 * vs;
-  cplx<T>* Z1 = base + 3 * vs;
-  cplx<T>* W = base + 4 * vs;
-  double2* ks = L.ks.as<double2>();
-  double2* part = L.kp.as<double2>();
-  const cplx<T>* none = nullptr;
-  launch_kc_sums<T>(c, N, ld, cols, nc, 0, 1, none, none, b, part, ks, 0);  // beta^2
-  launch_kc_scale<T>(c, N, ld, cols, nc, ks, 0, b, V0);
-  kcycle_precondition<T>(h, H, k, V0, Z0, cols, nc);
-  lev_op<T, T>(h, H, k, MODE_APPLY, Z0, none, W, cols, nc);
-  launch_kc_sums<T>(c, N, ld, cols, nc, 1, 0, V0, none, W, part, ks, 1);  // h00
-  launch_kc_update<T>(c, N, ld, cols, nc, 1, 1, ks, V0, none, W, part, 2);  // W -= h00 V0, h10^2
-  launch_kc_scale<T>(c, N, ld, cols, nc, ks, 2, W, V1);
-  kcycle_precondition<T>(h, H, k, V1, Z1, cols, nc);
-  lev_op<T, T>(h, H, k, MODE_APPLY, Z1, none, W, cols, nc);
-  launch_kc_sums<T>(c, N, ld, cols, nc, 2, 0, V0, V1, W, part, ks, 3);  // h01, h11
-  launch_kc_update<T>(c, N, ld, cols, nc, 2, 3, ks, V0, V1, W, part, 5);  // h21^2
-  launch_kc_lsq(c, cols, nc, ks);
-  launch_kc_combine<T>(c, N, ld, cols, nc, ks, Z0, Z1, out);
+  cplx<T>* W1 = L.kv.as<cplx<T>>();
+  cplx<T>* W2 = W1 + vs;
+  cplx<T>* Z0 = W1 + 2 * vs;
+  cplx<T>* Z1 = W1 + 3 * vs;
+  const KcSums s = sums_of(L.ks, L.kp, L.kn);
+  KStep<T> first{KC_FIRST, b, nullptr, W1, s}, second{KC_SECOND, b, W1, W2, s};
+  kcycle_precondition<T>(h, H, k, b, Z0, first, cols, nc);
+  launch_kc_update<T>(h->ctx, N, ld, cols, nc, b, W1, s);
+  kcycle_precondition<T>(h, H, k, W1, Z1, second, cols, nc);
+  launch_kc_last<T>(h->ctx, N, ld, cols, nc, b, W1, W2, s);
+  return Correction<T>{Z0, Z1, (const cplx<T>*)s.kt};
 }
 
 // Record the right-hand sides handed to the capture level (FP64 cycles only).
@@ -866,67 +885,66 @@ void capture_rhs(hz_handle* h, Level& L, const cplx<TB>* b, const int* cols, int
   }
 }
 
-// x += the relaxType "Jac-GMRES" smoothing step on level l: `steps` (1 or 2)
-// Arnoldi steps of GMRES on the level's operator from the current x,
-// right-preconditioned by one damped-Jacobi sweep (Z_j = w D^-1 V_j), and the
-// least-squares update x += sum_j y_j Z_j per column.  The K-cycle's kernels
-// with the smoother's own buffers; a column with zero residual is unchanged.
+// One GMRES step's direction on level l for the residual r (relaxType "Jac-GMRES":
+// GMRES on the level's operator right-preconditioned by one damped-Jacobi sweep):
+// Z = w D^-1 r, W = A Z and y = <W, r> / ||W||^2 (0 for a zero residual) in slot 6 of the
+// smoother's coefficients.
+template <typename T, typename TR>
+void smooth_direction(hz_handle* h, Hierarchy& H, int l, const cplx<TR>* r, cplx<T>* Z, cplx<T>* W, const int* cols,
+                      int nc) {
+  Level& L = *H.lv[l];
+  const cplx<T>* none = nullptr;
+  lev_jacobi0<T, TR>(h, H, l, r, Z, cols, nc);
+  lev_op<T, T>(h, H, l, MODE_APPLY, Z, none, W, cols, nc);
+  launch_kc_dots<T, TR>(h->ctx, KC_SMOOTH, L.g.N, L.ld, cols, nc, r, none, W, sums_of(L.gs, L.gp, L.gn));
+}
+
+// x += two such steps from the current x: the K-cycle's kernels with the Jacobi sweep as
+// preconditioner.
 template <typename T, typename TB>
-void gmres_smooth(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* x, const int* cols, int nc,
-                  int steps) {
+void smooth_two_steps(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* x, const int* cols, int nc) {
   Level& L = *H.lv[l];
   Ctx& c = h->ctx;
   const long long N = L.g.N, ld = L.ld, vs = (long long)h->rcap * ld;
-  cplx<T>* base = L.gv.as<cplx<T>>();
-  if (!base || !L.gs.p || !L.gp.p) fail(HZ_ERR_STATE, "internal: GMRES smoothing buffers missing on level %d", l);
-  cplx<T>* V0 = base;
-  cplx<T>* V1 = base + vs;
-  cplx<T>* Z0 = base + 2 * vs;
-  cplx<T>* Z1 = base + 3 * vs;
-  cplx<T>* W = base + 4 * vs;
-  double2* ks = L.gs.as<double2>();
-  double2* part = L.gp.as<double2>();
+  cplx<T>* R = L.gv.as<cplx<T>>();
+  cplx<T>*Z0 = R + vs, *W1 = R + 2 * vs, *Z1 = R + 3 * vs, *W2 = R + 4 * vs;
+  const KcSums s = sums_of(L.gs, L.gp, L.gn);
   const cplx<T>* none = nullptr;
-  lev_op<T, TB>(h, H, l, MODE_RESID, x, b, W, cols, nc);                    // W = b - A x
-  launch_kc_sums<T>(c, N, ld, cols, nc, 0, 1, none, none, W, part, ks, 0);  // beta^2
-  launch_kc_scale<T>(c, N, ld, cols, nc, ks, 0, W, V0);
-  lev_jacobi0<T, T>(h, H, l, V0, Z0, cols, nc);                              // Z0 = w D^-1 V0
-  lev_op<T, T>(h, H, l, MODE_APPLY, Z0, none, W, cols, nc);
-  launch_kc_sums<T>(c, N, ld, cols, nc, 1, 0, V0, none, W, part, ks, 1);     // h00
-  launch_kc_update<T>(c, N, ld, cols, nc, 1, 1, ks, V0, none, W, part, 2);   // W -= h00 V0, h10^2
-  if (steps == 1) {
-    launch_kc_lsq1(c, cols, nc, ks);
-    launch_kc_combine_add<T>(c, N, ld, cols, nc, ks, Z0, Z0, x);  // y1 = 0
-    return;
-  }
-  launch_kc_scale<T>(c, N, ld, cols, nc, ks, 2, W, V1);
-  lev_jacobi0<T, T>(h, H, l, V1, Z1, cols, nc);                              // Z1 = w D^-1 V1
-  lev_op<T, T>(h, H, l, MODE_APPLY, Z1, none, W, cols, nc);
-  launch_kc_sums<T>(c, N, ld, cols, nc, 2, 0, V0, V1, W, part, ks, 3);       // h01, h11
-  launch_kc_update<T>(c, N, ld, cols, nc, 2, 3, ks, V0, V1, W, part, 5);     // h21^2
-  launch_kc_lsq(c, cols, nc, ks);
-  launch_kc_combine_add<T>(c, N, ld, cols, nc, ks, Z0, Z1, x);
+  lev_op<T, TB>(h, H, l, MODE_RESID, x, b, R, cols, nc);
+  lev_jacobi0<T, T>(h, H, l, R, Z0, cols, nc);
+  lev_op<T, T>(h, H, l, MODE_APPLY, Z0, none, W1, cols, nc);
+  launch_kc_dots<T, T>(c, KC_FIRST, N, ld, cols, nc, R, none, W1, s);
+  launch_kc_update<T>(c, N, ld, cols, nc, R, W1, s);
+  lev_jacobi0<T, T>(h, H, l, W1, Z1, cols, nc);
+  lev_op<T, T>(h, H, l, MODE_APPLY, Z1, none, W2, cols, nc);
+  launch_kc_dots<T, T>(c, KC_SECOND, N, ld, cols, nc, R, W1, W2, s);
+  launch_kc_last<T>(c, N, ld, cols, nc, R, W1, W2, s);
+  launch_kc_combine<T>(c, true, N, ld, cols, nc, (const cplx<T>*)s.kt, Z0, Z1, x);
 }
 
-// C.x = the coarse-grid correction of level l + 1 for the right-hand sides in C.b:
+// The coarse-grid correction of level l for the right-hand sides in C.b of level l + 1:
 // the network, a K-cycle step or a recursive cycle.
 template <typename T>
-void coarse_correction(hz_handle* h, Hierarchy& H, int l, const int* cols, int nc) {
+Correction<T> coarse_correction(hz_handle* h, Hierarchy& H, int l, const int* cols, int nc) {
   Level& C = *H.lv[l + 1];
   const int last = (int)H.lv.size() - 1;
+  const cplx<T>* b = C.b.as<cplx<T>>();
+  cplx<T>* x = C.x.as<cplx<T>>();
   // K-cycle: the network preconditions the two FGMRES steps on its level
   // (kcycle_precondition); V and W cycles: it replaces the level's cycle
   if (h->net_active && l + 1 == h->net_level && !(h->opt.cycle == 'K' && l + 1 < last))
-    learned_correction<T>(h, H, l + 1, C.b.as<cplx<T>>(), C.x.as<cplx<T>>(), cols, nc);
+    learned_correction<T>(h, H, l + 1, b, x, cols, nc);
   else if (h->opt.cycle == 'K' && l + 1 < last)
-    kcycle_correction<T>(h, H, l + 1, C.b.as<cplx<T>>(), C.x.as<cplx<T>>(), cols, nc);
+    return kcycle_steps<T>(h, H, l + 1, b, cols, nc);
   else
-    mg_cycle<T, T>(h, H, l + 1, C.b.as<cplx<T>>(), C.x.as<cplx<T>>(), cols, nc);
+    mg_cycle<T, T>(h, H, l + 1, b, x, cols, nc);
+  return Correction<T>{x};
 }
 
 // x_out = cycle(b) on level l with zero initial guess.
 template <typename T, typename TB>
-void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out, const int* cols, int nc) {
+void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out, const int* cols, int nc,
+              KStep<T>* step) {
   Level& L = *H.lv[l];
   const int last = (int)H.lv.size() - 1;
   if (h->cap_on && l == h->cap_level) capture_rhs<TB>(h, L, b, cols, nc);
@@ -959,15 +977,46 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
   const int ncalls = (h->opt.cycle == 'W' && l + 1 < last) ? 2 : 1;
   if (h->opt.relax_type == HZ_RELAX_JAC_GMRES && l >= h->opt.relax_from) {
     // relaxType "Jac-GMRES": smoothing steps update `out` in place
-    launch_zero_cols<T>(h->ctx, L.g.N, out, L.ld, cols, nc);
-    if (pre > 0) gmres_smooth<T, TB>(h, H, l, b, out, cols, nc, pre);
+    const long long vs = (long long)h->rcap * L.ld;
+    cplx<T>* R = L.gv.as<cplx<T>>();
+    cplx<T>*Z = R + vs, *W = R + 2 * vs;
+    if (!R) fail(HZ_ERR_STATE, "internal: GMRES smoothing buffers missing on level %d", l);
+    const KcSums s = sums_of(L.gs, L.gp, L.gn);
     for (int call = 0; call < ncalls; ++call) {
-      lev_op<T, TB>(h, H, l, MODE_RESID, out, b, rb, cols, nc);
-      launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
-      coarse_correction<T>(h, H, l, cols, nc);
-      launch_prolong<T>(h->ctx, L.g, C.g, C.x.as<cplx<T>>(), C.ld, out, out, L.ld, cols, nc);
+      const cplx<T>* base = out;     // what the correction is added to
+      const cplx<T>* yt = nullptr;   // and its factor
+      if (call == 0 && pre == 0) {
+        launch_cast_cols<T, TB>(h->ctx, L.g.N, b, L.ld, rb, L.ld, cols, nc);
+        base = nullptr;
+      } else if (call == 0 && pre == 1) {
+        smooth_direction<T, TB>(h, H, l, b, Z, W, cols, nc);  // x = y Z, b - A x = b - y W
+        base = Z;
+        yt = (const cplx<T>*)s.kt;
+      } else {
+        if (call == 0) {
+          launch_zero_cols<T>(h->ctx, L.g.N, out, L.ld, cols, nc);
+          smooth_two_steps<T, TB>(h, H, l, b, out, cols, nc);
+        }
+        lev_op<T, TB>(h, H, l, MODE_RESID, out, b, rb, cols, nc);
+      }
+      if (yt)
+        launch_restrict_diff<T, TB>(h->ctx, L.g, C.g, b, W, yt, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
+      else
+        launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
+      const Correction<T> e = coarse_correction<T>(h, H, l, cols, nc);
+      launch_prolong<T>(h->ctx, L.g, C.g, e, C.ld, base, yt, out, L.ld, cols, nc);
     }
-    if (post > 0) gmres_smooth<T, TB>(h, H, l, b, out, cols, nc, post);
+    if (post == 1) {
+      const bool k = step != nullptr;
+      lev_op<T, TB>(h, H, l, MODE_RESID, out, b, R, cols, nc);
+      smooth_direction<T, T>(h, H, l, R, Z, W, cols, nc);
+      launch_kc_finish<T, TB>(h->ctx, k ? step->mode : KC_SMOOTH, L.g.N, L.ld, cols, nc,
+                              (const cplx<T>*)s.kt, out, Z, b, R, W,
+                              k ? step->b : nullptr, k ? step->W : nullptr, k ? step->sums : KcSums());
+      if (k) step->done = true;
+    } else if (post == 2) {
+      smooth_two_steps<T, TB>(h, H, l, b, out, cols, nc);
+    }
     return;
   }
   bool zero_guess = true;
@@ -992,8 +1041,8 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
       lev_op<T, TB>(h, H, l, MODE_RESID, cur, b, rb, cols, nc);
       launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
     }
-    coarse_correction<T>(h, H, l, cols, nc);
-    launch_prolong<T>(h->ctx, L.g, C.g, C.x.as<cplx<T>>(), C.ld, zero_guess ? nullptr : cur, cur, L.ld, cols, nc);
+    const Correction<T> e = coarse_correction<T>(h, H, l, cols, nc);
+    launch_prolong<T>(h->ctx, L.g, C.g, e, C.ld, zero_guess ? nullptr : cur, nullptr, cur, L.ld, cols, nc);
     zero_guess = false;
   }
   for (int s = 0; s < post; ++s) {
@@ -2450,9 +2499,8 @@ void collect_targets_iterative(hz_handle* h, Hierarchy& H, int level, int sweeps
   if (level >= last) sweeps = 1;
   Level& Lv = *H.lv[level];
   if (sweeps > 1 && !Lv.kv.p) {  // the two-step corrections' vectors (allocated by the K-cycle itself otherwise)
-    Lv.kv.alloc((size_t)5 * R * Lv.ld * sizeof(double2));
-    Lv.ks.alloc((size_t)R * 8 * 16);
-    Lv.kp.alloc((size_t)R * 3 * kcycle_nblk(Lv.g.N) * 16);
+    Lv.kv.alloc((size_t)4 * R * Lv.ld * sizeof(double2));
+    alloc_sums(h, Lv.g.N, R, Lv.ks, Lv.kp, Lv.kn);
   }
   DBuf xe, res, ev, x1, idc, sc, nrm;
   xe.alloc((size_t)R * N * 16);
@@ -2478,7 +2526,8 @@ void collect_targets_iterative(hz_handle* h, Hierarchy& H, int level, int sweeps
     ck(cudaMemcpyAsync(xd, x1.p, (size_t)k * N * 16, cudaMemcpyDeviceToDevice, h->ctx.stream), "first sweep");
     for (int s = 1; s < sweeps; ++s) {
       lev_op<double, double>(h, H, level, MODE_RESID, xd, r, res.as<double2>(), dc, k);
-      kcycle_correction<double>(h, H, level, res.as<double2>(), ev.as<double2>(), dc, k);
+      const Correction<double> e = kcycle_steps<double>(h, H, level, res.as<double2>(), dc, k);
+      launch_kc_combine<double>(h->ctx, false, N, Lv.ld, dc, k, e.kt, e.z0, e.z1, ev.as<double2>());
       launch_axpy_compact(h->ctx, N, k, ev.as<double2>(), xd);
     }
     lev_op<double, double>(h, H, level, MODE_RESID, xd, r, res.as<double2>(), dc, k);

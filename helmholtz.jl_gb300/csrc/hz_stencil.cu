@@ -405,10 +405,12 @@ void launch_jacobi0(Ctx& ctx, const Grid& g, const cplx<T>* dinv, int adj, const
 // ---------------------------------------------------------------------------
 // Transfers
 // ---------------------------------------------------------------------------
-template <typename T, bool IS3D>
-__global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<T>* __restrict__ rf, long long ldf,
-                                                  cplx<T>* __restrict__ rc, long long ldc, const int* __restrict__ cols,
-                                                  int ncols, int cpb) {
+// DIFF: the fine vector is rf - y W (a smoothing step from zero leaves that residual)
+template <typename T, typename TB, bool IS3D, bool DIFF>
+__global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<TB>* __restrict__ rf,
+                                                  const cplx<T>* __restrict__ W, const cplx<T>* __restrict__ yt,
+                                                  long long ldf, cplx<T>* __restrict__ rc, long long ldc,
+                                                  const int* __restrict__ cols, int ncols, int cpb) {
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= gc.N) return;
   const int I = (int)(q % gc.nx);
@@ -440,7 +442,9 @@ __global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<T
 #pragma unroll 4
   for (int ci = c0; ci < c1; ++ci) {
     const int col = cols[ci];
-    const cplx<T>* r = rf + (long long)col * ldf + pc;
+    const cplx<TB>* r = rf + (long long)col * ldf + pc;
+    const cplx<T>* wc = DIFF ? W + (long long)col * ldf + pc : nullptr;
+    const cplx<T> y = DIFF ? yt[col * 8 + 6] : mk<T>(0, 0);
     T ar = 0, ai = 0;
 #pragma unroll
     for (int c = 0; c < (IS3D ? 3 : 1); ++c) {
@@ -449,7 +453,9 @@ __global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<T
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           const T wgt = wx[a] * wy[bq] * (IS3D ? wz[c] : T(1));
-          const cplx<T> v = r[ox[a] + oy[bq] + (IS3D ? oz[c] : 0LL)];
+          const long long o = ox[a] + oy[bq] + (IS3D ? oz[c] : 0LL);
+          cplx<T> v = mk<T>((T)r[o].x, (T)r[o].y);
+          if (DIFF) v = cfms<T>(y, wc[o], v);
           ar += wgt * v.x;
           ai += wgt * v.y;
         }
@@ -459,26 +465,45 @@ __global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<T
   }
 }
 
-template <typename T>
-void launch_restrict(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<T>* rf, long long ldf, cplx<T>* rc,
-                     long long ldc, const int* cols, int ncols) {
+template <typename T, typename TB, bool DIFF>
+static void restrict_any(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<TB>* rf, const cplx<T>* W,
+                         const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols) {
   if (ncols <= 0) return;
   const int TPB = 256;
   long long nbx = (gc.N + TPB - 1) / TPB;
   int ch = chunks_for(nbx, ncols);
   int cpb = (ncols + ch - 1) / ch;
   dim3 grid((unsigned)nbx, (unsigned)ch);
-  const double tbytes = (double)ncols * (gf.N + gc.N) * sizeof(cplx<T>);
+  const double tbytes =
+      (double)ncols * (gf.N * (sizeof(cplx<TB>) + (DIFF ? sizeof(cplx<T>) : 0)) + gc.N * sizeof(cplx<T>));
   if (gf.nz > 1)
-    HZ_LAUNCH(ctx, "restrict", tbytes, (k_restrict<T, true>), grid, TPB, 0, gf, gc, rf, ldf, rc, ldc, cols, ncols, cpb);
+    HZ_LAUNCH(ctx, "restrict", tbytes, (k_restrict<T, TB, true, DIFF>), grid, TPB, 0, gf, gc, rf, W, yt, ldf, rc, ldc,
+              cols, ncols, cpb);
   else
-    HZ_LAUNCH(ctx, "restrict", tbytes, (k_restrict<T, false>), grid, TPB, 0, gf, gc, rf, ldf, rc, ldc, cols, ncols, cpb);
+    HZ_LAUNCH(ctx, "restrict", tbytes, (k_restrict<T, TB, false, DIFF>), grid, TPB, 0, gf, gc, rf, W, yt, ldf, rc, ldc,
+              cols, ncols, cpb);
 }
 
-template <typename T, bool IS3D>
-__global__ void __launch_bounds__(256) k_prolong(Grid gf, Grid gc, const cplx<T>* __restrict__ ec, long long ldc,
-                                                 const cplx<T>* xin, cplx<T>* xout, long long ldf,
-                                                 const int* __restrict__ cols, int ncols, int cpb) {
+template <typename T>
+void launch_restrict(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<T>* rf, long long ldf, cplx<T>* rc,
+                     long long ldc, const int* cols, int ncols) {
+  restrict_any<T, T, false>(ctx, gf, gc, rf, (const cplx<T>*)nullptr, nullptr, ldf, rc, ldc, cols, ncols);
+}
+
+template <typename T, typename TB>
+void launch_restrict_diff(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<TB>* b, const cplx<T>* W,
+                          const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols) {
+  restrict_any<T, TB, true>(ctx, gf, gc, b, W, yt, ldf, rc, ldc, cols, ncols);
+}
+
+// COMB: the coarse vector is Y0 e0 + Y1 e1 (a K-cycle correction, formed here instead of
+// in a pass of its own).  xin null: base 0; yt: base y xin.
+template <typename T, bool IS3D, bool COMB>
+__global__ void __launch_bounds__(256) k_prolong(Grid gf, Grid gc, const cplx<T>* __restrict__ ec0,
+                                                 const cplx<T>* __restrict__ ec1, const cplx<T>* __restrict__ kt,
+                                                 long long ldc, const cplx<T>* xin, const cplx<T>* __restrict__ yt,
+                                                 cplx<T>* xout, long long ldf, const int* __restrict__ cols, int ncols,
+                                                 int cpb) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= gf.N) return;
   const int i = (int)(p % gf.nx);
@@ -499,36 +524,48 @@ __global__ void __launch_bounds__(256) k_prolong(Grid gf, Grid gc, const cplx<T>
 #pragma unroll 4
   for (int ci = c0; ci < c1; ++ci) {
     const int col = cols[ci];
-    const cplx<T>* e = ec + (long long)col * ldc;
-    cplx<T> v0 = e[z0 + b0 + a0], v1 = e[z0 + b0 + a1], v2 = e[z0 + b1 + a0], v3 = e[z0 + b1 + a1];
+    const cplx<T>* e0 = ec0 + (long long)col * ldc;
+    const cplx<T>* e1 = COMB ? ec1 + (long long)col * ldc : nullptr;
+    const cplx<T> y0 = COMB ? kt[col * 8 + 6] : mk<T>(0, 0);
+    const cplx<T> y1 = COMB ? kt[col * 8 + 7] : mk<T>(0, 0);
+    auto e = [&](long long q) { return COMB ? cfma<T>(y1, e1[q], cmul<T>(y0, e0[q])) : e0[q]; };
+    const cplx<T> v0 = e(z0 + b0 + a0), v1 = e(z0 + b0 + a1), v2 = e(z0 + b1 + a0), v3 = e(z0 + b1 + a1);
     T ar = (v0.x + v1.x) + (v2.x + v3.x);
     T ai = (v0.y + v1.y) + (v2.y + v3.y);
     if (IS3D) {
-      cplx<T> u0 = e[z1 + b0 + a0], u1 = e[z1 + b0 + a1], u2 = e[z1 + b1 + a0], u3 = e[z1 + b1 + a1];
+      const cplx<T> u0 = e(z1 + b0 + a0), u1 = e(z1 + b0 + a1), u2 = e(z1 + b1 + a0), u3 = e(z1 + b1 + a1);
       ar += (u0.x + u1.x) + (u2.x + u3.x);
       ai += (u0.y + u1.y) + (u2.y + u3.y);
     }
     const long long o = (long long)col * ldf + p;
     // the fine vector is read and written once (streaming); the coarse one stays cached
-    const cplx<T> base = xin ? __ldcs(&xin[o]) : mk<T>(0, 0);
+    cplx<T> base = xin ? __ldcs(&xin[o]) : mk<T>(0, 0);
+    if (yt) base = cmul<T>(yt[col * 8 + 6], base);
     __stcs(&xout[o], mk<T>(base.x + wgt * ar, base.y + wgt * ai));
   }
 }
 
 template <typename T>
-void launch_prolong(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<T>* ec, long long ldc, const cplx<T>* xin,
-                    cplx<T>* xout, long long ldf, const int* cols, int ncols) {
+void launch_prolong(Ctx& ctx, const Grid& gf, const Grid& gc, const Correction<T>& e, long long ldc,
+                    const cplx<T>* xin, const cplx<T>* yt, cplx<T>* xout, long long ldf, const int* cols, int ncols) {
   if (ncols <= 0) return;
   const int TPB = 256;
   long long nbx = (gf.N + TPB - 1) / TPB;
   int ch = chunks_for(nbx, ncols);
   int cpb = (ncols + ch - 1) / ch;
   dim3 grid((unsigned)nbx, (unsigned)ch);
-  const double pbytes = (double)ncols * (gc.N + (xin ? 2 : 1) * gf.N) * sizeof(cplx<T>);
-  if (gf.nz > 1)
-    HZ_LAUNCH(ctx, "prolong", pbytes, (k_prolong<T, true>), grid, TPB, 0, gf, gc, ec, ldc, xin, xout, ldf, cols, ncols, cpb);
-  else
-    HZ_LAUNCH(ctx, "prolong", pbytes, (k_prolong<T, false>), grid, TPB, 0, gf, gc, ec, ldc, xin, xout, ldf, cols, ncols, cpb);
+  const double pbytes = (double)ncols * ((e.z1 ? 2 : 1) * gc.N + (xin ? 2 : 1) * gf.N) * sizeof(cplx<T>);
+#define HZ_PROLONG(D, C)                                                                                           \
+  HZ_LAUNCH(ctx, "prolong", pbytes, (k_prolong<T, D, C>), grid, TPB, 0, gf, gc, e.z0, e.z1, e.kt, ldc, xin, yt, xout, \
+            ldf, cols, ncols, cpb)
+  if (gf.nz > 1) {
+    if (e.z1) HZ_PROLONG(true, true);
+    else HZ_PROLONG(true, false);
+  } else {
+    if (e.z1) HZ_PROLONG(false, true);
+    else HZ_PROLONG(false, false);
+  }
+#undef HZ_PROLONG
 }
 
 // ---------------------------------------------------------------------------
@@ -1020,10 +1057,18 @@ template void launch_restrict<double>(Ctx&, const Grid&, const Grid&, const doub
                                       const int*, int);
 template void launch_restrict<float>(Ctx&, const Grid&, const Grid&, const float2*, long long, float2*, long long,
                                      const int*, int);
-template void launch_prolong<double>(Ctx&, const Grid&, const Grid&, const double2*, long long, const double2*,
-                                     double2*, long long, const int*, int);
-template void launch_prolong<float>(Ctx&, const Grid&, const Grid&, const float2*, long long, const float2*, float2*,
-                                    long long, const int*, int);
+#define HZ_INST_RD(T, TB)                                                                                       \
+  template void launch_restrict_diff<T, TB>(Ctx&, const Grid&, const Grid&, const cplx<TB>*, const cplx<T>*,     \
+                                            const cplx<T>*, long long, cplx<T>*, long long, const int*, int);
+HZ_INST_RD(double, double)
+HZ_INST_RD(float, float)
+HZ_INST_RD(float, double)
+HZ_INST_RD(float, df64_tag)
+#undef HZ_INST_RD
+template void launch_prolong<double>(Ctx&, const Grid&, const Grid&, const Correction<double>&, long long,
+                                     const double2*, const double2*, double2*, long long, const int*, int);
+template void launch_prolong<float>(Ctx&, const Grid&, const Grid&, const Correction<float>&, long long, const float2*,
+                                    const float2*, float2*, long long, const int*, int);
 template void launch_band_solve<double>(Ctx&, const BandSolveOps&, const double2*, double2*, long long, const int*, int,
                                         double2*);
 template void launch_band_solve<float>(Ctx&, const BandSolveOps&, const float2*, float2*, long long, const int*, int,

@@ -12,6 +12,7 @@
 
 #include <cooperative_groups.h>
 
+#include "hz_gs.cuh"
 #include "hz_launch.cuh"
 
 namespace cg = cooperative_groups;
@@ -207,66 +208,21 @@ template void launch_fine_df64<double2>(Ctx&, const FineOp&, const float4*, cons
 static constexpr int RT = 256;
 static constexpr int KG = 16;
 
-template <int NV>
-__device__ __forceinline__ void block_reduce_df(const double2 (&v)[NV], int nv, double nrm, int want_norm,
-                                                double2* part, int nblk) {
-  __shared__ double2 red[RT / 32][NV + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int s = 0; s < NV; ++s) {
-    if (s < nv) {
-      double a = v[s].x, b = v[s].y;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-      }
-      if (lane == 0) red[warp][s] = mk<double>(a, b);
-    }
-  }
-  if (want_norm) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-    if (lane == 0) red[warp][NV] = mk<double>(nrm, 0.0);
-  }
-  __syncthreads();
-  const int tot = nv + want_norm;
-  if (threadIdx.x < tot) {
-    const int src = (threadIdx.x < nv) ? threadIdx.x : NV;
-    double a = 0, b = 0;
-    for (int w = 0; w < RT / 32; ++w) {
-      a += red[w][src].x;
-      b += red[w][src].y;
-    }
-    part[(long long)threadIdx.x * nblk + blockIdx.x] = mk<double>(a, b);
-  }
-}
-
-__device__ __forceinline__ void zero_partials(int K1, double2* part, int nblk) {
-  if (threadIdx.x < K1) part[(long long)threadIdx.x * nblk + blockIdx.x] = mk<double>(0, 0);
-}
-
-// slots s < KT: sum conj(V_{i0+s}) w, slot KT (want_norm): ||w||^2
+// dots sum conj(V_{i0+s}) w for s < KT, and ||w||^2
 template <int KT>
 __global__ void __launch_bounds__(RT, 2) k_dots_df(long long N, const float4* __restrict__ V, long long vstride,
-                                                   long long ld, int i0, const float4* __restrict__ w, long long wld,
-                                                   const int* __restrict__ cols, const int* __restrict__ mask,
-                                                   int nblk, int want_norm, double2* __restrict__ part) {
-  constexpr int KA = KT > 0 ? KT : 1;
-  const int pos = blockIdx.y;
-  const int c = cols[pos];
-  const int K1 = KT + want_norm;
-  double2* pp = part + (long long)pos * K1 * nblk;
-  if (mask && !mask[c]) {
-    zero_partials(K1, pp, nblk);
-    return;
-  }
-  const float4* wc = w + (long long)c * wld;
+                                                   long long ld, int i0, const float4* __restrict__ w,
+                                                   const int* __restrict__ cols, int pass, int want_norm, GsColumn g) {
+  __shared__ double tot[2 * KT + 1];
+  const int c = cols[blockIdx.y];
+  if (pass && !g.flag[c]) return;
+  const int nblk = gridDim.x;
+  const float4* wc = w + (long long)c * ld;
   const float4* vb = V + ((long long)i0 * vstride + c) * ld;
   const long long vs = vstride * ld;
-  DAcc ar[KA], ai[KA], nn;
+  DAcc ar[KT], ai[KT], nn;
 #pragma unroll
-  for (int s = 0; s < KA; ++s) {
+  for (int s = 0; s < KT; ++s) {
     ar[s].init(0.f, 0.f);
     ai[s].init(0.f, 0.f);
   }
@@ -288,36 +244,36 @@ __global__ void __launch_bounds__(RT, 2) k_dots_df(long long N, const float4* __
       nn.mac(wv.y, wv.w, wv.y, wv.w);
     }
   }
-  double2 acc[KA];
+  double2 acc[KT];
 #pragma unroll
-  for (int s = 0; s < KA; ++s) acc[s] = mk<double>(ar[s].to_double(), ai[s].to_double());
-  block_reduce_df<KA>(acc, KT, nn.to_double(), want_norm, pp, nblk);
+  for (int s = 0; s < KT; ++s) acc[s] = mk<double>(ar[s].to_double(), ai[s].to_double());
+  double* part = g.part + (long long)blockIdx.y * (2 * KT + 1) * nblk;
+  block_partials<KT>(acc, KT, nn.to_double(), want_norm, part, nblk);
+  if (!last_of_column(g.count, c, nblk)) return;
+  fold_partials(part, nblk, 2 * KT + want_norm, tot);
+  gs_after_dots(g, c, i0, KT, want_norm, pass, tot);
 }
 
-// w -= sum_s h[c*hstride + i0 + s] V_{i0+s}; slot 0 (want_norm): ||w_new||^2
+// w -= sum_s coef_{i0+s} V_{i0+s}; with the last vectors ||w_new||^2 and the column's step
 template <int KT>
 __global__ void __launch_bounds__(RT, 2) k_update_df(long long N, const float4* __restrict__ V, long long vstride,
-                                                     long long ld, int i0, const double2* __restrict__ h,
-                                                     int hstride, float4* __restrict__ w, long long wld,
-                                                     const int* __restrict__ cols, const int* __restrict__ mask,
-                                                     int nblk, int want_norm, double2* __restrict__ part) {
-  const int pos = blockIdx.y;
-  const int c = cols[pos];
-  double2* pp = part + (long long)pos * want_norm * nblk;
-  if (mask && !mask[c]) {
-    zero_partials(want_norm, pp, nblk);
-    return;
-  }
+                                                     long long ld, int i0, float4* __restrict__ w,
+                                                     const int* __restrict__ cols, int j, int pass, int last,
+                                                     GsColumn g) {
+  __shared__ double tot[1];
+  const int c = cols[blockIdx.y];
+  if (pass && !g.flag[c]) return;
+  const int nblk = gridDim.x;
   float hrh[KT], hrl[KT], hih[KT], hil[KT];
 #pragma unroll
   for (int s = 0; s < KT; ++s) {
-    const double2 hv = h[(long long)c * hstride + i0 + s];
+    const double2 hv = g.coef[(long long)c * g.hstride + i0 + s];
     split(hv.x, hrh[s], hrl[s]);
     split(hv.y, hih[s], hil[s]);
   }
   const float4* vb = V + ((long long)i0 * vstride + c) * ld;
   const long long vs = vstride * ld;
-  float4* wc = w + (long long)c * wld;
+  float4* wc = w + (long long)c * ld;
   DAcc nn;
   nn.init(0.f, 0.f);
   const long long stride = (long long)nblk * RT;
@@ -338,55 +294,54 @@ __global__ void __launch_bounds__(RT, 2) k_update_df(long long N, const float4* 
     re.renorm();
     im.renorm();
     __stcs(&wc[p], make_float4(re.hi, im.hi, re.lo, im.lo));
-    if (want_norm) {
+    if (last) {
       nn.mac(re.hi, re.lo, re.hi, re.lo);
       nn.mac(im.hi, im.lo, im.hi, im.lo);
     }
   }
-  if (want_norm) {
-    const double2 none[1] = {mk<double>(0, 0)};
-    block_reduce_df<1>(none, 0, nn.to_double(), 1, pp, nblk);
-  }
+  if (!last) return;
+  double* part = g.part + (long long)blockIdx.y * nblk;
+  const double2 none[1] = {mk<double>(0, 0)};
+  block_partials<1>(none, 0, nn.to_double(), 1, part, nblk);
+  if (!last_of_column(g.count, c, nblk)) return;
+  fold_partials(part, nblk, 1, tot);
+  gs_after_update(g, c, j, pass, tot[0]);
 }
 
 #define HZ_K_CASES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 
-void launch_dots_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int i0, int K,
-                    const float4* w, long long wld, const int* cols, int ncols, int nblk, int want_norm,
-                    double2* part, const int* mask) {
+void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, int pass,
+                       const int* cols, int ncols, const GsColumn& g) {
   if (ncols <= 0) return;
-  dim3 grid(nblk, ncols);
-  const double bytes = mask ? 0.0 : (double)N * ncols * (K + 1) * 16.0;
-  switch (K) {
-#define HZ_DDF_CASE(k)                                                                                      \
-  case k:                                                                                                   \
-    HZ_LAUNCH(ctx, "krylov_dots", bytes, k_dots_df<k>, grid, RT, 0, N, V, vstride, ld, i0, w, wld, cols, mask, \
-              nblk, want_norm, part);                                                                       \
+  float4* w = const_cast<float4*>(V) + (long long)(j + 1) * vstride * ld;
+  const int K = j + 1;
+  const dim3 grid(krylov_nblk(N, ncols), ncols);
+  const double el = pass ? 0.0 : (double)N * ncols;
+  for (int i0 = 0; i0 < K; i0 += 16) {
+    const int k = std::min(16, K - i0);
+    const int wn = (pass == 0 && i0 + 16 >= K) ? 1 : 0;
+    switch (k) {
+#define HZ_GS_CASE(q)                                                                                             \
+  case q:                                                                                                         \
+    HZ_LAUNCH(ctx, "krylov_dots", el * (k + 1) * 16.0, k_dots_df<q>, grid, RT, 0, N, V, vstride, ld, i0, w, cols, \
+              pass, wn, g);                                                                                       \
     break;
-    HZ_DDF_CASE(0)
-    HZ_K_CASES(HZ_DDF_CASE)
-#undef HZ_DDF_CASE
-    default:
-      throw std::runtime_error("launch_dots_df: 0..16 vectors per pass");
+      HZ_K_CASES(HZ_GS_CASE)
+#undef HZ_GS_CASE
+    }
   }
-}
-
-void launch_update_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int i0, int K,
-                      const double2* h, int hstride, float4* w, long long wld, const int* cols, int ncols, int nblk,
-                      int want_norm, double2* part, const int* mask) {
-  if (ncols <= 0) return;
-  dim3 grid(nblk, ncols);
-  const double bytes = mask ? 0.0 : (double)N * ncols * (K + 2) * 16.0;
-  switch (K) {
-#define HZ_UDF_CASE(k)                                                                                            \
-  case k:                                                                                                         \
-    HZ_LAUNCH(ctx, "krylov_update", bytes, k_update_df<k>, grid, RT, 0, N, V, vstride, ld, i0, h, hstride, w, wld, \
-              cols, mask, nblk, want_norm, part);                                                                 \
+  for (int i0 = 0; i0 < K; i0 += 16) {
+    const int k = std::min(16, K - i0);
+    const int last = i0 + 16 >= K ? 1 : 0;
+    switch (k) {
+#define HZ_GS_CASE(q)                                                                                               \
+  case q:                                                                                                           \
+    HZ_LAUNCH(ctx, "krylov_update", el * (k + 2) * 16.0, k_update_df<q>, grid, RT, 0, N, V, vstride, ld, i0, w, cols, \
+              j, pass, last, g);                                                                                    \
     break;
-    HZ_K_CASES(HZ_UDF_CASE)
-#undef HZ_UDF_CASE
-    default:
-      throw std::runtime_error("launch_update_df: 1..16 vectors per pass");
+      HZ_K_CASES(HZ_GS_CASE)
+#undef HZ_GS_CASE
+    }
   }
 }
 

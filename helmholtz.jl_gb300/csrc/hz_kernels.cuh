@@ -129,12 +129,6 @@ int launch_fine_apply_noalloc(cudaStream_t stream, int dev, const FineOp& op, co
 template <typename TO>
 void launch_fine_df64(Ctx& ctx, const FineOp& op, const float4* dHd, const float2* z, TO* y, long long ld,
                       const int* cols, int ncols);
-void launch_dots_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int i0, int K,
-                    const float4* w, long long wld, const int* cols, int ncols, int nblk, int want_norm,
-                    double2* part, const int* mask = nullptr);
-void launch_update_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int i0, int K,
-                      const double2* h, int hstride, float4* w, long long wld, const int* cols, int ncols, int nblk,
-                      int want_norm, double2* part, const int* mask = nullptr);
 // y = s[c] x (FP64 x into df64 y; may run in place on the same memory)
 void launch_to_df(Ctx& ctx, long long N, const double2* x, long long xld, float4* y, long long yld, const double* s,
                   const int* cols, int ncols);
@@ -212,34 +206,38 @@ void launch_zero_cols(Ctx& ctx, long long N, cplx<T>* x, long long ld, const int
 // V + (i*vstride + c)*ld.  Partial sums go to part[(pos*K1 + slot)*nblk + blk]
 // and are folded in a fixed order by launch_reduce (deterministic results).
 int krylov_nblk(long long N, int ncols);
-// slots i < K: conj(V_{i0+i}) . w ; slot K (want_norm): ||w||^2.  Columns with
-// mask[c] == 0 (mask may be null) yield zeros; a masked launch adds no
-// algorithmic bytes (the caller adds those of the columns that took it).
-void launch_dots(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int i0, int K,
-                 const double2* w, long long wld, const int* cols, int ncols, int nblk, int want_norm, double2* part,
-                 const int* mask = nullptr);
-// w -= sum_{i<K} h[c*hstride + i0 + i] V_{i0+i}; with want_norm, slot 0 of the
-// partials holds ||w_new||^2.  Columns with mask[c] == 0 are left untouched.
-void launch_update(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int i0, int K,
-                   const double2* h, int hstride, double2* w, long long wld, const int* cols, int ncols, int nblk,
-                   int want_norm, double2* part, const int* mask = nullptr);
-// flag[c] = (after[c*astride] < before[c*bstride + bslot] / 2): DGKS test for a
-// second Gram-Schmidt pass.
-void launch_dgks(Ctx& ctx, const int* cols, int ncols, const double2* before, int bstride, int bslot,
-                 const double2* after, int astride, int* flag);
+// K (0 or 1) dots conj(V) . w and, with want_norm, ||w||^2 in slot K (norms and BiCGSTAB).
+void launch_dots(Ctx& ctx, long long N, const double2* V, long long ld, int K, const double2* w, long long wld,
+                 const int* cols, int ncols, int nblk, int want_norm, double2* part);
+// Classical Gram-Schmidt with the DGKS test on the unnormalised FGMRES basis: stored v_i
+// stands for sig_i v_i (sig[c*sstride + i]), w = v_{j+1} on entry.  Pass 0 runs for every
+// column, pass 1 only for the columns that the test flagged (||w'||^2 < ||w||^2 / 2).  The
+// per-column results and scalar work are in hz_gs.cuh.
+struct GsColumn {
+  int m = 0;                                      // restart length
+  double2 *hA = nullptr, *hB = nullptr;           // dots of pass 0 / 1 (pass 0: ||w||^2 in slot j + 1)
+  double2* coef = nullptr;                        // update coefficients sig_i^2 d_i
+  int hstride = 0;
+  double* sig = nullptr;
+  int sstride = 0;
+  double2 *Hh = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr;  // Hessenberg columns, rotations, right-hand side
+  int* flag = nullptr;                            // second pass due
+  double* host_est = nullptr;                     // pinned: residual estimates
+  int* host_flag = nullptr;                       // pinned copy of flag
+  int* count = nullptr;                           // block counters, zero
+  double* part = nullptr;                         // partial sums, gs_part_bytes
+};
+size_t gs_part_bytes(long long N, int R);
+// the dots of step j (K = j + 1 vectors) and the update w -= sum coef_i V_i of one pass
+void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int j, int pass,
+                    const int* cols, int ncols, const GsColumn& g);
+void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, int pass,
+                       const int* cols, int ncols, const GsColumn& g);
 // out[c*ostride + slot] = sum over blocks of part (slot < K1); accum adds to out.
 void launch_reduce(Ctx& ctx, const double2* part, const int* cols, int ncols, int K1, int nblk, double2* out,
                    int ostride, int accum);
-// Deferred normalisation of the FGMRES basis: stored v_i stands for sig_i v_i
-// (sig[c*sstride + i]).  init: sig_0 = 1; coef_i = sig_i^2 d_i for i < K (the
-// update's coefficients); true: hA_i, hB_i *= sig_i sig_j (i <= j) and the norm
-// slots nr, nr2 *= sig_j^2; next: sig_{j+1} = sig_j * invhn; y_i *= sig_i.
+// Deferred normalisation of the FGMRES basis: sig_0 = 1; y_i *= sig_i.
 void launch_sig_init(Ctx& ctx, const int* cols, int ncols, double* sig, int sstride);
-void launch_sig_coef(Ctx& ctx, const int* cols, int ncols, int K, const double* sig, int sstride, const double2* d,
-                     int hstride, double2* coef);
-void launch_sig_true(Ctx& ctx, int j, const int* cols, int ncols, const double* sig, int sstride, double2* hA,
-                     double2* hB, double2* nr, double2* nr2, int hstride);
-void launch_sig_next(Ctx& ctx, int j, const int* cols, int ncols, double* sig, int sstride, const double* invhn);
 void launch_sig_y(Ctx& ctx, const int* cols, int ncols, const int* kcol, const double* sig, int sstride, double2* y,
                   int ystride);
 // y[:, c] = s[c] * x[:, c]
@@ -256,14 +254,7 @@ void launch_norms(Ctx& ctx, const double2* red, int stride, int slot, const int*
                   double* inv);
 // g[c*(m+1) + 0] = beta[c], the other entries of g zero.
 void launch_cycle_init(Ctx& ctx, int m, const int* cols, int ncols, const double* beta, double2* g);
-// Arnoldi step j of column c: h = hA + hB (hB may be null), h_{j+1,j} =
-// sqrt(Re nrm[c*hstride]) or, where flag[c] is set (second pass taken),
-// sqrt(Re nrm2[c*hstride]); apply rotations 0..j-1, form rotation j, update
-// g, est[c] = |g_{j+1}|, inv_hn[c] = 1/h_{j+1,j}.
 // Hh[c*(m+1)*m + jj*(m+1) + i], cs/sn[c*m + i], g[c*(m+1) + i].
-void launch_arnoldi_step(Ctx& ctx, int j, int m, const int* cols, int ncols, const double2* hA, const double2* hB,
-                         const double2* nrm, const double2* nrm2, const int* flag, int hstride, double2* Hh,
-                         double2* cs, double2* sn, double2* g, double* est, double* inv_hn);
 // BiCGSTAB per-column scalars sc[c*8 + k] (0 rho, 1 rho_prev, 2 alpha, 3 omega,
 // 4 beta) from reduced dots red[c*rstride + slot]: stage -1 init, 0 beta from
 // <rh,r>, 1 alpha from <rh,v>, 2 omega from (conj<t,s>, ||t||^2).

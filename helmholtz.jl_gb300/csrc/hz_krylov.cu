@@ -8,15 +8,14 @@
 // (src/ShiftedLaplacianMultigridSolver.jl:64-65).
 #include <algorithm>
 
+#include "hz_fixed.cuh"
+#include "hz_gs.cuh"
 #include "hz_launch.cuh"
 
 namespace hz {
 
 static constexpr int KG = 16;  // dot products carried per pass in registers
 
-// sqrt of a reduced sum of squares: rounding can leave it a hair below zero;
-// NaN and Inf pass through so the host sees a corrupted column.
-__device__ __forceinline__ double safe_sqrt(double v) { return (v > 0.0 || v != v) ? sqrt(v) : 0.0; }
 static constexpr int RT = 256; // threads per reduction CTA
 
 int krylov_nblk(long long N, int ncols) {
@@ -27,176 +26,260 @@ int krylov_nblk(long long N, int ncols) {
   return (int)nb;
 }
 
-// Block-wide sums of nv complex values (v[0..nv)) and, when want_norm, one
-// real value; thread s writes slot s of this block's partials:
-// part[s*nblk + blockIdx.x] (the norm goes to slot nv).
-template <int NV>
-__device__ __forceinline__ void block_reduce_store(const double2 (&v)[NV], int nv, double nrm, int want_norm,
-                                                   double2* part, int nblk) {
-  __shared__ double2 red[RT / 32][NV + 1];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int s = 0; s < NV; ++s) {
-    if (s < nv) {
-      double a = v[s].x, b = v[s].y;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-      }
-      if (lane == 0) red[warp][s] = mk<double>(a, b);
-    }
-  }
-  if (want_norm) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-    if (lane == 0) red[warp][NV] = mk<double>(nrm, 0.0);
-  }
-  __syncthreads();
-  const int tot = nv + want_norm;
-  if (threadIdx.x < tot) {
-    const int src = (threadIdx.x < nv) ? threadIdx.x : NV;
-    double a = 0, b = 0;
-    for (int w = 0; w < RT / 32; ++w) {
-      a += red[w][src].x;
-      b += red[w][src].y;
-    }
-    part[(long long)threadIdx.x * nblk + blockIdx.x] = mk<double>(a, b);
-  }
-}
-
-// Zero partials of a masked-off column (the reduce then yields zeros).
-__device__ __forceinline__ void store_zero_partials(int K1, double2* part, int nblk) {
-  if (threadIdx.x < K1) part[(long long)threadIdx.x * nblk + blockIdx.x] = mk<double>(0, 0);
-}
-
+// KT (0 or 1) dots and the norm of w: native FP64, its rounding order is part of the
+// BiCGSTAB iteration.  Block totals in part[(pos * K1 + slot) * nblk + blk].
 template <int KT>
-__global__ void __launch_bounds__(RT, 2) k_dots(long long N, const double2* __restrict__ V, long long vstride,
-                                                long long ld, int i0, const double2* __restrict__ w, long long wld,
-                                                const int* __restrict__ cols, const int* __restrict__ mask, int nblk,
-                                                int want_norm, double2* __restrict__ part) {
+__global__ void __launch_bounds__(RT, 2) k_dots(long long N, const double2* __restrict__ V, long long ld,
+                                                const double2* __restrict__ w, long long wld,
+                                                const int* __restrict__ cols, int nblk, int want_norm,
+                                                double2* __restrict__ part) {
+  __shared__ double sh[RT / 32][4];
   const int pos = blockIdx.y;
   const int c = cols[pos];
   const int K1 = KT + want_norm;
   double2* pp = part + (long long)pos * K1 * nblk;
-  if (mask && !mask[c]) {
-    store_zero_partials(K1, pp, nblk);
-    return;
-  }
   const double2* wc = w + (long long)c * wld;
-  const double2* vb = V + ((long long)i0 * vstride + c) * ld;
-  const long long vs = vstride * ld;  // distance between consecutive basis vectors
-  constexpr int KA = KT > 0 ? KT : 1;  // KT = 0: the norm alone
-  double2 acc[KA];
-#pragma unroll
-  for (int s = 0; s < KA; ++s) acc[s] = mk<double>(0, 0);
+  const double2* vc = V + (long long)c * ld;
+  double2 acc = mk<double>(0, 0);
   double nrm = 0.0;
   const long long stride = (long long)nblk * RT;
+#pragma unroll 4
   for (long long p = (long long)blockIdx.x * RT + threadIdx.x; p < N; p += stride) {
     const double2 wv = wc[p];
-#pragma unroll
-    for (int s = 0; s < KT; ++s) acc[s] = cfma_conj<double>(vb[s * vs + p], wv, acc[s]);
+    if (KT) acc = cfma_conj<double>(vc[p], wv, acc);
     if (want_norm) nrm = fma(wv.x, wv.x, fma(wv.y, wv.y, nrm));
   }
-  block_reduce_store<KA>(acc, KT, nrm, want_norm, pp, nblk);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[4] = {acc.x, acc.y, nrm, 0.0};
+  const double t = warp_totals<4>(v, lane);
+  if ((lane & 7) == 0) sh[warp][warp_total_index<4>(lane)] = t;
+  __syncthreads();
+  if ((int)threadIdx.x < K1) {
+    const int i = (int)threadIdx.x < KT ? 0 : 2;
+    double a = 0, b = 0;
+    for (int q = 0; q < RT / 32; ++q) {
+      a += sh[q][i];
+      b += sh[q][i + 1];
+    }
+    pp[(long long)threadIdx.x * nblk + blockIdx.x] = mk<double>(a, b);
+  }
+}
+
+void launch_dots(Ctx& ctx, long long N, const double2* V, long long ld, int K, const double2* w, long long wld,
+                 const int* cols, int ncols, int nblk, int want_norm, double2* part) {
+  if (ncols <= 0) return;
+  const dim3 grid(nblk, ncols);
+  const double bytes = (double)N * ncols * (K + 1) * sizeof(double2);
+  // FP64 arithmetic: a complex multiply-add (8 flops) per vector and node, 4 for ||w||^2
+  ctx.add_flops("krylov_dots", (double)N * ncols * (8.0 * K + (want_norm ? 4.0 : 0.0)));
+  if (K == 0)
+    HZ_LAUNCH(ctx, "krylov_dots", bytes, k_dots<0>, grid, RT, 0, N, V, ld, w, wld, cols, nblk, want_norm, part);
+  else if (K == 1)
+    HZ_LAUNCH(ctx, "krylov_dots", bytes, k_dots<1>, grid, RT, 0, N, V, ld, w, wld, cols, nblk, want_norm, part);
+  else
+    throw std::runtime_error("launch_dots: 0 or 1 vectors");
+}
+
+// ---------------------------------------------------------------------------
+// Gram-Schmidt in FP64 on the integer pipe (hz_fixed.cuh)
+// ---------------------------------------------------------------------------
+// Native FP64 takes four FMAs per 16-byte basis element, two clocks of an SM; HBM delivers
+// the element in 0.7.  Dots: a thread takes four nodes at a time, relates the basis values
+// and w to the largest of its own four, sums the products in integers and adds the exact
+// total to its FP64 accumulator.  Update: all terms of a node are related to the
+// node's largest term, and their exact sum is subtracted from w with one rounding.
+// Values outside the range of hz_fixed.cuh take the native steps.
+// Measured, native -> fixed, per pass averaged over the steps of restart 10: 129^3 x 8: dots
+// 632 -> 486 us, update 642 -> 430 us; 1025 x 513 x 16: 333 -> 255, 320 -> 226 us (the second
+// pass included, which most columns take).  Errors against quadruple precision, 4,096 to
+// 200,000 nodes, waves, a point source's peak and noise: dots 3e-17 to 1.5e-16 of |V||w|
+// (native 5e-17 to 2.6e-16), update 6e-17 of |w'| rms (native 2.4e-16).
+static constexpr int kGsNodes = 4;
+
+template <int KT>
+__global__ void __launch_bounds__(RT, 2) k_gs_dots(long long N, const double2* __restrict__ V, long long vstride,
+                                                   long long ld, int i0, const double2* __restrict__ w,
+                                                   const int* __restrict__ cols, int pass, int want_norm, GsColumn g) {
+  __shared__ double tot[2 * KT + 1];
+  const int c = cols[blockIdx.y];
+  if (pass && !g.flag[c]) return;
+  const int nblk = gridDim.x;
+  const double2* wc = w + (long long)c * ld;
+  const double2* vb = V + ((long long)i0 * vstride + c) * ld;
+  const long long vs = vstride * ld;  // distance between consecutive basis vectors
+  double2 acc[KT];
+#pragma unroll
+  for (int s = 0; s < KT; ++s) acc[s] = mk<double>(0, 0);
+  double nrm = 0.0;
+  const long long stride = (long long)nblk * RT;
+  auto load = [&](const double2* x, long long p, uint4 (&r)[kGsNodes]) {
+    int e = 0;
+#pragma unroll
+    for (int q = 0; q < kGsNodes; ++q) {
+      r[q] = p + q * stride < N ? *reinterpret_cast<const uint4*>(x + p + q * stride) : make_uint4(0, 0, 0, 0);
+      e = max(e, max(fixed_exponent(r[q].y), fixed_exponent(r[q].w)));
+    }
+    return e;
+  };
+  auto value = [](const uint4& r) {
+    return mk<double>(__hiloint2double((int)r.y, (int)r.x), __hiloint2double((int)r.w, (int)r.z));
+  };
+  for (long long p = (long long)blockIdx.x * RT + threadIdx.x; p < N; p += kGsNodes * stride) {
+    uint4 wr[kGsNodes];
+    const int ew = load(wc, p, wr);
+    Fixed wx[kGsNodes], wy[kGsNodes];
+#pragma unroll
+    for (int q = 0; q < kGsNodes; ++q) {
+      wx[q] = fixed_from<6>(wr[q].y, wr[q].x, ew);
+      wy[q] = fixed_from<6>(wr[q].w, wr[q].z, ew);
+      if (want_norm) {
+        const double2 v = value(wr[q]);
+        nrm = fma(v.x, v.x, fma(v.y, v.y, nrm));
+      }
+    }
+    const bool wok = fixed_ref_ok(ew);
+#pragma unroll
+    for (int s = 0; s < KT; ++s) {
+      uint4 vr[kGsNodes];
+      const int ev = load(vb + s * vs, p, vr);
+      if (wok && fixed_ref_ok(ev) && fixed_ok(ev + ew)) {
+        FixedSum f{0, 0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < kGsNodes; ++q)
+          fixed_conj_mac(f, fixed_from<6>(vr[q].y, vr[q].x, ev), fixed_from<6>(vr[q].w, vr[q].z, ev), wx[q], wy[q]);
+        const double sc = __hiloint2double((int)fixed_scale_hi(ev + ew, 0), 0);
+        acc[s].x = fma((double)fixed_total(f.rh, f.rl), sc, acc[s].x);
+        acc[s].y = fma((double)fixed_total(f.ih, f.il), sc, acc[s].y);
+      } else {
+#pragma unroll
+        for (int q = 0; q < kGsNodes; ++q)
+          if (p + q * stride < N) acc[s] = cfma_conj<double>(value(vr[q]), wc[p + q * stride], acc[s]);
+      }
+    }
+  }
+  double* part = g.part + (long long)blockIdx.y * (2 * KT + 1) * nblk;
+  block_partials<KT>(acc, KT, nrm, want_norm, part, nblk);
+  if (!last_of_column(g.count, c, nblk)) return;
+  fold_partials(part, nblk, 2 * KT + want_norm, tot);
+  gs_after_dots(g, c, i0, KT, want_norm, pass, tot);
 }
 
 template <int KT>
-__global__ void __launch_bounds__(RT, 2) k_update(long long N, const double2* __restrict__ V, long long vstride,
-                                                  long long ld, int i0, const double2* __restrict__ h, int hstride,
-                                                  double2* __restrict__ w, long long wld,
-                                                  const int* __restrict__ cols, const int* __restrict__ mask,
-                                                  int nblk, int want_norm, double2* __restrict__ part) {
-  const int pos = blockIdx.y;
-  const int c = cols[pos];
-  double2* pp = part + (long long)pos * want_norm * nblk;
-  if (mask && !mask[c]) {
-    store_zero_partials(want_norm, pp, nblk);
-    return;
+__global__ void __launch_bounds__(RT, 2) k_gs_update(long long N, const double2* __restrict__ V, long long vstride,
+                                                     long long ld, int i0, double2* __restrict__ w,
+                                                     const int* __restrict__ cols, int j, int pass, int last,
+                                                     GsColumn g) {
+  __shared__ int4 hl[KT];
+  __shared__ int he[KT];
+  __shared__ double tot[1];
+  const int c = cols[blockIdx.y];
+  if (pass && !g.flag[c]) return;
+  const int nblk = gridDim.x;
+  const double2* h = g.coef + (long long)c * g.hstride + i0;
+  constexpr int kNone = -(1 << 20);  // exponent of a zero coefficient
+  int bad = 0;
+  if (threadIdx.x < KT) {
+    const uint4 r = *reinterpret_cast<const uint4*>(h + threadIdx.x);
+    const int e = max(fixed_exponent(r.y), fixed_exponent(r.w));
+    const bool zero = ((r.x | r.z) == 0) && (((r.y | r.w) & 0x7fffffffu) == 0);
+    bad = !zero && !fixed_ref_ok(e);
+    const Fixed a = fixed_from<6>(r.y, r.x, e), b = fixed_from<6>(r.w, r.z, e);
+    hl[threadIdx.x] = zero ? make_int4(0, 0, 0, 0) : make_int4(a.hi, a.lo, b.hi, b.lo);
+    he[threadIdx.x] = zero ? kNone : e;
   }
-  double2 hv[KT];
+  bad = __syncthreads_or(bad);
+  int hmax = kNone;
 #pragma unroll
-  for (int s = 0; s < KT; ++s) hv[s] = h[(long long)c * hstride + i0 + s];
+  for (int s = 0; s < KT; ++s) hmax = max(hmax, he[s]);
   const double2* vb = V + ((long long)i0 * vstride + c) * ld;
   const long long vs = vstride * ld;
+  double2* wc = w + (long long)c * ld;
   double nrm = 0.0;
-  double2* wc = w + (long long)c * wld;
   const long long stride = (long long)nblk * RT;
   for (long long p = (long long)blockIdx.x * RT + threadIdx.x; p < N; p += stride) {
-    double2 wv = wc[p];
+    uint4 vr[KT];
 #pragma unroll
-    for (int s = 0; s < KT; ++s) wv = cfms<double>(hv[s], vb[s * vs + p], wv);
+    for (int s = 0; s < KT; ++s) vr[s] = *reinterpret_cast<const uint4*>(vb + s * vs + p);
+    double2 wv = wc[p];
+    int vmax = 0, T = kNone;
+#pragma unroll
+    for (int s = 0; s < KT; ++s) {
+      const int e = max(fixed_exponent(vr[s].y), fixed_exponent(vr[s].w));
+      vmax = max(vmax, e);
+      T = max(T, e + he[s]);
+    }
+    if (!bad && vmax < 0x7ff && T - hmax >= kFixedMin && fixed_ok(T)) {
+      FixedSum f{0, 0, 0, 0};
+#pragma unroll
+      for (int s = 0; s < KT; ++s) {
+        const int4 a = hl[s];
+        const int e = T - he[s];
+        fixed_cmac(f, Fixed{a.x, a.y}, Fixed{a.z, a.w}, fixed_from<7>(vr[s].y, vr[s].x, e),
+                   fixed_from<7>(vr[s].w, vr[s].z, e));
+      }
+      const double sc = __hiloint2double((int)fixed_scale_hi(T, 1), 0);
+      wv.x = fma((double)-fixed_total(f.rh, f.rl), sc, wv.x);
+      wv.y = fma((double)-fixed_total(f.ih, f.il), sc, wv.y);
+    } else {
+#pragma unroll
+      for (int s = 0; s < KT; ++s)
+        wv = cfms<double>(h[s],
+                          mk<double>(__hiloint2double((int)vr[s].y, (int)vr[s].x),
+                                     __hiloint2double((int)vr[s].w, (int)vr[s].z)),
+                          wv);
+    }
     wc[p] = wv;
-    if (want_norm) nrm = fma(wv.x, wv.x, fma(wv.y, wv.y, nrm));
+    if (last) nrm = fma(wv.x, wv.x, fma(wv.y, wv.y, nrm));
   }
-  if (want_norm) {
-    const double2 none[1] = {mk<double>(0, 0)};
-    block_reduce_store<1>(none, 0, nrm, 1, pp, nblk);
-  }
+  if (!last) return;
+  double* part = g.part + (long long)blockIdx.y * nblk;
+  const double2 none[1] = {mk<double>(0, 0)};
+  block_partials<1>(none, 0, nrm, 1, part, nblk);
+  if (!last_of_column(g.count, c, nblk)) return;
+  fold_partials(part, nblk, 1, tot);
+  gs_after_update(g, c, j, pass, tot[0]);
 }
 
 #define HZ_K_CASES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 
-void launch_dots(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int i0, int K,
-                 const double2* w, long long wld, const int* cols, int ncols, int nblk, int want_norm, double2* part,
-                 const int* mask) {
+size_t gs_part_bytes(long long N, int R) { return (size_t)R * krylov_nblk(N, 1) * 33 * sizeof(double); }
+
+void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int j, int pass,
+                    const int* cols, int ncols, const GsColumn& g) {
   if (ncols <= 0) return;
-  dim3 grid(nblk, ncols);
+  double2* w = const_cast<double2*>(V) + (long long)(j + 1) * vstride * ld;
+  const int K = j + 1;
+  const dim3 grid(krylov_nblk(N, ncols), ncols);
   // a masked pass is charged by the host once it knows which columns took it
-  const double bytes = mask ? 0.0 : (double)N * ncols * (K + 1) * sizeof(double2);
-  // FP64 arithmetic: a complex multiply-add (8 flops) per vector and node, 4 for ||w||^2
-  if (!mask) ctx.add_flops("krylov_dots", (double)N * ncols * (8.0 * K + (want_norm ? 4.0 : 0.0)));
-  switch (K) {
-#define HZ_DOTS_CASE(k)                                                                                     \
-  case k:                                                                                                   \
-    HZ_LAUNCH(ctx, "krylov_dots", bytes, k_dots<k>, grid, RT, 0, N, V, vstride, ld, i0, w, wld, cols, mask, \
-              nblk, want_norm, part);                                                                       \
+  const double el = pass ? 0.0 : (double)N * ncols;
+  for (int i0 = 0; i0 < K; i0 += 16) {
+    const int k = std::min(16, K - i0);
+    const int wn = (pass == 0 && i0 + 16 >= K) ? 1 : 0;  // ||w||^2 before the update (slot K)
+    ctx.add_flops("krylov_dots", el * (8.0 * k + (wn ? 4.0 : 0.0)));
+    switch (k) {
+#define HZ_GS_CASE(q)                                                                                             \
+  case q:                                                                                                         \
+    HZ_LAUNCH(ctx, "krylov_dots", el * (k + 1) * 16.0, k_gs_dots<q>, grid, RT, 0, N, V, vstride, ld, i0, w, cols, \
+              pass, wn, g);                                                                                       \
     break;
-    HZ_DOTS_CASE(0)
-    HZ_K_CASES(HZ_DOTS_CASE)
-#undef HZ_DOTS_CASE
-    default:
-      throw std::runtime_error("launch_dots: 1..16 vectors per pass");
+      HZ_K_CASES(HZ_GS_CASE)
+#undef HZ_GS_CASE
+    }
   }
-}
-
-void launch_update(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int i0, int K,
-                   const double2* h, int hstride, double2* w, long long wld, const int* cols, int ncols, int nblk,
-                   int want_norm, double2* part, const int* mask) {
-  if (ncols <= 0) return;
-  dim3 grid(nblk, ncols);
-  const double bytes = mask ? 0.0 : (double)N * ncols * (K + 2) * sizeof(double2);
-  if (!mask) ctx.add_flops("krylov_update", (double)N * ncols * (8.0 * K + (want_norm ? 4.0 : 0.0)));
-  switch (K) {
-#define HZ_UPD_CASE(k)                                                                                           \
-  case k:                                                                                                        \
-    HZ_LAUNCH(ctx, "krylov_update", bytes, k_update<k>, grid, RT, 0, N, V, vstride, ld, i0, h, hstride, w, wld, \
-              cols, mask, nblk, want_norm, part);                                                                \
+  for (int i0 = 0; i0 < K; i0 += 16) {
+    const int k = std::min(16, K - i0);
+    const int last = i0 + 16 >= K ? 1 : 0;
+    ctx.add_flops("krylov_update", el * (8.0 * k + (last ? 4.0 : 0.0)));
+    switch (k) {
+#define HZ_GS_CASE(q)                                                                                               \
+  case q:                                                                                                           \
+    HZ_LAUNCH(ctx, "krylov_update", el * (k + 2) * 16.0, k_gs_update<q>, grid, RT, 0, N, V, vstride, ld, i0, w, cols, \
+              j, pass, last, g);                                                                                    \
     break;
-    HZ_K_CASES(HZ_UPD_CASE)
-#undef HZ_UPD_CASE
-    default:
-      throw std::runtime_error("launch_update: 1..16 vectors per pass");
+      HZ_K_CASES(HZ_GS_CASE)
+#undef HZ_GS_CASE
+    }
   }
-}
-
-// DGKS test per column: a second Gram-Schmidt pass is needed when the first
-// one removed more than half of the squared norm (||w'||^2 < ||w||^2 / 2).
-__global__ void k_dgks(const int* __restrict__ cols, int ncols, const double2* __restrict__ before, int bstride,
-                       int bslot, const double2* __restrict__ after, int astride, int* __restrict__ flag) {
-  const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= ncols) return;
-  const int c = cols[pos];
-  const double b = before[(long long)c * bstride + bslot].x;
-  const double a = after[(long long)c * astride].x;
-  flag[c] = (a < 0.5 * b) ? 1 : 0;
-}
-
-void launch_dgks(Ctx& ctx, const int* cols, int ncols, const double2* before, int bstride, int bslot,
-                 const double2* after, int astride, int* flag) {
-  if (ncols <= 0) return;
-  HZ_LAUNCH(ctx, "dgks", 0.0, k_dgks, (ncols + 127) / 128, 128, 0, cols, ncols, before, bstride, bslot, after, astride,
-            flag);
 }
 
 // One warp per (column, slot): fixed-order sum over the nblk partials.
@@ -241,47 +324,10 @@ void launch_reduce(Ctx& ctx, const double2* part, const int* cols, int ncols, in
 // normalising it.  From the stored dots d_i = conj(v_i) . w' of the stored
 // candidate w' (= H Z'_j, Z'_j the cycle applied to v_j): the update uses the
 // coefficients sig_i^2 d_i, the Hessenberg entries are sig_i sig_j d_i and
-// h_{j+1,j} = sig_j ||w''||.
+// h_{j+1,j} = sig_j ||w''|| (hz_gs.cuh).
 __global__ void k_sig_init(const int* __restrict__ cols, int ncols, double* __restrict__ sig, int sstride) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < ncols) sig[(long long)cols[i] * sstride] = 1.0;
-}
-
-__global__ void k_sig_coef(const int* __restrict__ cols, int ncols, int K, const double* __restrict__ sig, int sstride,
-                           const double2* __restrict__ d, int hstride, double2* __restrict__ coef) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncols * K) return;
-  const int c = cols[t / K], i = t % K;
-  const double s = sig[(long long)c * sstride + i];
-  const double2 v = d[(long long)c * hstride + i];
-  coef[(long long)c * hstride + i] = mk<double>(s * s * v.x, s * s * v.y);
-}
-
-__global__ void k_sig_true(int j, const int* __restrict__ cols, int ncols, const double* __restrict__ sig, int sstride,
-                           double2* __restrict__ hA, double2* __restrict__ hB, double2* __restrict__ nr,
-                           double2* __restrict__ nr2, int hstride) {
-  const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= ncols) return;
-  const int c = cols[pos];
-  const double* sc = sig + (long long)c * sstride;
-  const double sj = sc[j];
-  for (int i = 0; i <= j; ++i) {
-    const double f = sc[i] * sj;
-    double2& a = hA[(long long)c * hstride + i];
-    double2& b = hB[(long long)c * hstride + i];
-    a = mk<double>(f * a.x, f * a.y);
-    b = mk<double>(f * b.x, f * b.y);
-  }
-  nr[(long long)c * hstride].x *= sj * sj;
-  nr2[(long long)c * hstride].x *= sj * sj;
-}
-
-__global__ void k_sig_next(int j, const int* __restrict__ cols, int ncols, double* __restrict__ sig, int sstride,
-                           const double* __restrict__ invhn) {
-  const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= ncols) return;
-  const int c = cols[pos];
-  sig[(long long)c * sstride + j + 1] = sig[(long long)c * sstride + j] * invhn[c];
 }
 
 __global__ void k_sig_y(const int* __restrict__ cols, int ncols, const int* __restrict__ kcol,
@@ -299,22 +345,6 @@ __global__ void k_sig_y(const int* __restrict__ cols, int ncols, const int* __re
 void launch_sig_init(Ctx& ctx, const int* cols, int ncols, double* sig, int sstride) {
   if (ncols <= 0) return;
   HZ_LAUNCH(ctx, "basis_scale", 0.0, k_sig_init, (ncols + 127) / 128, 128, 0, cols, ncols, sig, sstride);
-}
-void launch_sig_coef(Ctx& ctx, const int* cols, int ncols, int K, const double* sig, int sstride, const double2* d,
-                     int hstride, double2* coef) {
-  if (ncols <= 0 || K <= 0) return;
-  HZ_LAUNCH(ctx, "basis_scale", 0.0, k_sig_coef, (ncols * K + 127) / 128, 128, 0, cols, ncols, K, sig, sstride, d,
-            hstride, coef);
-}
-void launch_sig_true(Ctx& ctx, int j, const int* cols, int ncols, const double* sig, int sstride, double2* hA,
-                     double2* hB, double2* nr, double2* nr2, int hstride) {
-  if (ncols <= 0) return;
-  HZ_LAUNCH(ctx, "basis_scale", 0.0, k_sig_true, (ncols + 127) / 128, 128, 0, j, cols, ncols, sig, sstride, hA, hB, nr,
-            nr2, hstride);
-}
-void launch_sig_next(Ctx& ctx, int j, const int* cols, int ncols, double* sig, int sstride, const double* invhn) {
-  if (ncols <= 0) return;
-  HZ_LAUNCH(ctx, "basis_scale", 0.0, k_sig_next, (ncols + 127) / 128, 128, 0, j, cols, ncols, sig, sstride, invhn);
 }
 void launch_sig_y(Ctx& ctx, const int* cols, int ncols, const int* kcol, const double* sig, int sstride, double2* y,
                   int ystride) {
@@ -389,7 +419,7 @@ __global__ void k_norms(const double2* __restrict__ red, int stride, int slot, c
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   if (pos >= ncols) return;
   const int c = cols[pos];
-  const double v = safe_sqrt(red[(long long)c * stride + slot].x);
+  const double v = gs_sqrt(red[(long long)c * stride + slot].x);
   nrm[c] = v;
   if (inv) inv[c] = (v > 0) ? 1.0 / v : 0.0;
 }
@@ -411,64 +441,6 @@ __global__ void k_cycle_init(int m, const int* __restrict__ cols, int ncols, con
 void launch_cycle_init(Ctx& ctx, int m, const int* cols, int ncols, const double* beta, double2* g) {
   if (ncols <= 0) return;
   HZ_LAUNCH(ctx, "cycle_init", 0.0, k_cycle_init, (ncols + 127) / 128, 128, 0, m, cols, ncols, beta, g);
-}
-
-// Complex Givens rotation convention: (u, v) -> (conj(c) u + conj(s) v, -s u + c v).
-__global__ void k_arnoldi_step(int j, int m, const int* __restrict__ cols, int ncols, const double2* __restrict__ hA,
-                               const double2* __restrict__ hB, const double2* __restrict__ nrm,
-                               const double2* __restrict__ nrm2, const int* __restrict__ flag, int hstride,
-                               double2* __restrict__ Hh, double2* __restrict__ cs, double2* __restrict__ sn,
-                               double2* __restrict__ g, double* __restrict__ est, double* __restrict__ inv_hn) {
-  const int pos = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pos >= ncols) return;
-  const int c = cols[pos];
-  double2* H = Hh + (long long)c * (m + 1) * m + (long long)j * (m + 1);
-  const double2* csc = cs + (long long)c * m;
-  const double2* snc = sn + (long long)c * m;
-  for (int i = 0; i <= j; ++i) {
-    double2 v = hA[(long long)c * hstride + i];
-    if (hB) v = cadd<double>(v, hB[(long long)c * hstride + i]);
-    H[i] = v;
-  }
-  const bool second = flag && flag[c];
-  const double hn = safe_sqrt((second ? nrm2 : nrm)[(long long)c * hstride].x);
-  H[j + 1] = mk<double>(hn, 0.0);
-  for (int i = 0; i < j; ++i) {
-    const double2 u = H[i], v = H[i + 1];
-    const double2 ci = csc[i], si = snc[i];
-    H[i] = cadd<double>(cmul<double>(cconj<double>(ci), u), cmul<double>(cconj<double>(si), v));
-    H[i + 1] = csub<double>(cmul<double>(ci, v), cmul<double>(si, u));
-  }
-  const double2 a = H[j], b = H[j + 1];
-  double den = sqrt(a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y);
-  double2 cj, sj;
-  if (den > 0) {
-    cj = mk<double>(a.x / den, a.y / den);
-    sj = mk<double>(b.x / den, b.y / den);
-  } else {
-    cj = mk<double>(1.0, 0.0);
-    sj = mk<double>(0.0, 0.0);
-    den = 0.0;
-  }
-  cs[(long long)c * m + j] = cj;
-  sn[(long long)c * m + j] = sj;
-  H[j] = mk<double>(den, 0.0);
-  H[j + 1] = mk<double>(0.0, 0.0);
-  double2* gc = g + (long long)c * (m + 1);
-  const double2 gj = gc[j];
-  gc[j] = cmul<double>(cconj<double>(cj), gj);
-  const double2 gn = cmul<double>(sj, gj);
-  gc[j + 1] = mk<double>(-gn.x, -gn.y);
-  est[c] = sqrt(gn.x * gn.x + gn.y * gn.y);
-  inv_hn[c] = (hn > 0) ? 1.0 / hn : 0.0;
-}
-
-void launch_arnoldi_step(Ctx& ctx, int j, int m, const int* cols, int ncols, const double2* hA, const double2* hB,
-                         const double2* nrm, const double2* nrm2, const int* flag, int hstride, double2* Hh,
-                         double2* cs, double2* sn, double2* g, double* est, double* inv_hn) {
-  if (ncols <= 0) return;
-  HZ_LAUNCH(ctx, "arnoldi_step", 0.0, k_arnoldi_step, (ncols + 63) / 64, 64, 0, j, m, cols, ncols, hA, hB, nrm, nrm2,
-            flag, hstride, Hh, cs, sn, g, est, inv_hn);
 }
 
 __global__ void k_lsq(int m, const int* __restrict__ cols, int ncols, const int* __restrict__ kcol,

@@ -150,8 +150,8 @@ struct hz_handle {
   // FGMRES workspace
   int rcap = 0;
   int mcap = 0;
-  DBuf Bd, Xd, V, Z, part, hA, hB, nr, nr2, flag, Hh, cs, sn, gv, yv, est, invhn, bnorm, bnorm_inv, beta, beta_inv,
-      cols, kcol;
+  DBuf Bd, Xd, V, Z, part, hA, hB, nr, flag, Hh, cs, sn, gv, yv, bnorm, bnorm_inv, beta, beta_inv, cols, kcol;
+  DBuf gscnt;       // block counters of the Gram-Schmidt kernels
   DBuf bsc;         // BiCGSTAB per-column scalars
   DBuf sig, hC;     // FGMRES basis scales (stored v_i stands for sig_i v_i) and update coefficients
   DBuf tmpA, tmpB;  // hz_apply staging
@@ -653,21 +653,19 @@ void ensure_workspace(hz_handle* h, int nrhs) {
   h->bsc.alloc((size_t)R * 8 * 16);
   h->sig.alloc((size_t)R * (m + 1) * sizeof(double));
   h->hC.alloc((size_t)R * (m + 2) * 16);
-  const int nblk = krylov_nblk(N, 1);
-  h->part.alloc((size_t)R * 18 * nblk * 16);
+  h->part.alloc(gs_part_bytes(N, R));
+  h->gscnt.alloc((size_t)R * sizeof(int));
+  ck(cudaMemsetAsync(h->gscnt.p, 0, (size_t)R * sizeof(int), h->ctx.stream), "zero block counters");
   const int HS = m + 2;
   h->hA.alloc((size_t)R * HS * 16);
   h->hB.alloc((size_t)R * HS * 16);
   h->nr.alloc((size_t)R * HS * 16);
-  h->nr2.alloc((size_t)R * HS * 16);
   h->flag.alloc((size_t)R * sizeof(int));
   h->Hh.alloc((size_t)R * (m + 1) * m * 16);
   h->cs.alloc((size_t)R * m * 16);
   h->sn.alloc((size_t)R * m * 16);
   h->gv.alloc((size_t)R * (m + 1) * 16);
   h->yv.alloc((size_t)R * m * 16);
-  h->est.alloc((size_t)R * 8);
-  h->invhn.alloc((size_t)R * 8);
   h->bnorm.alloc((size_t)R * 8);
   h->bnorm_inv.alloc((size_t)R * 8);
   h->beta.alloc((size_t)R * 8);
@@ -1091,7 +1089,7 @@ void col_norms(hz_handle* h, const double2* x, const std::vector<int>& cols, dou
   const int nblk = krylov_nblk(N, nc);
   const int* dc = h->cols.as<int>();
   const int HS = h->mcap + 2;
-  launch_dots(h->ctx, N, x, 0, N, 0, 0, x, N, dc, nc, nblk, 1, h->part.as<double2>());
+  launch_dots(h->ctx, N, x, N, 0, x, N, dc, nc, nblk, 1, h->part.as<double2>());
   launch_reduce(h->ctx, h->part.as<double2>(), dc, nc, 1, nblk, h->nr.as<double2>(), HS, 0);
   launch_norms(h->ctx, h->nr.as<double2>(), HS, 0, dc, nc, dev_nrm, dev_inv);
   if (host_out) {
@@ -1336,7 +1334,6 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
   const long long vstride = h->rcap;
   auto Vj = [&](int j) { return V + (long long)j * vstride * N; };
   auto Zj = [&](int j) { return (char*)h->Z.p + (size_t)j * vstride * N * zb; };
-  double2* part = h->part.as<double2>();
   int* dc = h->cols.as<int>();
 
   std::vector<int> all(nrhs);
@@ -1379,9 +1376,25 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
   launch_cycle_init(h->ctx, m, dc, (int)act.size(), h->bnorm.as<double>(), h->gv.as<double2>());
   // the basis is normalised lazily: stored v_i stands for sig_i v_i (V_0 is normalised)
   double* sig = h->sig.as<double>();
-  double2* hC = h->hC.as<double2>();
   const int SS = m + 1;
   launch_sig_init(h->ctx, dc, (int)act.size(), sig, SS);
+  GsColumn gs;
+  gs.m = m;
+  gs.hA = h->hA.as<double2>();
+  gs.hB = h->hB.as<double2>();
+  gs.coef = h->hC.as<double2>();
+  gs.hstride = HS;
+  gs.sig = sig;
+  gs.sstride = SS;
+  gs.Hh = h->Hh.as<double2>();
+  gs.cs = h->cs.as<double2>();
+  gs.sn = h->sn.as<double2>();
+  gs.g = h->gv.as<double2>();
+  gs.flag = h->flag.as<int>();
+  gs.host_est = h->h_est;
+  gs.host_flag = h->h_flag;
+  gs.count = h->gscnt.as<int>();
+  gs.part = h->part.as<double>();
   std::vector<int> kcol(h->rcap, 0);
   int outer = 0;
   for (outer = 1; outer <= std::max(1, h->opt.max_outer); ++outer) {
@@ -1390,7 +1403,6 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
     for (int j = 0; j < m && !live.empty(); ++j) {
       upload_cols(h, live);
       const int nl = (int)live.size();
-      double2* w = Vj(j + 1);
       if (df) {
         // the cycle reads the high parts of the df64 basis vector as its FP32 right-hand side
         cycle_graph(h, adj, j, nl, 2, [&] { mg_cycle<float, df64_tag>(h, H, 0, Vdj(j), (float2*)Zj(j), dc, nl); });
@@ -1400,54 +1412,21 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
       } else {
         cycle_graph(h, adj, j, nl, mixed ? 1 : 0, [&] { precondition(h, H, Vj(j), Zj(j), dc, nl); });
         if (mixed)
-          apply_H<float>(h, adj, MODE_APPLY, (const float2*)Zj(j), nullptr, w, dc, nl);
+          apply_H<float>(h, adj, MODE_APPLY, (const float2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
         else
-          apply_H<double>(h, adj, MODE_APPLY, (const double2*)Zj(j), nullptr, w, dc, nl);
+          apply_H<double>(h, adj, MODE_APPLY, (const double2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
       }
-      // classical Gram-Schmidt with the DGKS test: pass 1 (dots + ||w||^2,
-      // update + ||w'||^2) for every column, pass 2 only for the columns whose
-      // norm dropped below 1/sqrt(2) of its value (masked on the device)
+      // classical Gram-Schmidt with the DGKS test: pass 0 (dots + ||w||^2, update +
+      // ||w'||^2) for every column, pass 1 only for the columns whose norm dropped below
+      // 1/sqrt(2) of its value (masked on the device); the Hessenberg column, rotation and
+      // residual estimate follow in the column's last pass.  v_{j+1} = w'' stays
+      // unnormalised: sig_{j+1} = sig_j / h_{j+1,j}.  The estimates arrive in pinned memory.
       const int K = j + 1;
-      const int nblk = krylov_nblk(N, nl);
-      double2* hA = h->hA.as<double2>();
-      double2* hB = h->hB.as<double2>();
-      int* flag = h->flag.as<int>();
-      for (int pass = 0; pass < 2; ++pass) {
-        double2* hh = pass == 0 ? hA : hB;
-        double2* nrm = pass == 0 ? h->nr.as<double2>() : h->nr2.as<double2>();
-        const int* mask = pass == 0 ? nullptr : flag;
-        for (int i0 = 0; i0 < K; i0 += 16) {
-          const int k = std::min(16, K - i0);
-          const int wn = (pass == 0 && i0 + 16 >= K) ? 1 : 0;  // ||w||^2 before the update (slot K)
-          if (df)
-            launch_dots_df(h->ctx, N, Vd, vstride, N, i0, k, Vdj(j + 1), N, dc, nl, nblk, wn, part, mask);
-          else
-            launch_dots(h->ctx, N, V, vstride, N, i0, k, w, N, dc, nl, nblk, wn, part, mask);
-          launch_reduce(h->ctx, part, dc, nl, k + wn, nblk, hh + i0, HS, 0);
-        }
-        // update coefficients for the stored vectors: sig_i^2 d_i
-        launch_sig_coef(h->ctx, dc, nl, K, sig, SS, hh, HS, hC);
-        for (int i0 = 0; i0 < K; i0 += 16) {
-          const int k = std::min(16, K - i0);
-          const int wn = (i0 + 16 >= K) ? 1 : 0;
-          if (df)
-            launch_update_df(h->ctx, N, Vd, vstride, N, i0, k, hC, HS, Vdj(j + 1), N, dc, nl, nblk, wn, part, mask);
-          else
-            launch_update(h->ctx, N, V, vstride, N, i0, k, hC, HS, w, N, dc, nl, nblk, wn, part, mask);
-          if (wn) launch_reduce(h->ctx, part, dc, nl, 1, nblk, nrm, HS, 0);
-        }
-        if (pass == 0) launch_dgks(h->ctx, dc, nl, hA, HS, K, h->nr.as<double2>(), HS, flag);
-      }
-      // Hessenberg entries of the normalised basis: sig_i sig_j d_i, h_{j+1,j} = sig_j ||w''||
-      launch_sig_true(h->ctx, j, dc, nl, sig, SS, hA, hB, h->nr.as<double2>(), h->nr2.as<double2>(), HS);
-      launch_arnoldi_step(h->ctx, j, m, dc, nl, hA, hB, h->nr.as<double2>(), h->nr2.as<double2>(), flag, HS,
-                          h->Hh.as<double2>(), h->cs.as<double2>(), h->sn.as<double2>(), h->gv.as<double2>(),
-                          h->est.as<double>(), h->invhn.as<double>());
-      // v_{j+1} = w'' stays unnormalised: sig_{j+1} = sig_j / h_{j+1,j}
-      launch_sig_next(h->ctx, j, dc, nl, sig, SS, h->invhn.as<double>());
-      ck(cudaMemcpyAsync(h->h_est, h->est.p, (size_t)h->rcap * 8, cudaMemcpyDeviceToHost, h->ctx.stream), "est");
-      ck(cudaMemcpyAsync(h->h_flag, h->flag.p, (size_t)h->rcap * sizeof(int), cudaMemcpyDeviceToHost, h->ctx.stream),
-         "flags");
+      for (int pass = 0; pass < 2; ++pass)
+        if (df)
+          launch_gs_pass_df(h->ctx, N, Vd, vstride, N, j, pass, dc, nl, gs);
+        else
+          launch_gs_pass(h->ctx, N, V, vstride, N, j, pass, dc, nl, gs);
       sync(h);
       {
         int n2 = 0;  // columns that took the second Gram-Schmidt pass
@@ -1584,7 +1563,7 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
     na = (int)act.size();
     int nblk = krylov_nblk(N, na);
     // <rh, r> and ||r||^2 in one pass
-    launch_dots(h->ctx, N, rh, 0, N, 0, 1, r, N, dc, na, nblk, 1, part);
+    launch_dots(h->ctx, N, rh, N, 1, r, N, dc, na, nblk, 1, part);
     launch_reduce(h->ctx, part, dc, na, 2, nblk, red, HS, 0);
     launch_norms(h->ctx, red, HS, 1, dc, na, h->beta.as<double>(), nullptr);
     ck(cudaMemcpyAsync(h->h_nrm, h->beta.p, (size_t)h->rcap * 8, cudaMemcpyDeviceToHost, h->ctx.stream), "norms");
@@ -1612,7 +1591,7 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
       apply_H<float>(h, adj, MODE_APPLY, (const float2*)ph, nullptr, v, dc, na);
     else
       apply_H<double>(h, adj, MODE_APPLY, (const double2*)ph, nullptr, v, dc, na);
-    launch_dots(h->ctx, N, rh, 0, N, 0, 1, v, N, dc, na, nblk, 0, part);
+    launch_dots(h->ctx, N, rh, N, 1, v, N, dc, na, nblk, 0, part);
     launch_reduce(h->ctx, part, dc, na, 1, nblk, red, HS, 0);
     launch_bicg_scalars(h->ctx, 1, dc, na, red, HS, sc);
     launch_bicg_vec(h->ctx, 1, N, r, nullptr, v, sv, sc, dc, na);
@@ -1623,7 +1602,7 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
       apply_H<float>(h, adj, MODE_APPLY, (const float2*)sh, nullptr, t, dc, na);
     else
       apply_H<double>(h, adj, MODE_APPLY, (const double2*)sh, nullptr, t, dc, na);
-    launch_dots(h->ctx, N, sv, 0, N, 0, 1, t, N, dc, na, nblk, 1, part);
+    launch_dots(h->ctx, N, sv, N, 1, t, N, dc, na, nblk, 1, part);
     launch_reduce(h->ctx, part, dc, na, 2, nblk, red, HS, 0);
     launch_bicg_scalars(h->ctx, 2, dc, na, red, HS, sc);
     if (mixed)

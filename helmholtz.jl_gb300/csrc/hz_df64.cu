@@ -315,7 +315,7 @@ void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride
   if (ncols <= 0) return;
   float4* w = const_cast<float4*>(V) + (long long)(j + 1) * vstride * ld;
   const int K = j + 1;
-  const dim3 grid(krylov_nblk(N, ncols), ncols);
+  const dim3 grid(gs_nblk(N, ncols), ncols);
   const double el = pass ? 0.0 : (double)N * ncols;
   for (int i0 = 0; i0 < K; i0 += 16) {
     const int k = std::min(16, K - i0);

@@ -227,6 +227,7 @@ struct GsColumn {
   int* count = nullptr;                           // block counters, zero
   double* part = nullptr;                         // partial sums, gs_part_bytes
 };
+int gs_nblk(long long N, int ncols);
 size_t gs_part_bytes(long long N, int R);
 // the dots of step j (K = j + 1 vectors) and the update w -= sum coef_i V_i of one pass
 void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int j, int pass,

@@ -95,6 +95,9 @@ void launch_dots(Ctx& ctx, long long N, const double2* V, long long ld, int K, c
 // 200,000 nodes, waves, a point source's peak and noise: dots 3e-17 to 1.5e-16 of |V||w|
 // (native 5e-17 to 2.6e-16), update 6e-17 of |w'| rms (native 2.4e-16).
 static constexpr int kGsNodes = 4;
+// One vector in six stays on the FP64 pipe, which the integer dots leave idle (5 vectors, 129^3 x
+// 8: 465 -> 441 us; 10: 952 -> 932 us; one in four was no better).
+__host__ __device__ constexpr int gs_native(int vectors) { return (vectors + 1) / 6; }
 
 template <int KT>
 __global__ void __launch_bounds__(RT, 2) k_gs_dots(long long N, const double2* __restrict__ V, long long vstride,
@@ -142,7 +145,7 @@ __global__ void __launch_bounds__(RT, 2) k_gs_dots(long long N, const double2* _
     for (int s = 0; s < KT; ++s) {
       uint4 vr[kGsNodes];
       const int ev = load(vb + s * vs, p, vr);
-      if (wok && fixed_ref_ok(ev) && fixed_ok(ev + ew)) {
+      if (s >= gs_native(KT) && wok && fixed_ref_ok(ev) && fixed_ok(ev + ew)) {
         FixedSum f{0, 0, 0, 0};
 #pragma unroll
         for (int q = 0; q < kGsNodes; ++q)
@@ -242,6 +245,27 @@ __global__ void __launch_bounds__(RT, 2) k_gs_update(long long N, const double2*
 
 #define HZ_K_CASES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 
+// Blocks per column: two blocks fit an SM.  Four waves of them where a thread still has 64
+// nodes, else one wave, or as many as leave less than a tenth of the last one's slots empty:
+// a block's reduction costs as much as several nodes per thread.
+int gs_nblk(long long N, int ncols) {
+  const int slots = 2 * kSMs, cols = std::max(ncols, 1);
+  const long long most = std::max<long long>(1, (N + RT - 1) / RT);
+  auto blocks = [&](int waves) { return std::min<long long>(most, std::max(1, waves * slots / cols)); };
+  if (N >= 64 * RT * blocks(4)) return (int)blocks(4);
+  long long best = 1;
+  double eff = 0.0;
+  for (int waves = 1; waves <= 4; ++waves) {
+    const long long ctas = blocks(waves) * cols;
+    const double e = (double)ctas / (double)((ctas + slots - 1) / slots * slots);
+    if (e > eff + 0.1) {
+      best = blocks(waves);
+      eff = e;
+    }
+  }
+  return (int)best;
+}
+
 size_t gs_part_bytes(long long N, int R) { return (size_t)R * krylov_nblk(N, 1) * 33 * sizeof(double); }
 
 void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int j, int pass,
@@ -249,7 +273,7 @@ void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, 
   if (ncols <= 0) return;
   double2* w = const_cast<double2*>(V) + (long long)(j + 1) * vstride * ld;
   const int K = j + 1;
-  const dim3 grid(krylov_nblk(N, ncols), ncols);
+  const dim3 grid(gs_nblk(N, ncols), ncols);
   // a masked pass is charged by the host once it knows which columns took it
   const double el = pass ? 0.0 : (double)N * ncols;
   for (int i0 = 0; i0 < K; i0 += 16) {

@@ -152,6 +152,7 @@ struct hz_handle {
   int mcap = 0;
   DBuf Bd, Xd, V, Z, part, hA, hB, nr, flag, Hh, cs, sn, gv, yv, bnorm, bnorm_inv, beta, beta_inv, cols, kcol;
   DBuf gscnt;       // block counters of the Gram-Schmidt kernels
+  std::vector<int> cols_on_device;  // what cols holds
   DBuf bsc;         // BiCGSTAB per-column scalars
   DBuf sig, hC;     // FGMRES basis scales (stored v_i stands for sig_i v_i) and update coefficients
   DBuf tmpA, tmpB;  // hz_apply staging
@@ -179,7 +180,7 @@ struct hz_handle {
   int net_feat_level = -1;
   double net_h2 = 0.0;       // hx * hy of the network level
   DBuf net_feat;             // per node of the network level: (w^2 m hx hy, gamma / w), float2
-  // CUDA graphs of the preconditioner application, one per (orientation, basis
+  // CUDA graphs of one Krylov iteration, one per (orientation, basis
   // index, active columns, form); launch-table deltas of the captured kernels
   struct CycleGraph {
     cudaGraphExec_t exec = nullptr;
@@ -671,6 +672,7 @@ void ensure_workspace(hz_handle* h, int nrhs) {
   h->beta.alloc((size_t)R * 8);
   h->beta_inv.alloc((size_t)R * 8);
   h->cols.alloc((size_t)R * sizeof(int));
+  h->cols_on_device.clear();
   h->kcol.alloc((size_t)R * sizeof(int));
   if (h->h_est) cudaFreeHost(h->h_est);
   if (h->h_nrm) cudaFreeHost(h->h_nrm);
@@ -1074,11 +1076,16 @@ void apply_H(hz_handle* h, int adj, int mode, const cplx<TX>* x, const double2* 
                                   0.0);
 }
 
+// The active columns' list on the device; nothing to do where it is there already (most
+// iterations: columns leave a block only as they converge).
 void upload_cols(hz_handle* h, const std::vector<int>& c) {
+  if (h->cols_on_device == c) return;
+  h->cols_on_device.clear();
   ck(cudaMemcpyAsync(h->cols.p, c.data(), c.size() * sizeof(int), cudaMemcpyHostToDevice, h->ctx.stream),
      "upload cols");
   // the host vector must stay valid until the copy is done
   ck(cudaStreamSynchronize(h->ctx.stream), "sync cols");
+  h->cols_on_device = c;
 }
 
 // Column 2-norms of a block into host memory.
@@ -1238,8 +1245,8 @@ void drop_graphs(hz_handle* h) {
   h->graphs.clear();
 }
 
-// Run body (the launches of one preconditioner application) through a CUDA
-// graph: captured on the second application with the same key, replayed from
+// Run body (the launches of one Krylov iteration: the preconditioner application, the
+// operator and the method's own kernels) through a CUDA graph: captured on the second application with the same key, replayed from
 // then on.  The graph's kernels keep their launch counts in the table; with
 // profiling on, a replay is timed as one "vcycle_graph" entry carrying the
 // algorithmic bytes of all its kernels.  A failed capture (an API the graph
@@ -1403,30 +1410,33 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
     for (int j = 0; j < m && !live.empty(); ++j) {
       upload_cols(h, live);
       const int nl = (int)live.size();
-      if (df) {
-        // the cycle reads the high parts of the df64 basis vector as its FP32 right-hand side
-        cycle_graph(h, adj, j, nl, 2, [&] { mg_cycle<float, df64_tag>(h, H, 0, Vdj(j), (float2*)Zj(j), dc, nl); });
-        FineOp fop = h->fop;
-        fop.adj = adj;
-        launch_fine_df64(h->ctx, fop, h->diagHdf.as<float4>(), (const float2*)Zj(j), Vdj(j + 1), N, dc, nl);
-      } else {
-        cycle_graph(h, adj, j, nl, mixed ? 1 : 0, [&] { precondition(h, H, Vj(j), Zj(j), dc, nl); });
-        if (mixed)
-          apply_H<float>(h, adj, MODE_APPLY, (const float2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
-        else
-          apply_H<double>(h, adj, MODE_APPLY, (const double2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
-      }
-      // classical Gram-Schmidt with the DGKS test: pass 0 (dots + ||w||^2, update +
-      // ||w'||^2) for every column, pass 1 only for the columns whose norm dropped below
-      // 1/sqrt(2) of its value (masked on the device); the Hessenberg column, rotation and
-      // residual estimate follow in the column's last pass.  v_{j+1} = w'' stays
-      // unnormalised: sig_{j+1} = sig_j / h_{j+1,j}.  The estimates arrive in pinned memory.
       const int K = j + 1;
-      for (int pass = 0; pass < 2; ++pass)
-        if (df)
-          launch_gs_pass_df(h->ctx, N, Vd, vstride, N, j, pass, dc, nl, gs);
-        else
-          launch_gs_pass(h->ctx, N, V, vstride, N, j, pass, dc, nl, gs);
+      // One iteration's device work.  Classical Gram-Schmidt with the DGKS test: pass 0
+      // (dots + ||w||^2, update + ||w'||^2) for every column, pass 1 only for the columns
+      // whose norm dropped below 1/sqrt(2) of its value (masked on the device); the
+      // Hessenberg column, rotation and residual estimate follow in the column's last pass.
+      // v_{j+1} = w'' stays unnormalised: sig_{j+1} = sig_j / h_{j+1,j}.  The estimates
+      // arrive in pinned memory.
+      cycle_graph(h, adj, j, nl, df ? 2 : mixed ? 1 : 0, [&] {
+        if (df) {
+          // the cycle reads the high parts of the df64 basis vector as its FP32 right-hand side
+          mg_cycle<float, df64_tag>(h, H, 0, Vdj(j), (float2*)Zj(j), dc, nl);
+          FineOp fop = h->fop;
+          fop.adj = adj;
+          launch_fine_df64(h->ctx, fop, h->diagHdf.as<float4>(), (const float2*)Zj(j), Vdj(j + 1), N, dc, nl);
+        } else {
+          precondition(h, H, Vj(j), Zj(j), dc, nl);
+          if (mixed)
+            apply_H<float>(h, adj, MODE_APPLY, (const float2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
+          else
+            apply_H<double>(h, adj, MODE_APPLY, (const double2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
+        }
+        for (int pass = 0; pass < 2; ++pass)
+          if (df)
+            launch_gs_pass_df(h->ctx, N, Vd, vstride, N, j, pass, dc, nl, gs);
+          else
+            launch_gs_pass(h->ctx, N, V, vstride, N, j, pass, dc, nl, gs);
+      });
       sync(h);
       {
         int n2 = 0;  // columns that took the second Gram-Schmidt pass
@@ -1503,8 +1513,8 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
   return std::min(outer, std::max(1, h->opt.max_outer));
 }
 
-// Graph keys of BiCGSTAB's two preconditioner applications (FGMRES uses its basis
-// index, below the restart limit of 64); the handle runs one Krylov method.
+// Graph key of a BiCGSTAB iteration (FGMRES uses its basis index, below the restart
+// limit of 64); the handle runs one Krylov method.
 static constexpr int kBicgKey = 64;
 
 // Right-preconditioned BiCGSTAB on H (or H^H), one multigrid cycle per
@@ -1559,13 +1569,24 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
   launch_bicg_scalars(h->ctx, -1, dc, na, red, HS, sc);
   const int maxit = std::max(1, h->opt.max_outer);
   int it = 0;
+  // <rh, r> and ||r||^2 in one pass, the norms
+  auto head = [&](int nc) {
+    const int nblk = krylov_nblk(N, nc);
+    launch_dots(h->ctx, N, rh, N, 1, r, N, dc, nc, nblk, 1, part);
+    launch_reduce(h->ctx, part, dc, nc, 2, nblk, red, HS, 0);
+    launch_norms(h->ctx, red, HS, 1, dc, nc, h->beta.as<double>(), nullptr);
+  };
+  // y = H z for the preconditioned vector z
+  auto apply = [&](const void* z, double2* y, int nc) {
+    if (emu)
+      launch_fine_df64<double2>(h->ctx, fopa, h->diagHdf.as<float4>(), (const float2*)z, y, N, dc, nc);
+    else if (mixed)
+      apply_H<float>(h, adj, MODE_APPLY, (const float2*)z, nullptr, y, dc, nc);
+    else
+      apply_H<double>(h, adj, MODE_APPLY, (const double2*)z, nullptr, y, dc, nc);
+  };
+  head(na);
   for (; it <= maxit; ++it) {
-    na = (int)act.size();
-    int nblk = krylov_nblk(N, na);
-    // <rh, r> and ||r||^2 in one pass
-    launch_dots(h->ctx, N, rh, N, 1, r, N, dc, na, nblk, 1, part);
-    launch_reduce(h->ctx, part, dc, na, 2, nblk, red, HS, 0);
-    launch_norms(h->ctx, red, HS, 1, dc, na, h->beta.as<double>(), nullptr);
     ck(cudaMemcpyAsync(h->h_nrm, h->beta.p, (size_t)h->rcap * 8, cudaMemcpyDeviceToHost, h->ctx.stream), "norms");
     sync(h);
     std::vector<int> still;
@@ -1578,37 +1599,30 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
       act.swap(still);
       if (act.empty()) break;
       upload_cols(h, act);
-      na = (int)act.size();
-      nblk = krylov_nblk(N, na);
     }
     if (it == maxit) break;
-    launch_bicg_scalars(h->ctx, 0, dc, na, red, HS, sc);
-    launch_bicg_vec(h->ctx, 0, N, r, p, v, nullptr, sc, dc, na);
-    cycle_graph(h, adj, kBicgKey, na, mixed ? 1 : 0, [&] { precondition(h, H, p, ph, dc, na); });
-    if (emu)
-      launch_fine_df64<double2>(h->ctx, fopa, h->diagHdf.as<float4>(), (const float2*)ph, v, N, dc, na);
-    else if (mixed)
-      apply_H<float>(h, adj, MODE_APPLY, (const float2*)ph, nullptr, v, dc, na);
-    else
-      apply_H<double>(h, adj, MODE_APPLY, (const double2*)ph, nullptr, v, dc, na);
-    launch_dots(h->ctx, N, rh, N, 1, v, N, dc, na, nblk, 0, part);
-    launch_reduce(h->ctx, part, dc, na, 1, nblk, red, HS, 0);
-    launch_bicg_scalars(h->ctx, 1, dc, na, red, HS, sc);
-    launch_bicg_vec(h->ctx, 1, N, r, nullptr, v, sv, sc, dc, na);
-    cycle_graph(h, adj, kBicgKey + 1, na, mixed ? 1 : 0, [&] { precondition(h, H, sv, sh, dc, na); });
-    if (emu)
-      launch_fine_df64<double2>(h->ctx, fopa, h->diagHdf.as<float4>(), (const float2*)sh, t, N, dc, na);
-    else if (mixed)
-      apply_H<float>(h, adj, MODE_APPLY, (const float2*)sh, nullptr, t, dc, na);
-    else
-      apply_H<double>(h, adj, MODE_APPLY, (const double2*)sh, nullptr, t, dc, na);
-    launch_dots(h->ctx, N, sv, N, 1, t, N, dc, na, nblk, 1, part);
-    launch_reduce(h->ctx, part, dc, na, 2, nblk, red, HS, 0);
-    launch_bicg_scalars(h->ctx, 2, dc, na, red, HS, sc);
-    if (mixed)
-      launch_bicg_xr<float>(h->ctx, N, X, (const float2*)ph, (const float2*)sh, sv, t, r, sc, dc, na);
-    else
-      launch_bicg_xr<double>(h->ctx, N, X, (const double2*)ph, (const double2*)sh, sv, t, r, sc, dc, na);
+    na = (int)act.size();
+    cycle_graph(h, adj, kBicgKey, na, mixed ? 1 : 0, [&] {
+      const int nblk = krylov_nblk(N, na);
+      launch_bicg_scalars(h->ctx, 0, dc, na, red, HS, sc);
+      launch_bicg_vec(h->ctx, 0, N, r, p, v, nullptr, sc, dc, na);
+      precondition(h, H, p, ph, dc, na);
+      apply(ph, v, na);
+      launch_dots(h->ctx, N, rh, N, 1, v, N, dc, na, nblk, 0, part);
+      launch_reduce(h->ctx, part, dc, na, 1, nblk, red, HS, 0);
+      launch_bicg_scalars(h->ctx, 1, dc, na, red, HS, sc);
+      launch_bicg_vec(h->ctx, 1, N, r, nullptr, v, sv, sc, dc, na);
+      precondition(h, H, sv, sh, dc, na);
+      apply(sh, t, na);
+      launch_dots(h->ctx, N, sv, N, 1, t, N, dc, na, nblk, 1, part);
+      launch_reduce(h->ctx, part, dc, na, 2, nblk, red, HS, 0);
+      launch_bicg_scalars(h->ctx, 2, dc, na, red, HS, sc);
+      if (mixed)
+        launch_bicg_xr<float>(h->ctx, N, X, (const float2*)ph, (const float2*)sh, sv, t, r, sc, dc, na);
+      else
+        launch_bicg_xr<double>(h->ctx, N, X, (const double2*)ph, (const double2*)sh, sv, t, r, sc, dc, na);
+      head(na);
+    });
     for (int c : act) {
       h->col_iters[c] += 1;
       h->nprec += 2;

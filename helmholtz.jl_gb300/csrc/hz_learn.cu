@@ -251,129 +251,13 @@ __global__ void k_wflip(int Cout, int Cin, int K, const bf16* __restrict__ w, bf
   wt[idx] = (co < Cout) ? w[((long long)co * 9 + (8 - t)) * Cin + ci] : __float2bfloat16_rn(0.f);
 }
 
-// Per-channel resampling between grid levels (NHWC bf16, FP32 arithmetic).
-// mode 0, restriction (fine -> coarse): full weighting with weights 1, 1/2 per
-// axis, normalised by the weights that fall inside the grid.
-// mode 1, prolongation (coarse -> fine): bilinear, (c[i0] + c[i1]) / 2 per axis
-// with i0 = i / 2, i1 = (i + 1) / 2.
-// transpose = 1 applies the adjoint (fine <- coarse for mode 0, coarse <- fine for
-// mode 1).  The result, zeroed where mask <= 0 (mask may be null), is written or,
-// with accum, added to out (rounded to bf16 once).
-
-// One thread per (node, 8 channels): 16-byte loads and stores (every channel
-// count and offset is a multiple of 8).
-struct F8 {
-  float v[8];
-};
-__device__ __forceinline__ void ld8(const bf16* p, F8& f) {
-  const uint4 u = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 x = __bfloat1622float2(h[k]);
-    f.v[2 * k] = x.x;
-    f.v[2 * k + 1] = x.y;
-  }
-}
-__device__ __forceinline__ void axpy8(float a, const bf16* p, F8& acc) {
-  F8 f;
-  ld8(p, f);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc.v[k] = fmaf(a, f.v[k], acc.v[k]);
-}
-
-__global__ void k_resample(int mode, int transpose, int nxf, int nyf, int nxc, int nyc, int B, int C,
-                           const bf16* __restrict__ in, int ldi, int i_off, bf16* __restrict__ out, int ldo, int o_off,
-                           int accum, const bf16* __restrict__ mask, int ldm, int m_off) {
-  const int Nf = nxf * nyf, Nc = nxc * nyc;
-  const bool to_coarse = (mode == 0) != (transpose != 0);
-  const int No = to_coarse ? Nc : Nf, Ni = to_coarse ? Nf : Nc;
-  const int C8 = C / 8;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= B * No * C8) return;
-  const int c = (idx % C8) * 8;
-  const int q = idx / C8;
-  const int b = q / No, po = q % No;
-  const bf16* ib = in + (long long)b * Ni * ldi + i_off + c;
-  F8 acc;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc.v[k] = 0.f;
-  if (mode == 0 && !transpose) {  // restriction
-    const int I = po % nxc, J = po / nxc;
-    float wsum = 0.f;
-    for (int dj = -1; dj <= 1; ++dj)
-      for (int di = -1; di <= 1; ++di) {
-        const int fi = 2 * I + di, fj = 2 * J + dj;
-        if (fi < 0 || fi >= nxf || fj < 0 || fj >= nyf) continue;
-        const float wg = (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f);
-        axpy8(wg, ib + (long long)(fi + fj * nxf) * ldi, acc);
-        wsum += wg;
-      }
-    const float inv = 1.f / wsum;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc.v[k] *= inv;
-  } else if (mode == 0) {  // adjoint of the restriction: fine <- coarse parents I with |i - 2I| <= 1
-    const int i = po % nxf, j = po / nxf;
-    for (int J = j / 2 - 1; J <= j / 2 + 1; ++J)
-      for (int I = i / 2 - 1; I <= i / 2 + 1; ++I) {
-        if (I < 0 || I >= nxc || J < 0 || J >= nyc) continue;
-        const int di = i - 2 * I, dj = j - 2 * J;
-        if (di < -1 || di > 1 || dj < -1 || dj > 1) continue;
-        const float sx = 1.f + (2 * I - 1 >= 0 ? 0.5f : 0.f) + (2 * I + 1 < nxf ? 0.5f : 0.f);
-        const float sy = 1.f + (2 * J - 1 >= 0 ? 0.5f : 0.f) + (2 * J + 1 < nyf ? 0.5f : 0.f);
-        axpy8((di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) / (sx * sy), ib + (long long)(I + J * nxc) * ldi, acc);
-      }
-  } else if (!transpose) {  // prolongation
-    const int i = po % nxf, j = po / nxf;
-    const int i0 = i >> 1, i1 = (i + 1) >> 1, j0 = j >> 1, j1 = (j + 1) >> 1;
-    axpy8(1.f, ib + (long long)(i0 + j0 * nxc) * ldi, acc);
-    axpy8(1.f, ib + (long long)(i1 + j0 * nxc) * ldi, acc);
-    axpy8(1.f, ib + (long long)(i0 + j1 * nxc) * ldi, acc);
-    axpy8(1.f, ib + (long long)(i1 + j1 * nxc) * ldi, acc);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc.v[k] *= 0.25f;
-  } else {  // adjoint of the prolongation: coarse <- fine children
-    const int I = po % nxc, J = po / nxc;
-    for (int fj = 2 * J - 1; fj <= 2 * J + 1; ++fj)
-      for (int fi = 2 * I - 1; fi <= 2 * I + 1; ++fi) {
-        if (fi < 0 || fi >= nxf || fj < 0 || fj >= nyf) continue;
-        axpy8((fi == 2 * I ? 1.f : 0.5f) * (fj == 2 * J ? 1.f : 0.5f), ib + (long long)(fi + fj * nxf) * ldi, acc);
-      }
-  }
-  const long long row = (long long)b * No + po;
-  if (mask) {
-    F8 mk;
-    ld8(mask + row * ldm + m_off + c, mk);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (!(mk.v[k] > 0.f)) acc.v[k] = 0.f;
-  }
-  bf16* o = out + row * ldo + o_off + c;
-  if (accum) {
-    F8 old;
-    ld8(o, old);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc.v[k] += old.v[k];
-  }
-  __align__(16) __nv_bfloat162 r[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) r[k] = __floats2bfloat162_rn(acc.v[2 * k], acc.v[2 * k + 1]);
-  *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(r);
-}
-
+// Per-channel transfer between grid level lf and the next coarser one (hz_resample.cu).
 static void resample(Ctx& ctx, int mode, int transpose, const int* gx, const int* gy, int lf, int B, int C,
                      const bf16* in, int ldi, int i_off, bf16* out, int ldo, int o_off, int accum,
                      const bf16* mask = nullptr, int ldm = 0, int m_off = 0) {
-  if (C % 8 || ldi % 8 || i_off % 8 || ldo % 8 || o_off % 8 || (mask && (ldm % 8 || m_off % 8)))
-    throw std::runtime_error("resample: channel layout not aligned");
-  const int nxf = gx[lf], nyf = gy[lf], nxc = gx[lf + 1], nyc = gy[lf + 1];
-  const bool to_coarse = (mode == 0) != (transpose != 0);
-  const long long no = to_coarse ? (long long)nxc * nyc : (long long)nxf * nyf;
-  const long long ni = to_coarse ? (long long)nxf * nyf : (long long)nxc * nyc;
-  const long long total = (long long)B * no * (C / 8);
-  if (total >= (1LL << 31)) throw std::runtime_error("resample: batch too large");
-  HZ_LAUNCH(ctx, "net_resample", (double)B * (no + ni) * C * 2.0, k_resample, (unsigned)((total + 255) / 256), 256, 0,
-            mode, transpose, nxf, nyf, nxc, nyc, B, C, in, ldi, i_off, out, ldo, o_off, accum, mask, ldm, m_off);
+  const int f[2] = {gx[lf], gy[lf]}, c[2] = {gx[lf + 1], gy[lf + 1]};
+  launch_resample(ctx, "net_resample", mode, transpose, f, c, false, B, C, in, ldi, i_off, out, ldo, o_off, accum, mask,
+                  ldm, m_off);
 }
 
 // input assembly: X[b][p][0..16) = (x4[b][p][0..4), 0...) in bf16

@@ -249,6 +249,11 @@ class CoarseNet3 {
 // 16-channel rows, the loss and its gradient, Adam, FP32 -> BF16, and the
 // mini-batch gather of training pairs.
 __global__ void k_pack_in(long long BN, const float4* __restrict__ x4, __nv_bfloat16* __restrict__ x16);
+// Transfer of C channels between a fine and the next coarser grid: mode 0 full weighting, 1
+// prolongation, transpose: the adjoint; accum adds to out, mask zeroes where it is <= 0.
+void launch_resample(Ctx& ctx, const char* name, int mode, int transpose, const int* fine, const int* coarse, bool d3,
+                     int B, int C, const __nv_bfloat16* in, int ldi, int i_off, __nv_bfloat16* out, int ldo, int o_off,
+                     int accum, const __nv_bfloat16* mask, int ldm, int m_off);
 static constexpr int kLossChunks = 32;  // CTAs per sample
 size_t net_loss_bytes(int B);
 void launch_net_loss(Ctx& c, const char* name, int N, int B, const float* y, const float* t, __nv_bfloat16* dy,

@@ -281,136 +281,12 @@ __global__ void k_wflip3(int Cout, int Cin, int K, const bf16* __restrict__ w, b
   wt[idx] = (co < Cout) ? w[((long long)co * kTaps3 + (kTaps3 - 1 - t)) * Cin + ci] : __float2bfloat16_rn(0.f);
 }
 
-// Per-channel resampling between 3D grid levels (NDHWC bf16, FP32 arithmetic),
-// the 3D counterparts of the 2D network's transfers:
-// mode 0, restriction (fine -> coarse): full weighting, weights 1, 1/2 per axis,
-// normalised by the weights that fall inside the grid (the product of the 1D sums).
-// mode 1, prolongation (coarse -> fine): trilinear, the mean of c[i0] and c[i1]
-// per axis with i0 = i / 2, i1 = (i + 1) / 2.
-// transpose = 1 applies the adjoint.  The result, zeroed where mask <= 0 (mask
-// may be null), is written or, with accum, added to out (rounded to bf16 once).
-// One thread per (node, 8 channels): 16-byte loads and stores.
-struct F8x {
-  float v[8];
-};
-__device__ __forceinline__ void ld8x(const bf16* p, F8x& f) {
-  const uint4 u = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 x = __bfloat1622float2(h[k]);
-    f.v[2 * k] = x.x;
-    f.v[2 * k + 1] = x.y;
-  }
-}
-__device__ __forceinline__ void axpy8x(float a, const bf16* p, F8x& acc) {
-  F8x f;
-  ld8x(p, f);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc.v[k] = fmaf(a, f.v[k], acc.v[k]);
-}
-// 1D full-weighting sum of coarse node I on an axis of nf fine nodes
-__device__ __forceinline__ float fw_sum(int I, int nf) {
-  return 1.f + (2 * I - 1 >= 0 ? 0.5f : 0.f) + (2 * I + 1 < nf ? 0.5f : 0.f);
-}
-
-__global__ void k_resample3(int mode, int transpose, int nxf, int nyf, int nzf, int nxc, int nyc, int nzc, int B,
-                            int C, const bf16* __restrict__ in, int ldi, int i_off, bf16* __restrict__ out, int ldo,
-                            int o_off, int accum, const bf16* __restrict__ mask, int ldm, int m_off) {
-  const long long Nf = (long long)nxf * nyf * nzf, Nc = (long long)nxc * nyc * nzc;
-  const bool to_coarse = (mode == 0) != (transpose != 0);
-  const long long No = to_coarse ? Nc : Nf, Ni = to_coarse ? Nf : Nc;
-  const int C8 = C / 8;
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)B * No * C8) return;
-  const int c = (int)(idx % C8) * 8;
-  const long long q = idx / C8;
-  const int b = (int)(q / No);
-  const long long po = q % No;
-  const bf16* ib = in + (long long)b * Ni * ldi + i_off + c;
-  F8x acc;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc.v[k] = 0.f;
-  const int nxo = to_coarse ? nxc : nxf, nyo = to_coarse ? nyc : nyf;
-  const int io = (int)(po % nxo);
-  const long long t = po / nxo;
-  const int jo = (int)(t % nyo), ko = (int)(t / nyo);
-  if (mode == 0 && !transpose) {  // restriction: coarse (io, jo, ko) <- fine 2I + d
-    for (int dk = -1; dk <= 1; ++dk)
-      for (int dj = -1; dj <= 1; ++dj)
-        for (int di = -1; di <= 1; ++di) {
-          const int fi = 2 * io + di, fj = 2 * jo + dj, fk = 2 * ko + dk;
-          if (fi < 0 || fi >= nxf || fj < 0 || fj >= nyf || fk < 0 || fk >= nzf) continue;
-          const float wg = (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * (dk ? 0.5f : 1.f);
-          axpy8x(wg, ib + (fi + (long long)nxf * (fj + (long long)nyf * fk)) * ldi, acc);
-        }
-    const float inv = 1.f / (fw_sum(io, nxf) * fw_sum(jo, nyf) * fw_sum(ko, nzf));
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc.v[k] *= inv;
-  } else if (mode == 0) {  // adjoint of the restriction: fine (io, jo, ko) <- coarse parents
-    for (int K = ko / 2 - 1; K <= ko / 2 + 1; ++K)
-      for (int J = jo / 2 - 1; J <= jo / 2 + 1; ++J)
-        for (int I = io / 2 - 1; I <= io / 2 + 1; ++I) {
-          if (I < 0 || I >= nxc || J < 0 || J >= nyc || K < 0 || K >= nzc) continue;
-          const int di = io - 2 * I, dj = jo - 2 * J, dk = ko - 2 * K;
-          if (di < -1 || di > 1 || dj < -1 || dj > 1 || dk < -1 || dk > 1) continue;
-          const float wg = (di ? 0.5f : 1.f) * (dj ? 0.5f : 1.f) * (dk ? 0.5f : 1.f) /
-                           (fw_sum(I, nxf) * fw_sum(J, nyf) * fw_sum(K, nzf));
-          axpy8x(wg, ib + (I + (long long)nxc * (J + (long long)nyc * K)) * ldi, acc);
-        }
-  } else if (!transpose) {  // prolongation: fine (io, jo, ko) <- 8 coarse corners
-    const int i0 = io >> 1, i1 = (io + 1) >> 1, j0 = jo >> 1, j1 = (jo + 1) >> 1, k0 = ko >> 1, k1 = (ko + 1) >> 1;
-    const int is[2] = {i0, i1}, js[2] = {j0, j1}, ks[2] = {k0, k1};
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-      axpy8x(0.125f, ib + (is[a & 1] + (long long)nxc * (js[(a >> 1) & 1] + (long long)nyc * ks[a >> 2])) * ldi,
-             acc);
-  } else {  // adjoint of the prolongation: coarse (io, jo, ko) <- fine children
-    for (int fk = 2 * ko - 1; fk <= 2 * ko + 1; ++fk)
-      for (int fj = 2 * jo - 1; fj <= 2 * jo + 1; ++fj)
-        for (int fi = 2 * io - 1; fi <= 2 * io + 1; ++fi) {
-          if (fi < 0 || fi >= nxf || fj < 0 || fj >= nyf || fk < 0 || fk >= nzf) continue;
-          const float wg = (fi == 2 * io ? 1.f : 0.5f) * (fj == 2 * jo ? 1.f : 0.5f) * (fk == 2 * ko ? 1.f : 0.5f);
-          axpy8x(wg, ib + (fi + (long long)nxf * (fj + (long long)nyf * fk)) * ldi, acc);
-        }
-  }
-  const long long row = (long long)b * No + po;
-  if (mask) {
-    F8x mk;
-    ld8x(mask + row * ldm + m_off + c, mk);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (!(mk.v[k] > 0.f)) acc.v[k] = 0.f;
-  }
-  bf16* o = out + row * ldo + o_off + c;
-  if (accum) {
-    F8x old;
-    ld8x(o, old);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) acc.v[k] += old.v[k];
-  }
-  __align__(16) __nv_bfloat162 r[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) r[k] = __floats2bfloat162_rn(acc.v[2 * k], acc.v[2 * k + 1]);
-  *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(r);
-}
-
+// Per-channel transfer between grid level lf and the next coarser one (hz_resample.cu).
 static void resample3(Ctx& ctx, int mode, int transpose, const int (*gd)[3], int lf, int B, int C, const bf16* in,
                       int ldi, int i_off, bf16* out, int ldo, int o_off, int accum, const bf16* mask = nullptr,
                       int ldm = 0, int m_off = 0) {
-  if (C % 8 || ldi % 8 || i_off % 8 || ldo % 8 || o_off % 8 || (mask && (ldm % 8 || m_off % 8)))
-    throw std::runtime_error("resample3: channel layout not aligned");
-  const int* f = gd[lf];
-  const int* cg = gd[lf + 1];
-  const bool to_coarse = (mode == 0) != (transpose != 0);
-  const long long nf = (long long)f[0] * f[1] * f[2], nc = (long long)cg[0] * cg[1] * cg[2];
-  const long long no = to_coarse ? nc : nf, ni = to_coarse ? nf : nc;
-  const long long total = (long long)B * no * (C / 8);
-  const long long nblk = (total + 255) / 256;
-  if (nblk >= (1LL << 31)) throw std::runtime_error("resample3: batch too large");
-  HZ_LAUNCH(ctx, "net3_resample", (double)B * (no + ni) * C * 2.0, k_resample3, (unsigned)nblk, 256, 0, mode,
-            transpose, f[0], f[1], f[2], cg[0], cg[1], cg[2], B, C, in, ldi, i_off, out, ldo, o_off, accum, mask, ldm,
-            m_off);
+  launch_resample(ctx, "net3_resample", mode, transpose, gd[lf], gd[lf + 1], true, B, C, in, ldi, i_off, out, ldo,
+                  o_off, accum, mask, ldm, m_off);
 }
 
 // ---------------------------------------------------------------------------

@@ -211,11 +211,31 @@ size_t staged_bytes(const WgShape& s) {
 }
 
 template <int CO, int NC>
-void wg_launch(Ctx& ctx, const char* name, const WgShape& s, long long planes_total, const WgradTc& a) {
+void wg_launch(Ctx& ctx, const char* name, WgShape s, long long planes_total, const WgradTc& a) {
   const size_t smem = staged_bytes(s);
   if (cudaFuncSetAttribute(k_wgrad<CO, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     throw std::runtime_error("weight gradient: shared memory attribute");
+  }
+  // Rows per CTA: the CTAs that fit at once, times one to four rounds of them, whichever
+  // takes the fewest rows one after another (a chunk stages two rows more than it sums).
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wgrad<CO, NC>, kThreads, smem) != cudaSuccess) {
+    cudaGetLastError();
+    throw std::runtime_error("weight gradient: occupancy");
+  }
+  const long long slots = (long long)std::max(per_sm, 1) * kSMs;
+  const long long units = planes_total * s.segs * ((s.combos + NC * kWarps - 1) / (NC * kWarps));
+  long long best = 0;
+  for (int rounds = 1; rounds <= 4; ++rounds) {
+    const long long want = std::max<long long>(1, std::min<long long>(s.ny, rounds * slots / units));
+    const int rows = (int)((s.ny + want - 1) / want), chunks = (s.ny + rows - 1) / rows;
+    const long long cost = (units * chunks + slots - 1) / slots * (rows + 2);
+    if (best == 0 || cost < best) {
+      best = cost;
+      s.rows = rows;
+      s.chunks = chunks;
+    }
   }
   const long long ctas = planes_total * s.chunks * s.segs;
   if (ctas >= (1LL << 31)) throw std::runtime_error("weight gradient: batch too large");
@@ -248,17 +268,13 @@ void wgrad_launch(Ctx& ctx, const char* name, const WgradTc& a, int taps) {
   s.seg_blocks = (nblk + s.segs - 1) / s.segs;
   s.segs = (nblk + s.seg_blocks - 1) / s.seg_blocks;
   s.combos = taps * (s.Cin / 16);
-  // pairs per warp: up to 112 accumulator registers
+  // Pairs per warp: as many as leave two CTAs per SM (64 accumulators), though the rows are
+  // staged again for the others.  One CTA with 112 (96 for Cout = 64): 1,010 against 988 us
+  // per 129^2 x 32 step.
   const int co = s.C16 / 16, per = (s.combos + kWarps - 1) / kWarps;
-  const int cap = co == 1 ? 11 : co == 2 ? 7 : 3;
-  const int splits = (per + cap - 1) / cap, nc = (per + splits - 1) / splits;
-  // Rows per CTA: about two CTAs per SM over the whole layer (a chunk re-reads two
-  // rows and adds all its weights atomically, so no more than that)
+  const int cap = co == 1 ? 11 : co == 2 ? 4 : 2;
   const long long planes_total = a.nodes / ((long long)s.nx * s.ny);
-  const long long units = planes_total * s.segs * splits;  // CTAs with whole planes
-  const long long want = std::max<long long>(1, (2LL * kSMs + units - 1) / units);
-  s.rows = (int)std::max<long long>(std::min(4, s.ny), (s.ny + want - 1) / want);
-  s.chunks = (s.ny + s.rows - 1) / s.rows;
+  const int splits = (per + cap - 1) / cap, nc = (per + splits - 1) / splits;
 #define HZ_WG(C, K)                                          \
   if (co == C && nc <= K) {                                  \
     wg_launch<C, K>(ctx, name, s, planes_total, a);          \
@@ -270,8 +286,7 @@ void wgrad_launch(Ctx& ctx, const char* name, const WgradTc& a, int taps) {
   HZ_WG(1, 11)
   HZ_WG(2, 2)
   HZ_WG(2, 4)
-  HZ_WG(2, 7)
-  HZ_WG(4, 3)
+  HZ_WG(4, 2)
 #undef HZ_WG
   throw std::runtime_error("weight gradient: channel counts not supported");
 }

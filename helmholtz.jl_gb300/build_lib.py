@@ -23,7 +23,7 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
               "--expt-relaxed-constexpr", f"-I{INCLUDE}"]
 SOURCES = ["hz_stencil.cu", "hz_krylov.cu", "hz_df64.cu", "hz_kcycle.cu", "hz_learn.cu", "hz_learn3d.cu",
            "hz_conv_tc.cu", "hz_wgrad.cu", "hz_resample.cu",
-           "hz_coarse.cu", "hz_solver.cu", "hz_host.cpp"]
+           "hz_coarse.cu", "hz_fine_fixed.cu", "hz_solver.cu", "hz_host.cpp"]
 
 
 def _nvcc() -> str:

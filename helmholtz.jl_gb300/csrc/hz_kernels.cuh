@@ -8,6 +8,7 @@
 
 #include "../../include/helmgpu.h"
 #include "hz_common.cuh"
+#include "hz_fixed.cuh"
 #include "hz_host.h"
 
 namespace hz {
@@ -68,6 +69,24 @@ struct FineOp {
 template <typename T, typename TX, typename TB>
 void launch_fine(Ctx& ctx, int mode, const FineOp& op, const cplx<T>* diag, const cplx<T>* dinv, const cplx<TX>* x,
                  const cplx<TB>* b, cplx<T>* y, long long ld, const int* cols, int ncols, double w);
+
+// y = op(x) or b - op(x) in FP64 accuracy on the integer pipe (hz_fine_fixed.cu), where
+// fine_fixed_pays() says so.  Rounds otherwise than launch_fine: not for arithmetic whose
+// bits have to be those of another path.
+struct FixedRefs {
+  int exponent;  // the largest of the operator's coefficients, from launch_fine_setup
+  int ok;        // whether the rest lie near enough to it; this and below from launch_diag_fixed
+  Fixed o[3];    // minus the neighbours' coefficients per axis
+};
+struct FixedDiag {
+  const FixedRefs* refs;
+  const int4* d;  // the diagonal's limbs, from launch_diag_fixed
+};
+void launch_diag_fixed(Ctx& ctx, const FineOp& op, const double2* d, FixedRefs* refs, int4* out);
+bool fine_fixed_pays(const FineOp& op, int ncols);
+template <typename TX>
+void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag, const FixedDiag& fd,
+                       const cplx<TX>* x, const double2* b, double2* y, long long ld, const int* cols, int ncols);
 
 // Galerkin level: 3^d stored complex coefficients per node, coef[k*cld + p]
 // is the entry A(p, p + offset_k), offset_k = (k%3-1, k/3%3-1, k/9-1).
@@ -181,10 +200,11 @@ void launch_kc_combine(Ctx& ctx, bool add, long long N, long long ld, const int*
 
 // ---- setup kernels ---------------------------------------------------------
 // Fine-level diagonals on the device from nodal m and gamma (device arrays):
-// diag(H), diag(SH) with the shift i*shift*Re(w)^2*m, and 1/diag(SH).
+// diag(H), diag(SH) with the shift i*shift*Re(w)^2*m, and 1/diag(SH); refs[2]: the largest
+// exponent fields of H's and SH's coefficients.
 void launch_fine_setup(Ctx& ctx, const Grid& g, int dim, const double* h, double wr, double wi, double shift, double BC,
                        int neumann_on_top, int sommerfeld, const double* m, const double* gamma, double2* dH,
-                       double2* dSH, double2* iSH);
+                       double2* dSH, double2* iSH, FixedRefs* refs);
 void launch_probe_init(Ctx& ctx, const Grid& gc, int dim, double2* out, long long ld);
 void launch_probe_scatter(Ctx& ctx, const Grid& gc, int dim, const double2* y, long long ld, double2* coef,
                           long long cld);

@@ -605,7 +605,7 @@ template void launch_bicg_xr<float>(Ctx&, long long, double2*, const float2*, co
 __global__ void k_fine_setup(Grid g, int dim, double h0, double h1, double h2, double wr, double wi, double s,
                              double BC, int neumann_on_top, int sommerfeld, const double* __restrict__ m,
                              const double* __restrict__ gamma, double2* __restrict__ dH, double2* __restrict__ dSH,
-                             double2* __restrict__ iSH) {
+                             double2* __restrict__ iSH, FixedRefs* __restrict__ refs) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= g.N) return;
   const int i = (int)(p % g.nx);
@@ -647,14 +647,28 @@ __global__ void k_fine_setup(Grid g, int dim, double h0, double h1, double h2, d
   dSH[p] = mk<double>(sr, shi);
   const double den = sr * sr + shi * shi;
   iSH[p] = mk<double>(sr / den, -shi / den);
+  // the largest exponents of each operator's coefficients
+  auto ex = [](double v) { return __double2hiint(v) >> 20 & 0x7ff; };
+  int off = max(ex(1.0 / (h0 * h0)), ex(1.0 / (h1 * h1)));
+  if (dim == 3) off = max(off, ex(1.0 / (h2 * h2)));
+  const unsigned lanes = __activemask();
+  const int eH = __reduce_max_sync(lanes, max(off, max(ex(hr), ex(hi))));
+  const int eSH = __reduce_max_sync(lanes, max(off, max(ex(sr), ex(shi))));
+  if ((threadIdx.x & 31) == 0) {
+    if (eH > *(volatile int*)&refs[0].exponent) atomicMax(&refs[0].exponent, eH);
+    if (eSH > *(volatile int*)&refs[1].exponent) atomicMax(&refs[1].exponent, eSH);
+  }
 }
 
 void launch_fine_setup(Ctx& ctx, const Grid& g, int dim, const double* h, double wr, double wi, double shift, double BC,
                        int neumann_on_top, int sommerfeld, const double* m, const double* gamma, double2* dH,
-                       double2* dSH, double2* iSH) {
+                       double2* dSH, double2* iSH, FixedRefs* refs) {
   const long long nb = (g.N + 255) / 256;
+  if (cudaMemsetAsync(refs, 0, 2 * sizeof(FixedRefs), ctx.stream) != cudaSuccess)
+    throw std::runtime_error("fine setup: clear");
   HZ_LAUNCH(ctx, "fine_setup", (double)g.N * (2 * 8 + 3 * 16), k_fine_setup, (unsigned)nb, 256, 0, g, dim, h[0], h[1],
-            dim == 3 ? h[2] : 1.0, wr, wi, shift, BC, neumann_on_top, sommerfeld, m, gamma, dH, dSH, iSH);
+            dim == 3 ? h[2] : 1.0, wr, wi, shift, BC, neumann_on_top, sommerfeld, m, gamma, dH, dSH, iSH,
+            refs);
 }
 
 // ---------------------------------------------------------------------------

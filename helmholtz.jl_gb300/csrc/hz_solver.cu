@@ -145,6 +145,7 @@ struct hz_handle {
   FineOp fop{};
   // fine-level diagonals: H, SH (FP64), 1/diag(SH) (FP64), FP32 copies of SH
   DBuf diagH, diagSH, dinvSH, diagSH32, dinvSH32;
+  DBuf fixrefs, diagHfix, diagSHfix;  // H and SH for the integer pipe (FixedDiag)
   DBuf diagHdf;  // diag(H) in df64 (emulated-FP64 outer arithmetic)
   Hierarchy hier[2];
   // FGMRES workspace
@@ -1065,14 +1066,22 @@ void precondition(hz_handle* h, Hierarchy& H, const double2* vj, void* zj, const
   }
 }
 
-// y = H x (outer operator, FP64 arithmetic) for the active columns.
+FixedDiag fixed_diag(const hz_handle* h, int shifted) {
+  return FixedDiag{h->fixrefs.as<FixedRefs>() + shifted, (shifted ? h->diagSHfix : h->diagHfix).as<int4>()};
+}
+
+// y = H x (outer operator, FP64 accuracy) for the active columns.  native: in the FP64
+// pipe's own steps.
 template <typename TX>
 void apply_H(hz_handle* h, int adj, int mode, const cplx<TX>* x, const double2* b, double2* y, const int* cols,
-             int nc) {
+             int nc, bool native = false) {
   FineOp fop = h->fop;
   fop.adj = adj;
   fop.outer = 1;
-  launch_fine<double, TX, double>(h->ctx, mode, fop, h->diagH.as<double2>(), nullptr, x, b, y, h->g0.N, cols, nc,
+  if (!native && fine_fixed_pays(fop, nc))
+    launch_fine_fixed<TX>(h->ctx, mode, fop, h->diagH.as<double2>(), fixed_diag(h, 0), x, b, y, h->g0.N, cols, nc);
+  else
+    launch_fine<double, TX, double>(h->ctx, mode, fop, h->diagH.as<double2>(), nullptr, x, b, y, h->g0.N, cols, nc,
                                   0.0);
 }
 
@@ -1576,14 +1585,15 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
     launch_reduce(h->ctx, part, dc, nc, 2, nblk, red, HS, 0);
     launch_norms(h->ctx, red, HS, 1, dc, nc, h->beta.as<double>(), nullptr);
   };
-  // y = H z for the preconditioned vector z
+  // y = H z for the preconditioned vector z; native steps, as everything in this method: its
+  // iterates follow the rounding closely
   auto apply = [&](const void* z, double2* y, int nc) {
     if (emu)
       launch_fine_df64<double2>(h->ctx, fopa, h->diagHdf.as<float4>(), (const float2*)z, y, N, dc, nc);
     else if (mixed)
-      apply_H<float>(h, adj, MODE_APPLY, (const float2*)z, nullptr, y, dc, nc);
+      apply_H<float>(h, adj, MODE_APPLY, (const float2*)z, nullptr, y, dc, nc, true);
     else
-      apply_H<double>(h, adj, MODE_APPLY, (const double2*)z, nullptr, y, dc, nc);
+      apply_H<double>(h, adj, MODE_APPLY, (const double2*)z, nullptr, y, dc, nc, true);
   };
   head(na);
   for (; it <= maxit; ++it) {
@@ -1633,7 +1643,7 @@ int bicgstab(hz_handle* h, int adj, int nrhs) {
   for (int c = 0; c < nrhs; ++c)
     if (bn[c] > 0) nz.push_back(c);
   upload_cols(h, nz);
-  apply_H<double>(h, adj, MODE_RESID, X, B, r, dc, (int)nz.size());
+  apply_H<double>(h, adj, MODE_RESID, X, B, r, dc, (int)nz.size(), true);
   col_norms(h, r, nz, h->beta.as<double>(), nullptr, rn.data());
   int worst = 0;
   for (int c : nz) {
@@ -1652,6 +1662,9 @@ void init_fine(hz_handle* h) {
   h->diagH.alloc((size_t)N * 16);
   h->diagSH.alloc((size_t)N * 16);
   h->dinvSH.alloc((size_t)N * 16);
+  h->fixrefs.alloc(2 * sizeof(FixedRefs));
+  h->diagHfix.alloc((size_t)N * 16);
+  h->diagSHfix.alloc((size_t)N * 16);
   {
     DBuf dm, dg;
     dm.alloc((size_t)N * 8);
@@ -1660,7 +1673,10 @@ void init_fine(hz_handle* h) {
     ck(cudaMemcpyAsync(dg.p, p.gamma, N * 8, cudaMemcpyHostToDevice, h->ctx.stream), "upload gamma");
     launch_fine_setup(h->ctx, h->g0, p.dim, p.h, p.omega_re, p.omega_im, h->opt.shift,
                       p.order_neumann_bc == 1 ? 1.0 : 2.0, p.neumann_on_top, p.sommerfeld, dm.as<double>(),
-                      dg.as<double>(), h->diagH.as<double2>(), h->diagSH.as<double2>(), h->dinvSH.as<double2>());
+                      dg.as<double>(), h->diagH.as<double2>(), h->diagSH.as<double2>(), h->dinvSH.as<double2>(),
+                      h->fixrefs.as<FixedRefs>());
+    launch_diag_fixed(h->ctx, h->fop, h->diagH.as<double2>(), h->fixrefs.as<FixedRefs>(), h->diagHfix.as<int4>());
+    launch_diag_fixed(h->ctx, h->fop, h->diagSH.as<double2>(), h->fixrefs.as<FixedRefs>() + 1, h->diagSHfix.as<int4>());
     sync(h);
   }
   if (h->opt.precision == HZ_PREC_MIXED && h->opt.outer_arith == HZ_OUTER_EMULATED) {
@@ -1991,8 +2007,12 @@ int hz_apply(hz_handle* h, int32_t op, int32_t transpose, const double* X, doubl
     FineOp fop = h->fop;
     fop.adj = transpose ? 1 : 0;
     const double2* diag = (op == HZ_OP_H) ? h->diagH.as<double2>() : h->diagSH.as<double2>();
-    launch_fine<double, double, double>(h->ctx, MODE_APPLY, fop, diag, nullptr, xd, (const double2*)nullptr, yd, n,
-                                        h->apply_cols.as<int>(), nrhs, 0.0);
+    if (fine_fixed_pays(fop, nrhs))
+      launch_fine_fixed<double>(h->ctx, MODE_APPLY, fop, diag, fixed_diag(h, op == HZ_OP_H ? 0 : 1), xd, nullptr,
+                                yd, n, h->apply_cols.as<int>(), nrhs);
+    else
+      launch_fine<double, double, double>(h->ctx, MODE_APPLY, fop, diag, nullptr, xd, (const double2*)nullptr, yd, n,
+                                          h->apply_cols.as<int>(), nrhs, 0.0);
     if (mem == HZ_MEM_HOST) copy_out(h, yd, Y, n, nrhs, HZ_MEM_HOST);
     sync(h);
   });

@@ -5,8 +5,9 @@
 // in two signed limbs, v = (hi 2^29 + lo) 2^(E - 1080) up to its 59th bit; a product of two
 // values keeps hi hi, hi lo and lo hi (the dropped lo lo lies 60 bits below the product of
 // the references, with either sign), and sums of such products are exact in 64-bit integers.
-// Used with references local to a few terms (hz_krylov.cu), so an element's rounding is
-// relative to its neighbours in the sum, 2^-58, not to a vector's largest element.
+// Used with references local to a neighbourhood (128 nodes in hz_krylov.cu, a brick in
+// hz_fine_fixed.cu), so an element's rounding is relative to its neighbours, 2^-58, not to a
+// vector's largest element.
 //
 // Values this does not cover are told by their exponents: fixed_ok().
 #pragma once

@@ -246,11 +246,14 @@ struct GsColumn {
   int* host_flag = nullptr;                       // pinned copy of flag
   int* count = nullptr;                           // block counters, zero
   double* part = nullptr;                         // partial sums, gs_part_bytes
+  int* vexp = nullptr;                            // references of the stored basis, gs_exponents (FP64 form)
 };
 int gs_nblk(long long N, int ncols);
 size_t gs_part_bytes(long long N, int R);
+size_t gs_exponents(long long N, int vectors);
 // the dots of step j (K = j + 1 vectors) and the update w -= sum coef_i V_i of one pass
-void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int j, int pass,
+// (FP64 form: pass 0 leaves V_j as fixed-point words)
+void launch_gs_pass(Ctx& ctx, long long N, double2* V, long long vstride, long long ld, int j, int pass,
                     const int* cols, int ncols, const GsColumn& g);
 void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, int pass,
                        const int* cols, int ncols, const GsColumn& g);

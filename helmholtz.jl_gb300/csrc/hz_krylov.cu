@@ -84,84 +84,148 @@ void launch_dots(Ctx& ctx, long long N, const double2* V, long long ld, int K, c
 // Gram-Schmidt in FP64 on the integer pipe (hz_fixed.cuh)
 // ---------------------------------------------------------------------------
 // Native FP64 takes four FMAs per 16-byte basis element, two clocks of an SM; HBM delivers
-// the element in 0.7.  Dots: a thread takes four nodes at a time, relates the basis values
-// and w to the largest of its own four, sums the products in integers and adds the exact
-// total to its FP64 accumulator.  Update: all terms of a node are related to the
-// node's largest term, and their exact sum is subtracted from w with one rounding.
-// Values outside the range of hz_fixed.cuh take the native steps.
-// Measured, native -> fixed, per pass averaged over the steps of restart 10: 129^3 x 8: dots
-// 632 -> 486 us, update 642 -> 430 us; 1025 x 513 x 16: 333 -> 255, 320 -> 226 us (the second
-// pass included, which most columns take).  Errors against quadruple precision, 4,096 to
-// 200,000 nodes, waves, a point source's peak and noise: dots 3e-17 to 1.5e-16 of |V||w|
-// (native 5e-17 to 2.6e-16), update 6e-17 of |w'| rms (native 2.4e-16).
+// the element in 0.7.  So the basis is kept as fixed-point words (58 bits, hz_fixed.cuh) with one
+// reference per 128 nodes, the largest value's exponent: the first dots of step j, which read the
+// newest vector v_j as the preconditioner did, write it back so, in place.  Dots: a warp takes
+// such a group, four nodes per lane, relates w to the largest of a lane's four, sums the
+// products in integers and adds the exact total to its FP64 accumulator.  Update: the
+// coefficients are related to the group's largest term instead of the basis values; the exact sum
+// is subtracted from w with one rounding.  Groups outside the range of hz_fixed.cuh stay FP64
+// (kGsRaw) and take the native steps, as do values of w.
+// Measured per pass averaged over the steps of restart 10 (the second pass included, which most
+// columns take), native / converting every value in every pass / words: 129^3 x 8: dots 632 / 461 /
+// 301 us, update 642 / 427 / 359 us; 1025 x 513 x 16: 333 / 235 / 157, 320 / 215 / 181 us: 5.0 to
+// 5.4 TB/s.  What bounds them is latency: 16 warps per SM at 113 to 128 registers, dots with one
+// vector on its way (352 us without), update with all of a node's.  Errors against quadruple
+// precision, 4,096 to 200,000 nodes, waves, a point source's peak and noise: dots 5e-17 to
+// 1.1e-16 of |V||w| (native 5e-17 to 2.5e-16), update 5e-17 to 7e-17 of |w'| rms (2.4e-16).
 static constexpr int kGsNodes = 4;
-// One vector in six stays on the FP64 pipe, which the integer dots leave idle (5 vectors, 129^3 x
-// 8: 465 -> 441 us; 10: 952 -> 932 us; one in four was no better).
-__host__ __device__ constexpr int gs_native(int vectors) { return (vectors + 1) / 6; }
+static constexpr int kGsGroup = 32 * kGsNodes;
+enum { kGsZero = -1, kGsRaw = -2 };  // exponents of a group without a reference
+
+size_t gs_exponents(long long N, int vectors) { return (size_t)vectors * ((N + kGsGroup - 1) / kGsGroup) * sizeof(int); }
+
+// FP64 value of stored words (kept raw: their bits)
+__device__ __forceinline__ double gs_value(int hi, int lo, int e) {
+  if (e == kGsRaw) return __hiloint2double(lo, hi);
+  if (e < 0) return 0.0;
+  const double v = fma((double)hi, 536870912.0, (double)lo);  // 2^29
+  return v * __hiloint2double((e - 1080 + 1023) << 20, 0);
+}
+__device__ __forceinline__ double2 gs_value(int4 r, int e) { return mk<double>(gs_value(r.x, r.y, e), gs_value(r.z, r.w, e)); }
 
 template <int KT>
-__global__ void __launch_bounds__(RT, 2) k_gs_dots(long long N, const double2* __restrict__ V, long long vstride,
+__global__ void __launch_bounds__(RT, 2) k_gs_dots(long long N, double2* __restrict__ V, long long vstride,
                                                    long long ld, int i0, const double2* __restrict__ w,
-                                                   const int* __restrict__ cols, int pass, int want_norm, GsColumn g) {
+                                                   const int* __restrict__ cols, int pass, int want_norm, int fresh,
+                                                   GsColumn g) {
   __shared__ double tot[2 * KT + 1];
   const int c = cols[blockIdx.y];
   if (pass && !g.flag[c]) return;
   const int nblk = gridDim.x;
+  const int lane = threadIdx.x & 31;
   const double2* wc = w + (long long)c * ld;
-  const double2* vb = V + ((long long)i0 * vstride + c) * ld;
+  int4* vb = reinterpret_cast<int4*>(V + ((long long)i0 * vstride + c) * ld);
   const long long vs = vstride * ld;  // distance between consecutive basis vectors
-  double2 acc[KT];
+  const long long groups = (N + kGsGroup - 1) / kGsGroup, es = vstride * groups;
+  int* eb = g.vexp + ((long long)i0 * vstride + c) * groups;
+  // lanes below 16 carry the sums' real parts, the others the imaginary ones: a pair of lanes
+  // exchanges its exact totals, so that each converts one of them (the conversion takes two and
+  // a half slots of the FP64 pipe)
+  const bool upper = lane & 16;
+  double acc[KT];
 #pragma unroll
-  for (int s = 0; s < KT; ++s) acc[s] = mk<double>(0, 0);
+  for (int s = 0; s < KT; ++s) acc[s] = 0.0;
   double nrm = 0.0;
-  const long long stride = (long long)nblk * RT;
-  auto load = [&](const double2* x, long long p, uint4 (&r)[kGsNodes]) {
-    int e = 0;
+  // one vector's nodes and the next group's references (lane s: vector s's) are on their way while
+  // the vector before is worked on
+  const long long first = (long long)blockIdx.x * (RT / 32) + (threadIdx.x >> 5), round = (long long)nblk * (RT / 32);
+  int4 next[kGsNodes];
+  auto fetch = [&](int s, long long gi) {
+    const long long p = gi * kGsGroup + lane;
 #pragma unroll
-    for (int q = 0; q < kGsNodes; ++q) {
-      r[q] = p + q * stride < N ? *reinterpret_cast<const uint4*>(x + p + q * stride) : make_uint4(0, 0, 0, 0);
-      e = max(e, max(fixed_exponent(r[q].y), fixed_exponent(r[q].w)));
-    }
-    return e;
+    for (int q = 0; q < kGsNodes; ++q)
+      next[q] = gi < groups && p + q * 32 < N ? vb[s * vs + p + q * 32] : make_int4(0, 0, 0, 0);
   };
-  auto value = [](const uint4& r) {
-    return mk<double>(__hiloint2double((int)r.y, (int)r.x), __hiloint2double((int)r.w, (int)r.z));
-  };
-  for (long long p = (long long)blockIdx.x * RT + threadIdx.x; p < N; p += kGsNodes * stride) {
-    uint4 wr[kGsNodes];
-    const int ew = load(wc, p, wr);
+  const int* el = eb + (lane < KT ? lane : 0) * es;
+  int ahead = first < groups ? el[first] : kGsZero;
+  fetch(0, first);
+  for (long long gi = first; gi < groups; gi += round) {
+    const long long p = gi * kGsGroup + lane;
+    const int e = ahead;
+    if (gi + round < groups) ahead = el[gi + round];
+    double2 wv[kGsNodes];
     Fixed wx[kGsNodes], wy[kGsNodes];
+    int ew = 0;
 #pragma unroll
     for (int q = 0; q < kGsNodes; ++q) {
-      wx[q] = fixed_from<6>(wr[q].y, wr[q].x, ew);
-      wy[q] = fixed_from<6>(wr[q].w, wr[q].z, ew);
-      if (want_norm) {
-        const double2 v = value(wr[q]);
-        nrm = fma(v.x, v.x, fma(v.y, v.y, nrm));
-      }
+      wv[q] = p + q * 32 < N ? wc[p + q * 32] : mk<double>(0, 0);
+      ew = max(ew, max(fixed_exponent((uint32_t)__double2hiint(wv[q].x)), fixed_exponent((uint32_t)__double2hiint(wv[q].y))));
     }
+    ew = __reduce_max_sync(0xffffffffu, ew);
     const bool wok = fixed_ref_ok(ew);
 #pragma unroll
+    for (int q = 0; q < kGsNodes; ++q) {
+      wx[q] = fixed_from<6>((uint32_t)__double2hiint(wv[q].x), (uint32_t)__double2loint(wv[q].x), ew);
+      wy[q] = fixed_from<6>((uint32_t)__double2hiint(wv[q].y), (uint32_t)__double2loint(wv[q].y), ew);
+      if (want_norm) nrm = fma(wv[q].x, wv[q].x, fma(wv[q].y, wv[q].y, nrm));
+    }
+#pragma unroll
     for (int s = 0; s < KT; ++s) {
-      uint4 vr[kGsNodes];
-      const int ev = load(vb + s * vs, p, vr);
-      if (s >= gs_native(KT) && wok && fixed_ref_ok(ev) && fixed_ok(ev + ew)) {
+      int4 v[kGsNodes];
+#pragma unroll
+      for (int q = 0; q < kGsNodes; ++q) v[q] = next[q];
+      if (s + 1 < KT)
+        fetch(s + 1, gi);
+      else
+        fetch(0, gi + round);
+      int ev;
+      if (s == KT - 1 && fresh) {  // FP64 still: to words, in place
+        uint32_t top = 0, any = 0;
+#pragma unroll
+        for (int q = 0; q < kGsNodes; ++q) {
+          top = max(top, max((uint32_t)v[q].y & 0x7fffffffu, (uint32_t)v[q].w & 0x7fffffffu));
+          any |= (uint32_t)v[q].x | (uint32_t)v[q].z;
+        }
+        top = __reduce_max_sync(0xffffffffu, top);
+        any = __reduce_or_sync(0xffffffffu, any);
+        ev = (int)(top >> 20);
+        if (fixed_ref_ok(ev)) {
+#pragma unroll
+          for (int q = 0; q < kGsNodes; ++q) {
+            const Fixed a = fixed_from<6>((uint32_t)v[q].y, (uint32_t)v[q].x, ev);
+            const Fixed b = fixed_from<6>((uint32_t)v[q].w, (uint32_t)v[q].z, ev);
+            v[q] = make_int4(a.hi, a.lo, b.hi, b.lo);
+            if (p + q * 32 < N) vb[s * vs + p + q * 32] = v[q];
+          }
+        } else {
+          ev = (top | any) ? kGsRaw : kGsZero;
+        }
+        if (lane == 0) eb[s * es + gi] = ev;
+      } else {
+        ev = __shfl_sync(0xffffffffu, e, s);
+      }
+      if (ev >= 0 && wok && fixed_ok(ev + ew)) {
         FixedSum f{0, 0, 0, 0};
 #pragma unroll
         for (int q = 0; q < kGsNodes; ++q)
-          fixed_conj_mac(f, fixed_from<6>(vr[q].y, vr[q].x, ev), fixed_from<6>(vr[q].w, vr[q].z, ev), wx[q], wy[q]);
-        const double sc = __hiloint2double((int)fixed_scale_hi(ev + ew, 0), 0);
-        acc[s].x = fma((double)fixed_total(f.rh, f.rl), sc, acc[s].x);
-        acc[s].y = fma((double)fixed_total(f.ih, f.il), sc, acc[s].y);
-      } else {
+          fixed_conj_mac(f, Fixed{v[q].x, v[q].y}, Fixed{v[q].z, v[q].w}, wx[q], wy[q]);
+        const long long re = fixed_total(f.rh, f.rl), im = fixed_total(f.ih, f.il);
+        const long long t = (upper ? im : re) + __shfl_xor_sync(0xffffffffu, upper ? re : im, 16);
+        acc[s] = fma((double)t, __hiloint2double((int)fixed_scale_hi(ev + ew, 0), 0), acc[s]);
+      } else if (ev != kGsZero) {
+        double2 t = mk<double>(0, 0);
 #pragma unroll
-        for (int q = 0; q < kGsNodes; ++q)
-          if (p + q * stride < N) acc[s] = cfma_conj<double>(value(vr[q]), wc[p + q * stride], acc[s]);
+        for (int q = 0; q < kGsNodes; ++q) t = cfma_conj<double>(gs_value(v[q], ev), wv[q], t);
+        acc[s] += (upper ? t.y : t.x) + __shfl_xor_sync(0xffffffffu, upper ? t.x : t.y, 16);
       }
     }
   }
+  double2 sums[KT];
+#pragma unroll
+  for (int s = 0; s < KT; ++s) sums[s] = upper ? mk<double>(0, acc[s]) : mk<double>(acc[s], 0);
   double* part = g.part + (long long)blockIdx.y * (2 * KT + 1) * nblk;
-  block_partials<KT>(acc, KT, nrm, want_norm, part, nblk);
+  block_partials<KT>(sums, KT, nrm, want_norm, part, nblk);
   if (!last_of_column(g.count, c, nblk)) return;
   fold_partials(part, nblk, 2 * KT + want_norm, tot);
   gs_after_dots(g, c, i0, KT, want_norm, pass, tot);
@@ -172,66 +236,62 @@ __global__ void __launch_bounds__(RT, 2) k_gs_update(long long N, const double2*
                                                      long long ld, int i0, double2* __restrict__ w,
                                                      const int* __restrict__ cols, int j, int pass, int last,
                                                      GsColumn g) {
-  __shared__ int4 hl[KT];
-  __shared__ int he[KT];
+  __shared__ int4 hl[RT / 32][KT];
   __shared__ double tot[1];
   const int c = cols[blockIdx.y];
   if (pass && !g.flag[c]) return;
   const int nblk = gridDim.x;
   const double2* h = g.coef + (long long)c * g.hstride + i0;
   constexpr int kNone = -(1 << 20);  // exponent of a zero coefficient
-  int bad = 0;
-  if (threadIdx.x < KT) {
-    const uint4 r = *reinterpret_cast<const uint4*>(h + threadIdx.x);
-    const int e = max(fixed_exponent(r.y), fixed_exponent(r.w));
-    const bool zero = ((r.x | r.z) == 0) && (((r.y | r.w) & 0x7fffffffu) == 0);
-    bad = !zero && !fixed_ref_ok(e);
-    const Fixed a = fixed_from<6>(r.y, r.x, e), b = fixed_from<6>(r.w, r.z, e);
-    hl[threadIdx.x] = zero ? make_int4(0, 0, 0, 0) : make_int4(a.hi, a.lo, b.hi, b.lo);
-    he[threadIdx.x] = zero ? kNone : e;
-  }
-  bad = __syncthreads_or(bad);
-  int hmax = kNone;
-#pragma unroll
-  for (int s = 0; s < KT; ++s) hmax = max(hmax, he[s]);
-  const double2* vb = V + ((long long)i0 * vstride + c) * ld;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // lane s holds the coefficient of vector s
+  const uint4 hr = lane < KT ? *reinterpret_cast<const uint4*>(h + lane) : make_uint4(0, 0, 0, 0);
+  const bool hzero = ((hr.x | hr.z) == 0) && (((hr.y | hr.w) & 0x7fffffffu) == 0);
+  const int he = max(fixed_exponent(hr.y), fixed_exponent(hr.w));
+  const bool bad = __any_sync(0xffffffffu, !hzero && !fixed_ref_ok(he));
+  const int4* vb = reinterpret_cast<const int4*>(V + ((long long)i0 * vstride + c) * ld);
   const long long vs = vstride * ld;
+  const long long groups = (N + kGsGroup - 1) / kGsGroup;
+  const int* el = g.vexp + ((long long)(i0 + (lane < KT ? lane : 0)) * vstride + c) * groups;  // lane s: vector s's
   double2* wc = w + (long long)c * ld;
   double nrm = 0.0;
-  const long long stride = (long long)nblk * RT;
-  for (long long p = (long long)blockIdx.x * RT + threadIdx.x; p < N; p += stride) {
-    uint4 vr[KT];
+  // a warp's 32 nodes, a quarter of a group; their references one round ahead
+  const long long first = (long long)blockIdx.x * (RT / 32) + warp, round = (long long)nblk * (RT / 32);
+  const long long units = (N + 31) / 32;
+  int ahead = first < units ? el[first / kGsNodes] : kGsZero;
+  for (long long u = first; u < units; u += round) {
+    const long long p = u * 32 + lane;
+    int4 v[KT];
 #pragma unroll
-    for (int s = 0; s < KT; ++s) vr[s] = *reinterpret_cast<const uint4*>(vb + s * vs + p);
-    double2 wv = wc[p];
-    int vmax = 0, T = kNone;
-#pragma unroll
-    for (int s = 0; s < KT; ++s) {
-      const int e = max(fixed_exponent(vr[s].y), fixed_exponent(vr[s].w));
-      vmax = max(vmax, e);
-      T = max(T, e + he[s]);
-    }
-    if (!bad && vmax < 0x7ff && T - hmax >= kFixedMin && fixed_ok(T)) {
+    for (int s = 0; s < KT; ++s) v[s] = p < N ? vb[s * vs + p] : make_int4(0, 0, 0, 0);
+    double2 wv = p < N ? wc[p] : mk<double>(0, 0);
+    const int e = lane < KT ? ahead : kGsZero;
+    if (u + round < units) ahead = el[(u + round) / kGsNodes];
+    // the coefficients' words, related to the largest term of the group
+    const bool term = e >= 0 && !hzero;
+    const int T = __reduce_max_sync(0xffffffffu, term ? e + he : kNone);
+    const bool ok = !bad && (T == kNone || fixed_ok(T)) &&
+                    __all_sync(0xffffffffu, e != kGsRaw && (!term || T - e >= kFixedMin));
+    if (ok) {
+      const Fixed a = fixed_from<7>(hr.y, hr.x, term ? T - e : 2047), b = fixed_from<7>(hr.w, hr.z, term ? T - e : 2047);
+      __syncwarp();
+      if (lane < KT) hl[warp][lane] = term ? make_int4(a.hi, a.lo, b.hi, b.lo) : make_int4(0, 0, 0, 0);
+      __syncwarp();
       FixedSum f{0, 0, 0, 0};
 #pragma unroll
       for (int s = 0; s < KT; ++s) {
-        const int4 a = hl[s];
-        const int e = T - he[s];
-        fixed_cmac(f, Fixed{a.x, a.y}, Fixed{a.z, a.w}, fixed_from<7>(vr[s].y, vr[s].x, e),
-                   fixed_from<7>(vr[s].w, vr[s].z, e));
+        const int4 k = hl[warp][s];
+        fixed_cmac(f, Fixed{v[s].x, v[s].y}, Fixed{v[s].z, v[s].w}, Fixed{k.x, k.y}, Fixed{k.z, k.w});
       }
-      const double sc = __hiloint2double((int)fixed_scale_hi(T, 1), 0);
+      const double sc = T == kNone ? 0.0 : __hiloint2double((int)fixed_scale_hi(T, 1), 0);
       wv.x = fma((double)-fixed_total(f.rh, f.rl), sc, wv.x);
       wv.y = fma((double)-fixed_total(f.ih, f.il), sc, wv.y);
     } else {
 #pragma unroll
       for (int s = 0; s < KT; ++s)
-        wv = cfms<double>(h[s],
-                          mk<double>(__hiloint2double((int)vr[s].y, (int)vr[s].x),
-                                     __hiloint2double((int)vr[s].w, (int)vr[s].z)),
-                          wv);
+        wv = cfms<double>(h[s], gs_value(v[s], __shfl_sync(0xffffffffu, e, s)), wv);
     }
-    wc[p] = wv;
+    if (p < N) wc[p] = wv;
     if (last) nrm = fma(wv.x, wv.x, fma(wv.y, wv.y, nrm));
   }
   if (!last) return;
@@ -268,10 +328,10 @@ int gs_nblk(long long N, int ncols) {
 
 size_t gs_part_bytes(long long N, int R) { return (size_t)R * krylov_nblk(N, 1) * 33 * sizeof(double); }
 
-void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, long long ld, int j, int pass,
+void launch_gs_pass(Ctx& ctx, long long N, double2* V, long long vstride, long long ld, int j, int pass,
                     const int* cols, int ncols, const GsColumn& g) {
   if (ncols <= 0) return;
-  double2* w = const_cast<double2*>(V) + (long long)(j + 1) * vstride * ld;
+  double2* w = V + (long long)(j + 1) * vstride * ld;
   const int K = j + 1;
   const dim3 grid(gs_nblk(N, ncols), ncols);
   // a masked pass is charged by the host once it knows which columns took it
@@ -279,12 +339,13 @@ void launch_gs_pass(Ctx& ctx, long long N, const double2* V, long long vstride, 
   for (int i0 = 0; i0 < K; i0 += 16) {
     const int k = std::min(16, K - i0);
     const int wn = (pass == 0 && i0 + 16 >= K) ? 1 : 0;  // ||w||^2 before the update (slot K)
+    const int fresh = wn;                                // v_j's first use here
     ctx.add_flops("krylov_dots", el * (8.0 * k + (wn ? 4.0 : 0.0)));
     switch (k) {
 #define HZ_GS_CASE(q)                                                                                             \
   case q:                                                                                                         \
     HZ_LAUNCH(ctx, "krylov_dots", el * (k + 1) * 16.0, k_gs_dots<q>, grid, RT, 0, N, V, vstride, ld, i0, w, cols, \
-              pass, wn, g);                                                                                       \
+              pass, wn, fresh, g);                                                                                \
     break;
       HZ_K_CASES(HZ_GS_CASE)
 #undef HZ_GS_CASE

@@ -153,6 +153,7 @@ struct hz_handle {
   int mcap = 0;
   DBuf Bd, Xd, V, Z, part, hA, hB, nr, flag, Hh, cs, sn, gv, yv, bnorm, bnorm_inv, beta, beta_inv, cols, kcol;
   DBuf gscnt;       // block counters of the Gram-Schmidt kernels
+  DBuf vexp;        // references of the basis' fixed-point words
   std::vector<int> cols_on_device;  // what cols holds
   DBuf bsc;         // BiCGSTAB per-column scalars
   DBuf sig, hC;     // FGMRES basis scales (stored v_i stands for sig_i v_i) and update coefficients
@@ -657,6 +658,7 @@ void ensure_workspace(hz_handle* h, int nrhs) {
   h->hC.alloc((size_t)R * (m + 2) * 16);
   h->part.alloc(gs_part_bytes(N, R));
   h->gscnt.alloc((size_t)R * sizeof(int));
+  h->vexp.alloc(gs_exponents(N, (m + 1) * R));
   ck(cudaMemsetAsync(h->gscnt.p, 0, (size_t)R * sizeof(int), h->ctx.stream), "zero block counters");
   const int HS = m + 2;
   h->hA.alloc((size_t)R * HS * 16);
@@ -1410,6 +1412,7 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
   gs.host_est = h->h_est;
   gs.host_flag = h->h_flag;
   gs.count = h->gscnt.as<int>();
+  gs.vexp = h->vexp.as<int>();
   gs.part = h->part.as<double>();
   std::vector<int> kcol(h->rcap, 0);
   int outer = 0;

@@ -216,7 +216,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_kc_update(long long N, long long ld, const int* __restrict__ cols,
                                                    const cplx<T>* __restrict__ B, cplx<T>* __restrict__ W,
                                                    double* part, int* count, double2* __restrict__ ks,
-                                                   cplx<T>* __restrict__ kt) {
+                                                   cplx<T>* __restrict__ kt, Sweep<T> sw) {
   const int c = cols[blockIdx.y];
   const long long off = (long long)c * ld;
   const cplx<T> h = kt[c * 8];
@@ -225,6 +225,10 @@ __global__ void __launch_bounds__(256) k_kc_update(long long N, long long ld, co
   for (long long p = (long long)blockIdx.x * 256 + threadIdx.x; p < N; p += (long long)gridDim.x * 256) {
     const cplx<T> w = cfms<T>(h, B[off + p], W[off + p]);
     W[off + p] = w;
+    if (sw.y) {
+      const cplx<T> d = sw.dinv[p];
+      sw.y[off + p] = cmul<T>(mk<T>(d.x * sw.w, d.y * sw.w), w);
+    }
     add_norm<T>(v, 0, w);
   }
   double t[kNV];
@@ -319,9 +323,9 @@ void launch_kc_dots(Ctx& ctx, int mode, long long N, long long ld, const int* co
 
 template <typename T>
 void launch_kc_update(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const cplx<T>* B, cplx<T>* W,
-                      const KcSums& s) {
-  HZ_LAUNCH(ctx, "kcycle_update", (double)N * nc * 3 * sizeof(cplx<T>), k_kc_update<T>, dim3(kc_nblk(N), nc), 256, 0, N,
-            ld, cols, B, W, s.part, s.count, s.ks, (cplx<T>*)s.kt);
+                      const KcSums& s, const Sweep<T>& sweep) {
+  HZ_LAUNCH(ctx, "kcycle_update", (double)N * nc * (sweep.y ? 4 : 3) * sizeof(cplx<T>), k_kc_update<T>,
+            dim3(kc_nblk(N), nc), 256, 0, N, ld, cols, B, W, s.part, s.count, s.ks, (cplx<T>*)s.kt, sweep);
 }
 
 template <typename T>
@@ -370,7 +374,7 @@ void launch_kc_combine(Ctx& ctx, bool add, long long N, long long ld, const int*
 #define HZ_KC_INST(T)                                                                                                  \
   HZ_KC_INST_TB(T, T)                                                                                                  \
   template void launch_kc_update<T>(Ctx&, long long, long long, const int*, int, const cplx<T>*, cplx<T>*,             \
-                                    const KcSums&);                                                                    \
+                                    const KcSums&, const Sweep<T>&);                                                   \
   template void launch_kc_last<T>(Ctx&, long long, long long, const int*, int, const cplx<T>*, const cplx<T>*,         \
                                   const cplx<T>*, const KcSums&);                                                      \
   template void launch_kc_combine<T>(Ctx&, bool, long long, long long, const int*, int, const cplx<T>*,                \

@@ -88,11 +88,21 @@ template <typename TX>
 void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag, const FixedDiag& fd,
                        const cplx<TX>* x, const double2* b, double2* y, long long ld, const int* cols, int ncols);
 
+// The first Jacobi sweep y = w dinv .* r of a Galerkin level, written by the kernel that makes
+// its right-hand side r (y null: none): the same numbers as launch_jacobi0, which on small
+// levels is a launch of 1 us for each visit (129^2, one source, V-cycle: 18.2 -> 17.9 ms a
+// solve; 257 x 129 x 4, W-cycle: 114 -> 113; 3D: 0.1% to 0.6%).
+template <typename T> struct Sweep {
+  const cplx<T>* dinv = nullptr;
+  cplx<T>* y = nullptr;
+  T w = T(0);
+};
 // Galerkin level: 3^d stored complex coefficients per node, coef[k*cld + p]
 // is the entry A(p, p + offset_k), offset_k = (k%3-1, k/3%3-1, k/9-1).
 template <typename T, typename TB>
 void launch_rap(Ctx& ctx, int mode, const Grid& g, const cplx<T>* coef, long long cld, const cplx<T>* dinv,
-                const cplx<T>* x, const cplx<TB>* b, cplx<T>* y, long long ld, const int* cols, int ncols, double w);
+                const cplx<T>* x, const cplx<TB>* b, cplx<T>* y, long long ld, const int* cols, int ncols, double w,
+                const Sweep<T>& sweep = Sweep<T>());
 
 // y = w * dinv .* b  (first Jacobi sweep from a zero guess); adj conjugates dinv.
 template <typename T, typename TB>
@@ -102,11 +112,12 @@ void launch_jacobi0(Ctx& ctx, const Grid& g, const cplx<T>* dinv, int adj, const
 // Full-weighting restriction rc = P^T rf / 2^d (fine grid gf, coarse grid gc).
 template <typename T>
 void launch_restrict(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<T>* rf, long long ldf, cplx<T>* rc,
-                     long long ldc, const int* cols, int ncols);
+                     long long ldc, const int* cols, int ncols, const Sweep<T>& sweep = Sweep<T>());
 // The same of b - y W, y = yt[c*8 + 6].
 template <typename T, typename TB>
 void launch_restrict_diff(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<TB>* b, const cplx<T>* W,
-                          const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols);
+                          const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols,
+                          const Sweep<T>& sweep);
 
 // A coarse-grid correction: z0, or Y0 z0 + Y1 z1 with the K-cycle's coefficients kt (slots 6, 7).
 template <typename T> struct Correction {
@@ -182,7 +193,7 @@ void launch_kc_dots(Ctx& ctx, int mode, long long N, long long ld, const int* co
 // W -= (<b, W> / ||b||^2) b and its norm
 template <typename T>
 void launch_kc_update(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const cplx<T>* B, cplx<T>* W,
-                      const KcSums& s);
+                      const KcSums& s, const Sweep<T>& sweep = Sweep<T>());
 // the norm of W2 orthogonalised against b and W1, and the 3x2 least squares -> Y0, Y1
 template <typename T>
 void launch_kc_last(Ctx& ctx, long long N, long long ld, const int* cols, int nc, const cplx<T>* B, const cplx<T>* W1,

@@ -750,13 +750,13 @@ template <> const float2* lev_dinv<float>(Level& L) { return L.dinv32.as<float2>
 // One level operation in precision T with right-hand side of precision TB.
 template <typename T, typename TB>
 void lev_op(hz_handle* h, Hierarchy& H, int l, int mode, const cplx<T>* x, const cplx<TB>* b, cplx<T>* y,
-            const int* cols, int nc) {
+            const int* cols, int nc, const Sweep<T>& sweep = Sweep<T>()) {
   Level& L = *H.lv[l];
   const double w = h->opt.relax_param;
   if (L.fine) {
     launch_fine<T, T, TB>(h->ctx, mode, L.fop, fine_diag<T>(L), fine_dinv<T>(L), x, b, y, L.ld, cols, nc, w);
   } else {
-    launch_rap<T, TB>(h->ctx, mode, L.g, lev_coef<T>(L), L.g.N, lev_dinv<T>(L), x, b, y, L.ld, cols, nc, w);
+    launch_rap<T, TB>(h->ctx, mode, L.g, lev_coef<T>(L), L.g.N, lev_dinv<T>(L), x, b, y, L.ld, cols, nc, w, sweep);
   }
 }
 
@@ -765,6 +765,25 @@ void lev_jacobi0(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* 
   Level& L = *H.lv[l];
   const cplx<T>* dinv = L.fine ? fine_dinv<T>(L) : lev_dinv<T>(L);
   launch_jacobi0<T, TB>(h->ctx, L.g, dinv, L.fine ? L.fop.adj : 0, b, y, L.ld, cols, nc, h->opt.relax_param);
+}
+
+// The first sweep that the cycle on a coarse level l takes on its right-hand side, for the
+// kernel that makes this one: none on the coarsest level, without pre-smoothing, under the
+// network and where two GMRES smoothing steps start from zero.
+template <typename T> Sweep<T> first_sweep(hz_handle* h, Hierarchy& H, int l, cplx<T>* out) {
+  Level& L = *H.lv[l];
+  const int pre = std::max(0, h->opt.relax_pre), post = std::max(0, h->opt.relax_post);
+  Sweep<T> s;
+  if (l + 1 == (int)H.lv.size() || pre == 0 || L.fine || (h->net_active && l == h->net_level)) return s;
+  if (h->opt.relax_type == HZ_RELAX_JAC_GMRES && l >= h->opt.relax_from) {
+    if (pre != 1) return s;
+    s.y = L.gv.as<cplx<T>>() + (long long)h->rcap * L.ld;  // smooth_direction's Z
+  } else {
+    s.y = (pre + post) % 2 == 1 ? out : L.t.as<cplx<T>>();  // mg_cycle's first buffer
+  }
+  s.dinv = lev_dinv<T>(L);
+  s.w = (T)h->opt.relax_param;
+  return s;
 }
 
 // Network input features on level l: the medium restricted l times by nodal
@@ -837,7 +856,7 @@ template <typename T> struct KStep {
 
 template <typename T, typename TB>
 void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out, const int* cols, int nc,
-              KStep<T>* step = nullptr);
+              KStep<T>* step = nullptr, bool swept = false);
 
 // The preconditioner of a K-cycle step on level k (the level's own cycle, or
 // the network when it is attached to level k: it then stands for everything
@@ -845,13 +864,13 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
 // recursion to the coarsest LU), the operator product and its sums.
 template <typename T>
 void kcycle_precondition(hz_handle* h, Hierarchy& H, int k, const cplx<T>* v, cplx<T>* z, KStep<T>& step,
-                         const int* cols, int nc) {
+                         const int* cols, int nc, bool swept) {
   Level& L = *H.lv[k];
   const cplx<T>* none = nullptr;
   if (h->net_active && k == h->net_level)
     learned_correction<T>(h, H, k, v, z, cols, nc);
   else
-    mg_cycle<T, T>(h, H, k, v, z, cols, nc, &step);
+    mg_cycle<T, T>(h, H, k, v, z, cols, nc, &step, swept);
   if (step.done) return;
   lev_op<T, T>(h, H, k, MODE_APPLY, z, none, step.W, cols, nc);
   launch_kc_dots<T, T>(h->ctx, step.mode, L.g.N, L.ld, cols, nc, step.b, step.W1, step.W, step.sums);
@@ -861,7 +880,7 @@ void kcycle_precondition(hz_handle* h, Hierarchy& H, int k, const cplx<T>* v, cp
 // level k's operator, right-preconditioned by level k's own cycle (zero
 // initial guess; Multigrid.jl cycleType 'K').  The correction is Y0 Z0 + Y1 Z1.
 template <typename T>
-Correction<T> kcycle_steps(hz_handle* h, Hierarchy& H, int k, const cplx<T>* b, const int* cols, int nc) {
+Correction<T> kcycle_steps(hz_handle* h, Hierarchy& H, int k, const cplx<T>* b, const int* cols, int nc, bool swept) {
   Level& L = *H.lv[k];
   const long long N = L.g.N, ld = L.ld, vs = (long long)h->rcap * ld;
   cplx<T>* W1 = L.kv.as<cplx<T>>();
@@ -870,9 +889,10 @@ Correction<T> kcycle_steps(hz_handle* h, Hierarchy& H, int k, const cplx<T>* b, 
   cplx<T>* Z1 = W1 + 3 * vs;
   const KcSums s = sums_of(L.ks, L.kp, L.kn);
   KStep<T> first{KC_FIRST, b, nullptr, W1, s}, second{KC_SECOND, b, W1, W2, s};
-  kcycle_precondition<T>(h, H, k, b, Z0, first, cols, nc);
-  launch_kc_update<T>(h->ctx, N, ld, cols, nc, b, W1, s);
-  kcycle_precondition<T>(h, H, k, W1, Z1, second, cols, nc);
+  kcycle_precondition<T>(h, H, k, b, Z0, first, cols, nc, swept);
+  const Sweep<T> sweep = first_sweep<T>(h, H, k, Z1);
+  launch_kc_update<T>(h->ctx, N, ld, cols, nc, b, W1, s, sweep);
+  kcycle_precondition<T>(h, H, k, W1, Z1, second, cols, nc, sweep.y != nullptr);
   launch_kc_last<T>(h->ctx, N, ld, cols, nc, b, W1, W2, s);
   return Correction<T>{Z0, Z1, (const cplx<T>*)s.kt};
 }
@@ -891,13 +911,13 @@ void capture_rhs(hz_handle* h, Level& L, const cplx<TB>* b, const int* cols, int
 // One GMRES step's direction on level l for the residual r (relaxType "Jac-GMRES":
 // GMRES on the level's operator right-preconditioned by one damped-Jacobi sweep):
 // Z = w D^-1 r, W = A Z and y = <W, r> / ||W||^2 (0 for a zero residual) in slot 6 of the
-// smoother's coefficients.
+// smoother's coefficients.  swept: Z is there already.
 template <typename T, typename TR>
 void smooth_direction(hz_handle* h, Hierarchy& H, int l, const cplx<TR>* r, cplx<T>* Z, cplx<T>* W, const int* cols,
-                      int nc) {
+                      int nc, bool swept) {
   Level& L = *H.lv[l];
   const cplx<T>* none = nullptr;
-  lev_jacobi0<T, TR>(h, H, l, r, Z, cols, nc);
+  if (!swept) lev_jacobi0<T, TR>(h, H, l, r, Z, cols, nc);
   lev_op<T, T>(h, H, l, MODE_APPLY, Z, none, W, cols, nc);
   launch_kc_dots<T, TR>(h->ctx, KC_SMOOTH, L.g.N, L.ld, cols, nc, r, none, W, sums_of(L.gs, L.gp, L.gn));
 }
@@ -928,7 +948,7 @@ void smooth_two_steps(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx
 // The coarse-grid correction of level l for the right-hand sides in C.b of level l + 1:
 // the network, a K-cycle step or a recursive cycle.
 template <typename T>
-Correction<T> coarse_correction(hz_handle* h, Hierarchy& H, int l, const int* cols, int nc) {
+Correction<T> coarse_correction(hz_handle* h, Hierarchy& H, int l, const int* cols, int nc, bool swept) {
   Level& C = *H.lv[l + 1];
   const int last = (int)H.lv.size() - 1;
   const cplx<T>* b = C.b.as<cplx<T>>();
@@ -938,16 +958,16 @@ Correction<T> coarse_correction(hz_handle* h, Hierarchy& H, int l, const int* co
   if (h->net_active && l + 1 == h->net_level && !(h->opt.cycle == 'K' && l + 1 < last))
     learned_correction<T>(h, H, l + 1, b, x, cols, nc);
   else if (h->opt.cycle == 'K' && l + 1 < last)
-    return kcycle_steps<T>(h, H, l + 1, b, cols, nc);
+    return kcycle_steps<T>(h, H, l + 1, b, cols, nc, swept);
   else
-    mg_cycle<T, T>(h, H, l + 1, b, x, cols, nc);
+    mg_cycle<T, T>(h, H, l + 1, b, x, cols, nc, nullptr, swept);
   return Correction<T>{x};
 }
 
-// x_out = cycle(b) on level l with zero initial guess.
+// x_out = cycle(b) on level l with zero initial guess.  swept: first_sweep()'s is done.
 template <typename T, typename TB>
 void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out, const int* cols, int nc,
-              KStep<T>* step) {
+              KStep<T>* step, bool swept) {
   Level& L = *H.lv[l];
   const int last = (int)H.lv.size() - 1;
   if (h->cap_on && l == h->cap_level) capture_rhs<TB>(h, L, b, cols, nc);
@@ -978,6 +998,9 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
     oth = (cur == out) ? tb : out;
   }
   const int ncalls = (h->opt.cycle == 'W' && l + 1 < last) ? 2 : 1;
+  // the coarse level's first sweep (into the first K-cycle step's Z0 or the correction)
+  const Sweep<T> sweep = first_sweep<T>(
+      h, H, l + 1, h->opt.cycle == 'K' && l + 1 < last ? C.kv.as<cplx<T>>() + 2LL * h->rcap * C.ld : C.x.as<cplx<T>>());
   if (h->opt.relax_type == HZ_RELAX_JAC_GMRES && l >= h->opt.relax_from) {
     // relaxType "Jac-GMRES": smoothing steps update `out` in place
     const long long vs = (long long)h->rcap * L.ld;
@@ -992,7 +1015,7 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
         launch_cast_cols<T, TB>(h->ctx, L.g.N, b, L.ld, rb, L.ld, cols, nc);
         base = nullptr;
       } else if (call == 0 && pre == 1) {
-        smooth_direction<T, TB>(h, H, l, b, Z, W, cols, nc);  // x = y Z, b - A x = b - y W
+        smooth_direction<T, TB>(h, H, l, b, Z, W, cols, nc, swept);  // x = y Z, b - A x = b - y W
         base = Z;
         yt = (const cplx<T>*)s.kt;
       } else {
@@ -1003,16 +1026,17 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
         lev_op<T, TB>(h, H, l, MODE_RESID, out, b, rb, cols, nc);
       }
       if (yt)
-        launch_restrict_diff<T, TB>(h->ctx, L.g, C.g, b, W, yt, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
+        launch_restrict_diff<T, TB>(h->ctx, L.g, C.g, b, W, yt, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc, sweep);
       else
-        launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
-      const Correction<T> e = coarse_correction<T>(h, H, l, cols, nc);
+        launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc, sweep);
+      const Correction<T> e = coarse_correction<T>(h, H, l, cols, nc, sweep.y != nullptr);
       launch_prolong<T>(h->ctx, L.g, C.g, e, C.ld, base, yt, out, L.ld, cols, nc);
     }
     if (post == 1) {
       const bool k = step != nullptr;
-      lev_op<T, TB>(h, H, l, MODE_RESID, out, b, R, cols, nc);
-      smooth_direction<T, T>(h, H, l, R, Z, W, cols, nc);
+      const Sweep<T> own = L.fine ? Sweep<T>() : Sweep<T>{lev_dinv<T>(L), Z, (T)h->opt.relax_param};
+      lev_op<T, TB>(h, H, l, MODE_RESID, out, b, R, cols, nc, own);
+      smooth_direction<T, T>(h, H, l, R, Z, W, cols, nc, own.y != nullptr);
       launch_kc_finish<T, TB>(h->ctx, k ? step->mode : KC_SMOOTH, L.g.N, L.ld, cols, nc,
                               (const cplx<T>*)s.kt, out, Z, b, R, W,
                               k ? step->b : nullptr, k ? step->W : nullptr, k ? step->sums : KcSums());
@@ -1024,7 +1048,7 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
   }
   bool zero_guess = true;
   if (pre > 0) {
-    lev_jacobi0<T, TB>(h, H, l, b, cur, cols, nc);
+    if (!swept) lev_jacobi0<T, TB>(h, H, l, b, cur, cols, nc);
     for (int s = 1; s < pre; ++s) {
       lev_op<T, TB>(h, H, l, MODE_JACOBI, cur, b, oth, cols, nc);
       std::swap(cur, oth);
@@ -1035,16 +1059,16 @@ void mg_cycle(hz_handle* h, Hierarchy& H, int l, const cplx<TB>* b, cplx<T>* out
     if (zero_guess) {
       // residual = b: restrict b directly
       if (std::is_same<T, TB>::value) {
-        launch_restrict<T>(h->ctx, L.g, C.g, (const cplx<T>*)b, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
+        launch_restrict<T>(h->ctx, L.g, C.g, (const cplx<T>*)b, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc, sweep);
       } else {
         launch_cast_cols<T, TB>(h->ctx, L.g.N, b, L.ld, rb, L.ld, cols, nc);
-        launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
+        launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc, sweep);
       }
     } else {
       lev_op<T, TB>(h, H, l, MODE_RESID, cur, b, rb, cols, nc);
-      launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc);
+      launch_restrict<T>(h->ctx, L.g, C.g, rb, L.ld, C.b.as<cplx<T>>(), C.ld, cols, nc, sweep);
     }
-    const Correction<T> e = coarse_correction<T>(h, H, l, cols, nc);
+    const Correction<T> e = coarse_correction<T>(h, H, l, cols, nc, sweep.y != nullptr);
     launch_prolong<T>(h->ctx, L.g, C.g, e, C.ld, zero_guess ? nullptr : cur, nullptr, cur, L.ld, cols, nc);
     zero_guess = false;
   }
@@ -2542,7 +2566,7 @@ void collect_targets_iterative(hz_handle* h, Hierarchy& H, int level, int sweeps
     ck(cudaMemcpyAsync(xd, x1.p, (size_t)k * N * 16, cudaMemcpyDeviceToDevice, h->ctx.stream), "first sweep");
     for (int s = 1; s < sweeps; ++s) {
       lev_op<double, double>(h, H, level, MODE_RESID, xd, r, res.as<double2>(), dc, k);
-      const Correction<double> e = kcycle_steps<double>(h, H, level, res.as<double2>(), dc, k);
+      const Correction<double> e = kcycle_steps<double>(h, H, level, res.as<double2>(), dc, k, false);
       launch_kc_combine<double>(h->ctx, false, N, Lv.ld, dc, k, e.kt, e.z0, e.z1, ev.as<double2>());
       launch_axpy_compact(h->ctx, N, k, ev.as<double2>(), xd);
     }

@@ -230,11 +230,18 @@ void launch_fine(Ctx& ctx, int mode, const FineOp& op, const cplx<T>* diag, cons
 // ---------------------------------------------------------------------------
 // Galerkin (stored-coefficient) stencil
 // ---------------------------------------------------------------------------
+// w dinv of a node, as k_jacobi0 takes it
+template <typename T>
+__device__ __forceinline__ cplx<T> scaled_dinv(const Sweep<T>& sw, long long p) {
+  const cplx<T> d = sw.dinv[p];
+  return mk<T>(d.x * sw.w, d.y * sw.w);
+}
+
 template <typename T, typename TB, int MODE, bool IS3D>
 __global__ void __launch_bounds__(128) k_rap(Grid g, const cplx<T>* __restrict__ coef, long long cld,
                                              const cplx<T>* __restrict__ dinv, const cplx<T>* __restrict__ x,
                                              const cplx<TB>* __restrict__ b, cplx<T>* __restrict__ y, long long ld,
-                                             const int* __restrict__ cols, int ncols, int cpb, T w) {
+                                             const int* __restrict__ cols, int ncols, int cpb, T w, Sweep<T> sw) {
   constexpr int NS = IS3D ? 27 : 9;
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= g.N) return;
@@ -258,6 +265,7 @@ __global__ void __launch_bounds__(128) k_rap(Grid g, const cplx<T>* __restrict__
   }
   cplx<T> di = mk<T>(0, 0);
   if (MODE == MODE_JACOBI) di = dinv[p];
+  if (MODE == MODE_RESID && sw.y) di = scaled_dinv<T>(sw, p);
   const int c0 = blockIdx.y * cpb;
   const int c1 = min(ncols, c0 + cpb);
   // columns are independent: unrolled so that several columns' loads are in flight
@@ -282,6 +290,7 @@ __global__ void __launch_bounds__(128) k_rap(Grid g, const cplx<T>* __restrict__
       const cplx<T> r = mk<T>((T)bb.x - ax.x, (T)bb.y - ax.y);
       if (MODE == MODE_RESID) {
         __stcs(&y[off + p], r);
+        if (sw.y) __stcs(&sw.y[off + p], cmul<T>(di, r));
       } else {
         const cplx<T> dr = cmul<T>(di, r);
         __stcs(&y[off + p], mk<T>(xp.x + w * dr.x, xp.y + w * dr.y));
@@ -332,7 +341,8 @@ void launch_rap_tile(Ctx& ctx, int mode, const Grid& g, const float2* coef, long
 
 template <typename T, typename TB>
 void launch_rap(Ctx& ctx, int mode, const Grid& g, const cplx<T>* coef, long long cld, const cplx<T>* dinv,
-                const cplx<T>* x, const cplx<TB>* b, cplx<T>* y, long long ld, const int* cols, int ncols, double w) {
+                const cplx<T>* x, const cplx<TB>* b, cplx<T>* y, long long ld, const int* cols, int ncols, double w,
+                const Sweep<T>& sweep) {
   if (ncols <= 0) return;
   const int TPB = 128;
   long long nbx = (g.N + TPB - 1) / TPB;
@@ -344,14 +354,17 @@ void launch_rap(Ctx& ctx, int mode, const Grid& g, const cplx<T>* coef, long lon
   double rbytes = (double)g.N * ncols * 2 * sizeof(cplx<T>) + (double)g.N * ns * sizeof(cplx<T>);
   if (mode != MODE_APPLY) rbytes += (double)g.N * ncols * sizeof(cplx<TB>);
   if (mode == MODE_JACOBI) rbytes += (double)g.N * sizeof(cplx<T>);
+  if (sweep.y) rbytes += (double)g.N * (ncols + 1) * sizeof(cplx<T>);
   if constexpr (std::is_same<T, float>::value) {
     if (is3d && ctx.rap_tiled) {
       launch_rap_tile<TB>(ctx, mode, g, coef, cld, dinv, x, b, y, ld, cols, ncols, w, rbytes);
+      if (sweep.y) launch_jacobi0<T, T>(ctx, g, sweep.dinv, 0, y, sweep.y, ld, cols, ncols, (double)sweep.w);
       return;
     }
   }
-#define HZ_RAP_CASE(M, D, NAME) \
-  HZ_LAUNCH(ctx, NAME, rbytes, (k_rap<T, TB, M, D>), grid, TPB, 0, g, coef, cld, dinv, x, b, y, ld, cols, ncols, cpb, (T)w)
+#define HZ_RAP_CASE(M, D, NAME)                                                                                         \
+  HZ_LAUNCH(ctx, NAME, rbytes, (k_rap<T, TB, M, D>), grid, TPB, 0, g, coef, cld, dinv, x, b, y, ld, cols, ncols, cpb, (T)w, \
+            sweep)
   if (mode == MODE_APPLY) {
     if (is3d) HZ_RAP_CASE(MODE_APPLY, true, "rap_apply");
     else HZ_RAP_CASE(MODE_APPLY, false, "rap_apply");
@@ -410,7 +423,7 @@ template <typename T, typename TB, bool IS3D, bool DIFF>
 __global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<TB>* __restrict__ rf,
                                                   const cplx<T>* __restrict__ W, const cplx<T>* __restrict__ yt,
                                                   long long ldf, cplx<T>* __restrict__ rc, long long ldc,
-                                                  const int* __restrict__ cols, int ncols, int cpb) {
+                                                  const int* __restrict__ cols, int ncols, int cpb, Sweep<T> sw) {
   const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= gc.N) return;
   const int I = (int)(q % gc.nx);
@@ -436,6 +449,7 @@ __global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<T
     oz[2] = (fk < gf.nz - 1) ? sz : 0;
   }
   const T scale = IS3D ? T(0.125) : T(0.25);
+  const cplx<T> di = sw.y ? scaled_dinv<T>(sw, q) : mk<T>(0, 0);
   const int c0 = blockIdx.y * cpb;
   const int c1 = min(ncols, c0 + cpb);
   // columns are independent: unrolled so that several columns' loads are in flight
@@ -461,13 +475,16 @@ __global__ void __launch_bounds__(256) k_restrict(Grid gf, Grid gc, const cplx<T
         }
       }
     }
-    rc[(long long)col * ldc + q] = mk<T>(scale * ar, scale * ai);
+    const cplx<T> v = mk<T>(scale * ar, scale * ai);
+    rc[(long long)col * ldc + q] = v;
+    if (sw.y) sw.y[(long long)col * ldc + q] = cmul<T>(di, v);
   }
 }
 
 template <typename T, typename TB, bool DIFF>
 static void restrict_any(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<TB>* rf, const cplx<T>* W,
-                         const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols) {
+                         const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols,
+                         const Sweep<T>& sweep) {
   if (ncols <= 0) return;
   const int TPB = 256;
   long long nbx = (gc.N + TPB - 1) / TPB;
@@ -475,25 +492,27 @@ static void restrict_any(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<TB
   int cpb = (ncols + ch - 1) / ch;
   dim3 grid((unsigned)nbx, (unsigned)ch);
   const double tbytes =
-      (double)ncols * (gf.N * (sizeof(cplx<TB>) + (DIFF ? sizeof(cplx<T>) : 0)) + gc.N * sizeof(cplx<T>));
+      (double)ncols * (gf.N * (sizeof(cplx<TB>) + (DIFF ? sizeof(cplx<T>) : 0)) +
+                       gc.N * (sweep.y ? 2 : 1) * sizeof(cplx<T>));
   if (gf.nz > 1)
     HZ_LAUNCH(ctx, "restrict", tbytes, (k_restrict<T, TB, true, DIFF>), grid, TPB, 0, gf, gc, rf, W, yt, ldf, rc, ldc,
-              cols, ncols, cpb);
+              cols, ncols, cpb, sweep);
   else
     HZ_LAUNCH(ctx, "restrict", tbytes, (k_restrict<T, TB, false, DIFF>), grid, TPB, 0, gf, gc, rf, W, yt, ldf, rc, ldc,
-              cols, ncols, cpb);
+              cols, ncols, cpb, sweep);
 }
 
 template <typename T>
 void launch_restrict(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<T>* rf, long long ldf, cplx<T>* rc,
-                     long long ldc, const int* cols, int ncols) {
-  restrict_any<T, T, false>(ctx, gf, gc, rf, (const cplx<T>*)nullptr, nullptr, ldf, rc, ldc, cols, ncols);
+                     long long ldc, const int* cols, int ncols, const Sweep<T>& sweep) {
+  restrict_any<T, T, false>(ctx, gf, gc, rf, (const cplx<T>*)nullptr, nullptr, ldf, rc, ldc, cols, ncols, sweep);
 }
 
 template <typename T, typename TB>
 void launch_restrict_diff(Ctx& ctx, const Grid& gf, const Grid& gc, const cplx<TB>* b, const cplx<T>* W,
-                          const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols) {
-  restrict_any<T, TB, true>(ctx, gf, gc, b, W, yt, ldf, rc, ldc, cols, ncols);
+                          const cplx<T>* yt, long long ldf, cplx<T>* rc, long long ldc, const int* cols, int ncols,
+                          const Sweep<T>& sweep) {
+  restrict_any<T, TB, true>(ctx, gf, gc, b, W, yt, ldf, rc, ldc, cols, ncols, sweep);
 }
 
 // COMB: the coarse vector is Y0 e0 + Y1 e1 (a K-cycle correction, formed here instead of
@@ -1092,7 +1111,8 @@ int launch_fine_apply_noalloc(cudaStream_t stream, int dev, const FineOp& op, co
   template void launch_fine<T, T, TB>(Ctx&, int, const FineOp&, const cplx<T>*, const cplx<T>*, const cplx<T>*,     \
                                       const cplx<TB>*, cplx<T>*, long long, const int*, int, double);               \
   template void launch_rap<T, TB>(Ctx&, int, const Grid&, const cplx<T>*, long long, const cplx<T>*,                \
-                                  const cplx<T>*, const cplx<TB>*, cplx<T>*, long long, const int*, int, double);   \
+                                  const cplx<T>*, const cplx<TB>*, cplx<T>*, long long, const int*, int, double,    \
+                                  const Sweep<T>&);                                                                 \
   template void launch_jacobi0<T, TB>(Ctx&, const Grid&, const cplx<T>*, int, const cplx<TB>*, cplx<T>*, long long, \
                                       const int*, int, double);
 HZ_INST_T_TB(double, double)
@@ -1104,12 +1124,13 @@ template void launch_fine<double, float, double>(Ctx&, int, const FineOp&, const
                                                  double);
 #undef HZ_INST_T_TB
 template void launch_restrict<double>(Ctx&, const Grid&, const Grid&, const double2*, long long, double2*, long long,
-                                      const int*, int);
+                                      const int*, int, const Sweep<double>&);
 template void launch_restrict<float>(Ctx&, const Grid&, const Grid&, const float2*, long long, float2*, long long,
-                                     const int*, int);
+                                     const int*, int, const Sweep<float>&);
 #define HZ_INST_RD(T, TB)                                                                                       \
   template void launch_restrict_diff<T, TB>(Ctx&, const Grid&, const Grid&, const cplx<TB>*, const cplx<T>*,     \
-                                            const cplx<T>*, long long, cplx<T>*, long long, const int*, int);
+                                            const cplx<T>*, long long, cplx<T>*, long long, const int*, int,     \
+                                            const Sweep<T>&);
 HZ_INST_RD(double, double)
 HZ_INST_RD(float, float)
 HZ_INST_RD(float, double)

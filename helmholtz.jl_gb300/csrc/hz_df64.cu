@@ -307,16 +307,92 @@ __global__ void __launch_bounds__(RT, 2) k_update_df(long long N, const float4* 
   gs_after_update(g, c, j, pass, tot[0]);
 }
 
+// The first pass's update and the second pass's dots of the new w in one read of the basis:
+// HBM is the bound of the separate kernels (6.1 to 6.4 TB/s), so the read saved counts: 193 x
+// 161 x 97 x 16, per step averaged over restart 10: 1626 us for both -> 1070; 641 x 321 x 33:
+// 267 -> 170.  Near the FP32 pipe's bound at 10 vectors (960 operations per node).  Columns whose
+// second pass is not due waste their dots, which cost no traffic; most columns take it.
+template <int KT>
+__global__ void __launch_bounds__(RT, 2) k_update_dots_df(long long N, const float4* __restrict__ V, long long vstride,
+                                                          long long ld, float4* __restrict__ w,
+                                                          const int* __restrict__ cols, GsColumn g) {
+  __shared__ double tot[2 * KT + 1];
+  __shared__ float4 h[KT];  // Re hi, Re lo, Im hi, Im lo
+  const int c = cols[blockIdx.y];
+  const int nblk = gridDim.x;
+  if (threadIdx.x < KT) {
+    const double2 hv = g.coef[(long long)c * g.hstride + threadIdx.x];
+    float4 q;
+    split(hv.x, q.x, q.y);
+    split(hv.y, q.z, q.w);
+    h[threadIdx.x] = q;
+  }
+  __syncthreads();
+  const float4* vb = V + (long long)c * ld;
+  const long long vs = vstride * ld;
+  float4* wc = w + (long long)c * ld;
+  DAcc ar[KT], ai[KT], nn;
+#pragma unroll
+  for (int s = 0; s < KT; ++s) {
+    ar[s].init(0.f, 0.f);
+    ai[s].init(0.f, 0.f);
+  }
+  nn.init(0.f, 0.f);
+  const long long stride = (long long)nblk * RT;
+  for (long long p = (long long)blockIdx.x * RT + threadIdx.x; p < N; p += stride) {
+    float4 v[KT];
+#pragma unroll
+    for (int s = 0; s < KT; ++s) v[s] = vb[s * vs + p];
+    const float4 wv = wc[p];
+    DAcc re, im;
+    re.init(wv.x, wv.z);
+    im.init(wv.y, wv.w);
+#pragma unroll
+    for (int s = 0; s < KT; ++s) {
+      const float4 q = h[s];
+      re.msub(q.x, q.y, v[s].x, v[s].z);
+      re.mac(q.z, q.w, v[s].y, v[s].w);
+      im.msub(q.x, q.y, v[s].y, v[s].w);
+      im.msub(q.z, q.w, v[s].x, v[s].z);
+    }
+    re.renorm();
+    im.renorm();
+    __stcs(&wc[p], make_float4(re.hi, im.hi, re.lo, im.lo));
+    nn.mac(re.hi, re.lo, re.hi, re.lo);
+    nn.mac(im.hi, im.lo, im.hi, im.lo);
+#pragma unroll
+    for (int s = 0; s < KT; ++s) {
+      ar[s].mac(v[s].x, v[s].z, re.hi, re.lo);
+      ar[s].mac(v[s].y, v[s].w, im.hi, im.lo);
+      ai[s].mac(v[s].x, v[s].z, im.hi, im.lo);
+      ai[s].msub(v[s].y, v[s].w, re.hi, re.lo);
+    }
+  }
+  double2 acc[KT];
+#pragma unroll
+  for (int s = 0; s < KT; ++s) acc[s] = mk<double>(ar[s].to_double(), ai[s].to_double());
+  double* part = g.part + (long long)blockIdx.y * (2 * KT + 1) * nblk;
+  block_partials<KT>(acc, KT, nn.to_double(), 1, part, nblk);
+  if (!last_of_column(g.count, c, nblk)) return;
+  fold_partials(part, nblk, 2 * KT + 1, tot);
+  gs_after_update(g, c, KT - 1, 0, tot[2 * KT]);
+  gs_after_dots(g, c, 0, KT, 0, 1, tot);  // read by the second pass where it is due
+}
+
 #define HZ_K_CASES(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 
-void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, int pass,
-                       const int* cols, int ncols, const GsColumn& g) {
-  if (ncols <= 0) return;
+// The basis in registers beside the sums: up to this many vectors (the restart length's default)
+static constexpr int kFuse = 10;
+bool gs_fused_df(int vectors) { return vectors <= kFuse; }
+
+// dots: whether the dots are due; update: 1 alone, 2 with the next pass's dots
+static void gs_launches_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, int pass,
+                           int dots, int update, const int* cols, int ncols, const GsColumn& g) {
   float4* w = const_cast<float4*>(V) + (long long)(j + 1) * vstride * ld;
   const int K = j + 1;
   const dim3 grid(gs_nblk(N, ncols), ncols);
   const double el = pass ? 0.0 : (double)N * ncols;
-  for (int i0 = 0; i0 < K; i0 += 16) {
+  for (int i0 = 0; dots && i0 < K; i0 += 16) {
     const int k = std::min(16, K - i0);
     const int wn = (pass == 0 && i0 + 16 >= K) ? 1 : 0;
     switch (k) {
@@ -328,6 +404,19 @@ void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride
       HZ_K_CASES(HZ_GS_CASE)
 #undef HZ_GS_CASE
     }
+  }
+  if (update == 2) {
+    switch (K) {
+#define HZ_GS_CASE(q)                                                                                              \
+  case q:                                                                                                          \
+    HZ_LAUNCH(ctx, "krylov_update", el * (K + 2) * 16.0, k_update_dots_df<q>, grid, RT, 0, N, V, vstride, ld, w, cols, \
+              g);                                                                                                  \
+    break;
+      HZ_GS_CASE(1) HZ_GS_CASE(2) HZ_GS_CASE(3) HZ_GS_CASE(4) HZ_GS_CASE(5)
+      HZ_GS_CASE(6) HZ_GS_CASE(7) HZ_GS_CASE(8) HZ_GS_CASE(9) HZ_GS_CASE(10)
+#undef HZ_GS_CASE
+    }
+    return;
   }
   for (int i0 = 0; i0 < K; i0 += 16) {
     const int k = std::min(16, K - i0);
@@ -342,6 +431,14 @@ void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride
 #undef HZ_GS_CASE
     }
   }
+}
+
+void launch_gs_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, const int* cols,
+                  int ncols, const GsColumn& g) {
+  if (ncols <= 0) return;
+  const bool fused = gs_fused_df(j + 1);
+  gs_launches_df(ctx, N, V, vstride, ld, j, 0, 1, fused ? 2 : 1, cols, ncols, g);
+  gs_launches_df(ctx, N, V, vstride, ld, j, 1, fused ? 0 : 1, 1, cols, ncols, g);
 }
 
 // ---- coarsest solve with emulated-FP64 window operators ---------------------

@@ -266,8 +266,10 @@ size_t gs_exponents(long long N, int vectors);
 // (FP64 form: pass 0 leaves V_j as fixed-point words)
 void launch_gs_pass(Ctx& ctx, long long N, double2* V, long long vstride, long long ld, int j, int pass,
                     const int* cols, int ncols, const GsColumn& g);
-void launch_gs_pass_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, int pass,
-                       const int* cols, int ncols, const GsColumn& g);
+// both passes of the double-float form; fused: the second pass's dots read no basis of their own
+void launch_gs_df(Ctx& ctx, long long N, const float4* V, long long vstride, long long ld, int j, const int* cols,
+                  int ncols, const GsColumn& g);
+bool gs_fused_df(int vectors);
 // out[c*ostride + slot] = sum over blocks of part (slot < K1); accum adds to out.
 void launch_reduce(Ctx& ctx, const double2* part, const int* cols, int ncols, int K1, int nblk, double2* out,
                    int ostride, int accum);

@@ -1467,17 +1467,16 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
           else
             apply_H<double>(h, adj, MODE_APPLY, (const double2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
         }
-        for (int pass = 0; pass < 2; ++pass)
-          if (df)
-            launch_gs_pass_df(h->ctx, N, Vd, vstride, N, j, pass, dc, nl, gs);
-          else
-            launch_gs_pass(h->ctx, N, V, vstride, N, j, pass, dc, nl, gs);
+        if (df)
+          launch_gs_df(h->ctx, N, Vd, vstride, N, j, dc, nl, gs);
+        else
+          for (int pass = 0; pass < 2; ++pass) launch_gs_pass(h->ctx, N, V, vstride, N, j, pass, dc, nl, gs);
       });
       sync(h);
       {
         int n2 = 0;  // columns that took the second Gram-Schmidt pass
         for (int c : live) n2 += h->h_flag[c] ? 1 : 0;
-        h->ctx.add_bytes("krylov_dots", (double)N * n2 * (K + 1) * 16.0);
+        if (!df || !gs_fused_df(K)) h->ctx.add_bytes("krylov_dots", (double)N * n2 * (K + 1) * 16.0);
         h->ctx.add_bytes("krylov_update", (double)N * n2 * (K + 2) * 16.0);
         if (!df) {  // the second pass's FP64 arithmetic (no ||w||^2 in its dots)
           h->ctx.add_flops("krylov_dots", (double)N * n2 * 8.0 * K);

@@ -35,3 +35,23 @@ def test_solves_around_a_group(hz, cells, levels, restart):
         iters.append(np.asarray(S.last_iters))
         assert np.linalg.norm(X / scale - Xref) <= 1e-6 * np.linalg.norm(Xref)
     assert np.abs(iters[0] - iters[1]).max() <= 1
+
+
+@pytest.mark.parametrize("restart", [1, 10, 11, 20])
+def test_emulated_passes(hz, restart):
+    """The double-float form: the first update with the second pass's dots up to 10 vectors,
+    separate launches above.  Iterations as in the FP64 form to within one; the residual bound
+    1e-6 times the condition number (below 1e2 on this grid) bounds the error."""
+    P = layered((24, 16), seed=6, pad=2)
+    B = rhs(P["m"].size, 3, seed=4)
+    Xref = O.direct_solve(P["H"], B)
+    iters = []
+    for outer in ("fp64", "emulated"):
+        MG = hz.getMGparam(complex, int, 2, 1, 400, 1e-6, "Jac", 0.8, 1, 1, "V", "Julia", 0.5, 0.0, precision="mixed",
+                           outerArithmetic=outer)
+        S = hz.getShiftedLaplacianMultigridSolver(hz_param(hz, P), MG, 0.5, "GMRES", restart)
+        X, S = hz.solveLinearSystem(None, B, S)
+        assert (S.last_relres <= 1e-6).all()
+        iters.append(np.asarray(S.last_iters))
+        assert np.linalg.norm(X - Xref) <= 1e-4 * np.linalg.norm(Xref)
+    assert np.abs(iters[0] - iters[1]).max() <= 1

@@ -385,7 +385,7 @@ class MGparam:
     precision: str = "fp64"  # "fp64" or "mixed" (complex-FP32 cycle)
     coarseOperator: str = "Galerkin"  # or "Rediscretize" (src/ShiftedLaplacianMultigridSolver.jl:51-62)
     outerArithmetic: str = "fp64"     # or "emulated": FP64 emulated with FP32 pairs (mixed form, FGMRES)
-    cudaGraph: bool = True            # replay the FGMRES preconditioner applications from CUDA graphs
+    cudaGraph: bool = True            # replay the Krylov iterations from CUDA graphs
     autotune: bool = True             # time the stencils' launch shapes at the first solve
     relaxFrom: int = 0                # "Jac-GMRES": first level smoothed by GMRES steps (finer: "Jac")
     doTranspose: int = 0

@@ -107,7 +107,7 @@ typedef struct hz_options {
   int32_t profile;       /* 1: time every kernel launch with CUDA events */
   int32_t device;        /* CUDA device ordinal */
   int32_t outer_arith;   /* FGMRES outer arithmetic: HZ_OUTER_FP64 (native) or HZ_OUTER_EMULATED */
-  int32_t cuda_graph;    /* 1 (default): replay each FGMRES preconditioner application from a CUDA graph */
+  int32_t cuda_graph;    /* 1 (default): replay each Krylov iteration from a CUDA graph */
   int32_t autotune;      /* 1 (default): time the stencils' launch shapes at the first solve (see hz_tune_info) */
   int32_t relax_type;    /* HZ_RELAX_* (default HZ_RELAX_JAC) */
   int32_t relax_from;    /* HZ_RELAX_JAC_GMRES: first level smoothed by GMRES steps (0: every level) */
@@ -222,7 +222,7 @@ int hz_tune_info(const hz_handle* h, int32_t* fine_ctas, int32_t* rap_ctas);
  * method (krylov_dots, krylov_update, update_x, outer_apply, outer_resid: the
  * complex arithmetic they do in FP64); 0 for the other, memory-bound kernels. */
 int hz_kernel_flops(hz_handle* h, int32_t idx, double* alg_flops);
-/* Replay the preconditioner applications from CUDA graphs (1) or launch them
+/* Replay the Krylov iterations from CUDA graphs (1) or launch them
  * eagerly (0) from the next application on (options.cuda_graph at create time);
  * graphs already captured are kept for when replay is switched back on.  Eager
  * launches let per-launch profiling time each kernel of the cycle. */

@@ -21,7 +21,8 @@
 // 3.8 u of the row's sum of magnitudes, u = 2^-53 (native 1.7 u): a node 2^-5 below its brick.
 //
 // Measured: 157 x 131 x 101 nodes, 13 columns, adjoint: 887 us native, 452; 129^3 nodes, 8 columns of
-// FP32 537 and 355; 1025 x 513 nodes, 16 columns of FP32 176 and 114.  What bounds it is
+// FP32 537 and 355; 1025 x 513 nodes, 16 columns of FP32 176 and 114; the FP64 cycle's residual
+// and Jacobi sweep, 65 x 65 x 33 nodes, 8 columns, 48 and 34, 59 and 49.  What bounds it is
 // instructions (36 per cell converted, 1.75 cells per node in 3D; 106 per sum; 4 additions of the
 // FP64 pipe) at half the issue rate: the rest is the wait for a brick's loads, with four
 // bricks in flight per SM.  Bringing a block's next column by asynchronous copies, 2 or 3
@@ -29,6 +30,7 @@
 // two; giving every third or fourth brick to the native steps took a quarter longer.
 #include <algorithm>
 #include <stdexcept>
+#include <type_traits>
 
 #include "hz_fixed.cuh"
 #include "hz_kernels.cuh"
@@ -156,7 +158,8 @@ template <typename TX, int MODE, bool IS3D, int ROWS>
 __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
     k_fine_fixed(const __grid_constant__ FixOp op, const FixedRefs* __restrict__ refs,
                  const int4* __restrict__ dfix, const double2* __restrict__ diag, const cplx<TX>* __restrict__ x,
-                 const double2* __restrict__ b, double2* __restrict__ y, long long ld, const int* __restrict__ cols) {
+                 const double2* __restrict__ b, double2* __restrict__ y, long long ld, const int* __restrict__ cols,
+                 const double2* __restrict__ dinv, double weight) {
   using R = Raw<TX>;
   using RT = typename R::type;
   constexpr int ZH = IS3D ? 1 : 0, NL = kN + 2 * ZH;
@@ -251,6 +254,16 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
   const double2* bc = b + off;
   double2* yc = y + off;
   const Fixed ox = refs->o[0], oy = refs->o[1], oz = refs->o[2];
+  // a = (op x) of node p to the mode's result
+  auto result = [&](double2 a, int p, double2 bb) {
+    if (MODE == MODE_APPLY) return a;
+    const double2 r = mk<double>(bb.x - a.x, bb.y - a.y);
+    if (MODE == MODE_RESID) return r;
+    double2 di = dinv[p];
+    if (op.adj) di.y = -di.y;
+    const double2 dr = cmul<double>(di, r), xp = ccast<double, TX>(x[off + p]);
+    return mk<double>(xp.x + weight * dr.x, xp.y + weight * dr.y);
+  };
   uint32_t native = 0;  // nodes left to the native steps
 #pragma unroll
   for (int k = 0; k < kN; ++k) {
@@ -258,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
     const int p = p0 + k * gs;
     const int4 d = __ldg(dfix + p);
     double2 bb = mk<double>(0, 0);
-    if (MODE == MODE_RESID) bb = __ldcs(bc + p);
+    if (MODE != MODE_APPLY) bb = __ldcs(bc + p);
     const int4* ck = c + k * step;
     const int4 n0 = ck[0], nl = ck[-1], nr = ck[1], nu = ck[-pitch], nd = ck[pitch];
     const int4 zero = make_int4(0, 0, 0, 0);
@@ -289,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
       }
       const Assemble out(e0 - pown[k + ZH]);
       const double2 a = mk<double>(out(re.total()), out(im.total()));
-      __stcs(yc + p, MODE == MODE_APPLY ? a : mk<double>(bb.x - a.x, bb.y - a.y));
+      __stcs(yc + p, result(a, p, bb));
     } else {
       native |= 1u << k;
     }
@@ -300,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
     const int p = p0 + k * gs;
     const double2 a = IS3D ? native_node<TX, IS3D>(op, diag[p], x + off, i, j, z0 + k)
                            : native_node<TX, IS3D>(op, diag[p], x + off, i, j + k * h, 0);
-    yc[p] = MODE == MODE_APPLY ? a : mk<double>(bc[p].x - a.x, bc[p].y - a.y);
+    yc[p] = result(a, p, MODE == MODE_APPLY ? a : bc[p]);
   }
 }
 
@@ -369,7 +382,8 @@ bool fine_fixed_pays(const FineOp& op, int ncols) {
 
 template <typename TX>
 void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag, const FixedDiag& fd,
-                       const cplx<TX>* x, const double2* b, double2* y, long long ld, const int* cols, int ncols) {
+                       const cplx<TX>* x, const double2* b, double2* y, long long ld, const int* cols, int ncols,
+                       const double2* dinv, double weight) {
   if (ncols <= 0) return;
   const bool is3d = op.g.nz > 1;
   FixOp o{};
@@ -389,13 +403,15 @@ void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag
   const int threads = (o.w * o.h + 31) / 32 * 32;
   const size_t smem = (size_t)(is3d ? kN + 2 : 1) * (rows + 2) * (o.w + 2) * sizeof(int4);
   const double nn = (double)op.g.N * ncols;
-  const double bytes = nn * (sizeof(cplx<TX>) + 16.0 + (mode == MODE_RESID ? 16.0 : 0.0)) + op.g.N * 16.0;
-  const char* name =
-      mode == MODE_APPLY ? (op.outer ? "outer_apply" : "fine_apply") : (op.outer ? "outer_resid" : "fine_resid");
+  const double bytes = nn * (sizeof(cplx<TX>) + 16.0 + (mode == MODE_APPLY ? 0.0 : 16.0)) +
+                       op.g.N * (mode == MODE_JACOBI ? 32.0 : 16.0);
+  const char* name = mode == MODE_APPLY   ? (op.outer ? "outer_apply" : "fine_apply")
+                     : mode == MODE_RESID ? (op.outer ? "outer_resid" : "fine_resid")
+                                          : "fine_jacobi";
   if (op.outer) ctx.add_flops(name, (8.0 * (is3d ? 3 : 2) + 8.0 + (mode == MODE_RESID ? 2.0 : 0.0)) * nn);
 #define HZ_FF(M, D, W)                                                                                               \
   HZ_LAUNCH(ctx, name, bytes, (k_fine_fixed<TX, M, D, W>), grid, threads, smem, o, fd.refs, fd.d, diag, x, b, y, \
-            ld, cols)
+            ld, cols, dinv, weight)
 #define HZ_FF_FORMS(M)                                   \
   do {                                                   \
     if (is3d && plain) HZ_FF(M, true, kPlain);           \
@@ -407,13 +423,15 @@ void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag
   } while (0)
   const bool plain = op.b[0] == op.o[0];
   if (mode == MODE_APPLY) HZ_FF_FORMS(MODE_APPLY);
-  else HZ_FF_FORMS(MODE_RESID);
+  else if (mode == MODE_RESID) HZ_FF_FORMS(MODE_RESID);
+  else if constexpr (std::is_same<TX, double>::value) HZ_FF_FORMS(MODE_JACOBI);
+  else throw std::runtime_error("fine operator: FP64 sweeps only");
 #undef HZ_FF_FORMS
 #undef HZ_FF
 }
 template void launch_fine_fixed<double>(Ctx&, int, const FineOp&, const double2*, const FixedDiag&, const double2*,
-                                        const double2*, double2*, long long, const int*, int);
+                                        const double2*, double2*, long long, const int*, int, const double2*, double);
 template void launch_fine_fixed<float>(Ctx&, int, const FineOp&, const double2*, const FixedDiag&, const float2*,
-                                       const double2*, double2*, long long, const int*, int);
+                                       const double2*, double2*, long long, const int*, int, const double2*, double);
 
 }  // namespace hz

@@ -1,7 +1,8 @@
 // Folding of the Gram-Schmidt sums and the per-column scalar steps of FGMRES, shared
 // by the FP64 (hz_krylov.cu) and the double-float (hz_df64.cu) kernels.
 //
-// A pass is two launches, dots and update.  The last block of a column to finish folds the
+// A pass is two launches, dots and update (the double-float form's first update carries the
+// second pass's dots).  The last block of a column to finish folds the
 // blocks' partial sums in block order (deterministic) and does the column's scalar work
 // there: the update coefficients after the dots, the DGKS test and, when no second pass is
 // due, the Hessenberg column, Givens rotation and residual estimate after the update.

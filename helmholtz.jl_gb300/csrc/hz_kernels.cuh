@@ -70,7 +70,7 @@ template <typename T, typename TX, typename TB>
 void launch_fine(Ctx& ctx, int mode, const FineOp& op, const cplx<T>* diag, const cplx<T>* dinv, const cplx<TX>* x,
                  const cplx<TB>* b, cplx<T>* y, long long ld, const int* cols, int ncols, double w);
 
-// y = op(x) or b - op(x) in FP64 accuracy on the integer pipe (hz_fine_fixed.cu), where
+// y = op(x), b - op(x) or x + weight dinv (b - op(x)) in FP64 accuracy on the integer pipe (hz_fine_fixed.cu), where
 // fine_fixed_pays() says so.  Rounds otherwise than launch_fine: not for arithmetic whose
 // bits have to be those of another path.
 struct FixedRefs {
@@ -86,7 +86,8 @@ void launch_diag_fixed(Ctx& ctx, const FineOp& op, const double2* d, FixedRefs* 
 bool fine_fixed_pays(const FineOp& op, int ncols);
 template <typename TX>
 void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag, const FixedDiag& fd,
-                       const cplx<TX>* x, const double2* b, double2* y, long long ld, const int* cols, int ncols);
+                       const cplx<TX>* x, const double2* b, double2* y, long long ld, const int* cols, int ncols,
+                       const double2* dinv = nullptr, double weight = 0.0);
 
 // The first Jacobi sweep y = w dinv .* r of a Galerkin level, written by the kernel that makes
 // its right-hand side r (y null: none): the same numbers as launch_jacobi0, which on small

@@ -747,6 +747,10 @@ template <typename T> const cplx<T>* lev_dinv(Level& L);
 template <> const double2* lev_dinv<double>(Level& L) { return L.dinv64.as<double2>(); }
 template <> const float2* lev_dinv<float>(Level& L) { return L.dinv32.as<float2>(); }
 
+FixedDiag fixed_diag(const hz_handle* h, int shifted) {
+  return FixedDiag{h->fixrefs.as<FixedRefs>() + shifted, (shifted ? h->diagSHfix : h->diagHfix).as<int4>()};
+}
+
 // One level operation in precision T with right-hand side of precision TB.
 template <typename T, typename TB>
 void lev_op(hz_handle* h, Hierarchy& H, int l, int mode, const cplx<T>* x, const cplx<TB>* b, cplx<T>* y,
@@ -754,6 +758,14 @@ void lev_op(hz_handle* h, Hierarchy& H, int l, int mode, const cplx<T>* x, const
   Level& L = *H.lv[l];
   const double w = h->opt.relax_param;
   if (L.fine) {
+    // FGMRES's FP64 cycle on large blocks (the finest level: a re-discretised one has its own
+    // diagonal); BiCGSTAB keeps the native steps' bits
+    if constexpr (std::is_same<T, double>::value && std::is_same<TB, double>::value)
+      if (h->opt.krylov == HZ_KRYLOV_FGMRES && L.fd64 == h->diagSH.as<double2>() && fine_fixed_pays(L.fop, nc)) {
+        launch_fine_fixed<double>(h->ctx, mode, L.fop, fine_diag<T>(L), fixed_diag(h, 1), x, b, y, L.ld, cols, nc,
+                                  fine_dinv<T>(L), w);
+        return;
+      }
     launch_fine<T, T, TB>(h->ctx, mode, L.fop, fine_diag<T>(L), fine_dinv<T>(L), x, b, y, L.ld, cols, nc, w);
   } else {
     launch_rap<T, TB>(h->ctx, mode, L.g, lev_coef<T>(L), L.g.N, lev_dinv<T>(L), x, b, y, L.ld, cols, nc, w, sweep);
@@ -1090,10 +1102,6 @@ void precondition(hz_handle* h, Hierarchy& H, const double2* vj, void* zj, const
   } else {
     mg_cycle<double, double>(h, H, 0, vj, (double2*)zj, cols, nc);
   }
-}
-
-FixedDiag fixed_diag(const hz_handle* h, int shifted) {
-  return FixedDiag{h->fixrefs.as<FixedRefs>() + shifted, (shifted ? h->diagSHfix : h->diagHfix).as<int4>()};
 }
 
 // y = H x (outer operator, FP64 accuracy) for the active columns.  native: in the FP64

@@ -72,3 +72,28 @@ def test_large_blocks_match_oracle(hz, O, cells, lengths, order):
                 bad = fin & ((abs(d.real) > bound) | (abs(d.imag) > bound))
             assert not bad.any(), (np.argwhere(bad)[:5], np.nanmax(np.where(fin, abs(d) / bound, 0)))
 
+
+
+@pytest.mark.parametrize("adjoint", [0, 1])
+@pytest.mark.parametrize("cells", [(64, 32), (16, 12, 10)])
+def test_cycle_on_large_blocks(hz, O, cells, adjoint):
+    """The FP64 cycle's finest level: a block above the threshold against its first columns
+    alone.  Both stop at a relative residual of 1e-10, so they differ by twice that times the
+    condition number (below 1e3 here); rounding may move the last iteration by one."""
+    P = PB.layered(cells, seed=3, pad=2)
+    n = P["m"].size
+    nrhs = -(-(1 << 17) // n)
+    B = PB.rhs(n, nrhs, seed=1)
+
+    def solve(C):
+        MG = hz.getMGparam(complex, int, 2 if len(cells) == 3 else 3, 1, 200, 1e-10, "Jac", 0.8, 1, 1, "V", "Julia", 0.5,
+                           0.0)
+        S = hz.getShiftedLaplacianMultigridSolver(PB.hz_param(hz, P), MG, 0.5, "GMRES", 10)
+        X, S = hz.solveLinearSystem(None, C, S, adjoint)
+        assert (S.last_relres <= 1e-10).all()
+        return X, np.asarray(S.last_iters)
+
+    X, it = solve(B)
+    Y, jt = solve(B[:, :3].copy())
+    assert np.abs(it[:3] - jt).max() <= 1
+    assert np.linalg.norm(X[:, :3] - Y) <= 2e-7 * np.linalg.norm(Y)

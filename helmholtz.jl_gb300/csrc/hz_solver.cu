@@ -2545,7 +2545,7 @@ void collect_targets_iterative(hz_handle* h, Hierarchy& H, int level, int sweeps
   const int last = (int)H.lv.size() - 1;
   if (level >= last) sweeps = 1;
   Level& Lv = *H.lv[level];
-  if (sweeps > 1 && !Lv.kv.p) {  // the two-step corrections' vectors (allocated by the K-cycle itself otherwise)
+  if (sweeps > 1) {  // the two-step corrections' vectors, for as many columns as this call's blocks hold
     Lv.kv.alloc((size_t)4 * R * Lv.ld * sizeof(double2));
     alloc_sums(h, Lv.g.N, R, Lv.ks, Lv.kp, Lv.kn);
   }

@@ -669,6 +669,7 @@ __global__ void k_fine_setup(Grid g, int dim, double h0, double h1, double h2, d
                              const double* __restrict__ gamma, double2* __restrict__ dH, double2* __restrict__ dSH,
                              double2* __restrict__ iSH, FixedRefs* __restrict__ refs) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned lanes = __ballot_sync(0xffffffffu, p < g.N);  // the lanes that take part in the maxima below
   if (p >= g.N) return;
   const int i = (int)(p % g.nx);
   const long long t = p / g.nx;
@@ -713,7 +714,6 @@ __global__ void k_fine_setup(Grid g, int dim, double h0, double h1, double h2, d
   auto ex = [](double v) { return __double2hiint(v) >> 20 & 0x7ff; };
   int off = max(ex(1.0 / (h0 * h0)), ex(1.0 / (h1 * h1)));
   if (dim == 3) off = max(off, ex(1.0 / (h2 * h2)));
-  const unsigned lanes = __activemask();
   const int eH = __reduce_max_sync(lanes, max(off, max(ex(hr), ex(hi))));
   const int eSH = __reduce_max_sync(lanes, max(off, max(ex(sr), ex(shi))));
   if ((threadIdx.x & 31) == 0) {

@@ -141,7 +141,11 @@ struct BandSolveOps {
   const BandBlock* dblocks = nullptr;  // device copy of blocks: one cooperative launch per solve
   const double2* T = nullptr;
   const double2* G = nullptr;
+  int cluster = 0, resident = 0;  // CTAs per cluster and clusters at once, from plan_band_solve (0: no clusters)
 };
+// The cluster schedule for T columns of op.N rows on the current device.
+template <typename T>
+void plan_band_solve(BandSolveOps& op);
 template <typename T>
 void launch_band_solve(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cplx<T>* x, long long ld, const int* cols,
                        int ncols, double2* work);

@@ -2,7 +2,9 @@
 #pragma once
 
 #include <cstdio>
+#include <mutex>
 #include <stdexcept>
+#include <string>
 
 #include "hz_kernels.cuh"
 
@@ -34,6 +36,30 @@ static inline void check_launch(const char* name) {
   } while (0)
 
 static constexpr int kSMs = 152;
+
+// A kernel's limit of dynamic shared memory belongs to the kernel on its device, not to a
+// launch or a thread.  So it is raised once per device, to the most that any launch takes: a
+// launch that set its own size could find it lowered by another thread's before it starts.
+struct SmemLimit {
+  std::mutex mu;
+  bool raised[kMaxDevices] = {};
+};
+static inline void raise_smem_limit(SmemLimit& limit, const void* kernel, size_t bytes, const char* name,
+                                    bool large_clusters = false) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= kMaxDevices) throw std::runtime_error(std::string(name) + ": device ordinal out of range");
+  std::lock_guard<std::mutex> lk(limit.mu);
+  if (limit.raised[dev]) return;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && large_clusters)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    throw std::runtime_error(std::string(name) + ": shared memory attribute: " + cudaGetErrorString(e));
+  }
+  limit.raised[dev] = true;
+}
 
 // Column chunking: enough CTAs in flight for 152 SMs while each CTA reuses
 // its per-node coefficients across as many right-hand sides as possible.

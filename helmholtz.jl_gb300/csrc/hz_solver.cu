@@ -528,6 +528,10 @@ void factor_coarsest(hz_handle* h, Hierarchy& H) {
   H.band.dblocks = H.bandB.as<BandBlock>();
 }
 
+  if (h->opt.precision == HZ_PREC_MIXED)
+    plan_band_solve<float>(H.band);
+  else
+    plan_band_solve<double>(H.band);
 void build_hierarchy(hz_handle* h, int adj) {
   Hierarchy& H = h->hier[adj];
   const int dim = h->prob.dim;
@@ -2657,6 +2661,7 @@ int hz_collect_pairs(hz_handle* h, const double* B, double* X, int64_t n, int32_
     res.alloc((size_t)R * N * 16);
     ev.alloc((size_t)R * N * 16);
     x1.alloc((size_t)R * N * 16);
+    plan_band_solve<double>(lu);
     sc.alloc((size_t)R * 4);
     nrm.alloc((size_t)R * 6 * 8);
     idc.alloc((size_t)R * sizeof(int));

@@ -905,33 +905,45 @@ __global__ void __launch_bounds__(32 * kBandWarps) k_band_cluster(int N, int nbk
   }
 }
 
-// Clusters of 16 CTAs (8 where the GPU takes no larger ones) with the given shared
-// memory that can be resident at once, per device; 0: not available.
+// Shared memory of a cluster's CTA: the column's three vectors.
+static constexpr size_t kBandSmemMax = 220 * 1024;
+static size_t band_smem(long long N) { return (size_t)N * 3 * sizeof(double2); }
+
+// Clusters of 16 CTAs (8 where the GPU takes no larger ones) with the column's vectors in
+// shared memory that can be resident at once; 0: not available.
 template <typename T>
-void band_cluster_shape(cudaStream_t st, size_t smem, int& ctas, int& resident) {
-  for (ctas = 16; ctas >= 8; ctas /= 2) {
+void plan_band_solve(BandSolveOps& op) {
+  op.cluster = op.resident = 0;
+  const size_t smem = band_smem(op.N);
+  if (smem > kBandSmemMax) return;
+  static SmemLimit limit;
+  try {
+    raise_smem_limit(limit, (const void*)k_band_cluster<T>, kBandSmemMax, "band_solve", true);
+  } catch (const std::runtime_error&) {
+    return;  // no such clusters here: the cooperative kernel
+  }
+  for (int ctas = 16; ctas >= 8; ctas /= 2) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(32 * kBandWarps);
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = (unsigned)ctas;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    resident = 0;
-    if (cudaFuncSetAttribute(k_band_cluster<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-            cudaSuccess &&
-        (ctas <= 8 || cudaFuncSetAttribute(k_band_cluster<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                          cudaSuccess) &&
-        cudaOccupancyMaxActiveClusters(&resident, k_band_cluster<T>, &cfg) == cudaSuccess && resident > 0)
+    int resident = 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, k_band_cluster<T>, &cfg) == cudaSuccess && resident > 0) {
+      op.cluster = ctas;
+      op.resident = resident;
       return;
+    }
     cudaGetLastError();
   }
-  ctas = resident = 0;
 }
+template void plan_band_solve<double>(BandSolveOps&);
+template void plan_band_solve<float>(BandSolveOps&);
 
 template <typename T>
 void launch_band_solve(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cplx<T>* x, long long ld, const int* cols,
@@ -957,9 +969,7 @@ void launch_band_solve(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cplx<
     // Clocks of both schedules: a cluster per column (as many at once as fit) and a
     // cluster barrier per step, or the columns over the whole GPU and a grid barrier
     // over as many CTAs as the widest step fills; two FP64 FMA lanes per SM and clock.
-    const size_t smem = (size_t)N * 3 * sizeof(double2);
-    int ctas = 0, resident = 0;
-    if (smem <= 220 * 1024) band_cluster_shape<T>(ctx.stream, smem, ctas, resident);
+    const int ctas = op.cluster, resident = op.resident;
     double cl = 0.0, gr = 0.0;
     long long rows = 1;
     for (const BandBlock& B : op.blocks) {
@@ -980,7 +990,7 @@ void launch_band_solve(Ctx& ctx, const BandSolveOps& op, const cplx<T>* b, cplx<
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3((unsigned)(ctas * ncols));
       cfg.blockDim = dim3(32 * kBandWarps);
-      cfg.dynamicSmemBytes = smem;
+      cfg.dynamicSmemBytes = band_smem(N);
       cfg.stream = ctx.stream;
       cudaLaunchAttribute at{};
       at.id = cudaLaunchAttributeClusterDimension;

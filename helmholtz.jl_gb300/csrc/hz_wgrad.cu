@@ -29,6 +29,7 @@ namespace {
 constexpr int kThreads = 256, kWarps = 8;
 constexpr int kSegBlocks = 18;  // 8-node blocks of a row segment: 144 nodes
 constexpr int kRing = 4;        // staged input rows per z-plane: three in use, one in flight
+constexpr size_t kSmemMax = 227 * 1024;
 
 struct WgShape {
   int nx, ny, nz, planes;  // planes: 1 (3 x 3 taps) or 3 (3 x 3 x 3)
@@ -213,10 +214,9 @@ size_t staged_bytes(const WgShape& s) {
 template <int CO, int NC>
 void wg_launch(Ctx& ctx, const char* name, WgShape s, long long planes_total, const WgradTc& a) {
   const size_t smem = staged_bytes(s);
-  if (cudaFuncSetAttribute(k_wgrad<CO, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    throw std::runtime_error("weight gradient: shared memory attribute");
-  }
+  if (smem > kSmemMax) throw std::runtime_error("weight gradient: channel counts not supported");
+  static SmemLimit limit;
+  raise_smem_limit(limit, (const void*)k_wgrad<CO, NC>, kSmemMax, "weight gradient");
   // Rows per CTA: the CTAs that fit at once, times one to four rounds of them, whichever
   // takes the fewest rows one after another (a chunk stages two rows more than it sums).
   int per_sm = 0;

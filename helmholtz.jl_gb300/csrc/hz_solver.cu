@@ -526,12 +526,12 @@ void factor_coarsest(hz_handle* h, Hierarchy& H) {
   ck(cudaMemcpy(H.bandB.p, H.band.blocks.data(), H.band.blocks.size() * sizeof(BandBlock), cudaMemcpyHostToDevice),
      "upload band blocks");
   H.band.dblocks = H.bandB.as<BandBlock>();
-}
-
   if (h->opt.precision == HZ_PREC_MIXED)
     plan_band_solve<float>(H.band);
   else
     plan_band_solve<double>(H.band);
+}
+
 void build_hierarchy(hz_handle* h, int adj) {
   Hierarchy& H = h->hier[adj];
   const int dim = h->prob.dim;
@@ -2655,13 +2655,13 @@ int hz_collect_pairs(hz_handle* h, const double* B, double* X, int64_t n, int32_
     lu.T = dT.as<double2>();
     lu.G = dG.as<double2>();
     lu.dblocks = dB.as<BandBlock>();
+    plan_band_solve<double>(lu);
     bw.alloc((size_t)3 * R * N * 16);
     DBuf xe, res, ev, x1, idc, sc, nrm;
     xe.alloc((size_t)R * N * 16);
     res.alloc((size_t)R * N * 16);
     ev.alloc((size_t)R * N * 16);
     x1.alloc((size_t)R * N * 16);
-    plan_band_solve<double>(lu);
     sc.alloc((size_t)R * 4);
     nrm.alloc((size_t)R * 6 * 8);
     idc.alloc((size_t)R * sizeof(int));

@@ -122,6 +122,18 @@ __device__ __forceinline__ double widen_f32(float f) {
 }
 #endif
 
+#ifdef __CUDACC__
+// FGMRES stores its basis unnormalised: v_j stands for sig_j v_j.  The next candidate is
+// 2^k H Z_j, k = basis_exponent(sig_j), so that it stands for tau_j = sig_j 2^-k in [1, 2) times itself
+// and the stored vectors keep to within one iteration's gain of 1.  (0 for a zero sig: a zero vector.)
+__device__ __forceinline__ int basis_exponent(double sig) {
+  const int f = __double2hiint(sig) >> 20 & 0x7ff;
+  return f == 0 || f == 0x7ff ? 0 : max(-100, min(100, f - 1023));
+}
+__device__ __forceinline__ double basis_power(int k) { return __hiloint2double((k + 1023) << 20, 0); }
+__device__ __forceinline__ double basis_tau(double sig) { return sig * basis_power(-basis_exponent(sig)); }
+#endif
+
 template <typename To, typename From> __host__ __device__ __forceinline__ cplx<To> ccast(cplx<From> a) {
   return mk<To>((To)a.x, (To)a.y);
 }

@@ -87,6 +87,8 @@ struct DFOp {
   long long N;
   float oh[3], ol[3], bh[3], bl[3];
   int adj;
+  const double* sig = nullptr;
+  int sig_stride = 0;
 };
 
 __device__ __forceinline__ void axis_df(int i, int n, const DFOp& op, int a, float& clh, float& cll, float& crh,
@@ -167,6 +169,11 @@ __global__ void __launch_bounds__(256) k_fine_df64(DFOp op, const float4* __rest
     }
     re.renorm();
     im.renorm();
+    if (op.sig) {
+      const float s = (float)basis_power(basis_exponent(op.sig[(long long)cols[ci] * op.sig_stride]));
+      re.init(s * re.hi, s * re.lo);
+      im.init(s * im.hi, s * im.lo);
+    }
     store_out(y, off + p, re, im);
   }
 }
@@ -187,6 +194,8 @@ void launch_fine_df64(Ctx& ctx, const FineOp& op, const float4* dHd, const float
     d.bl[a] = (float)(op.b[a] - (double)d.bh[a]);
   }
   d.adj = op.adj;
+  d.sig = op.sig;
+  d.sig_stride = op.sig_stride;
   const int TPB = 256;
   const long long nbx = (op.g.N + TPB - 1) / TPB;
   const int ch = chunks_for(nbx, ncols);

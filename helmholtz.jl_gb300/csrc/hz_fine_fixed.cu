@@ -58,6 +58,8 @@ struct FixOp {
   double o[3], b[3];
   int w, h;     // tile: w x h nodes (3D), w x kN h (2D)
   int tiles_x, tiles;
+  const double* sig;
+  int sig_stride;
   unsigned inv_w, inv_ring;  // 2^16 / w and 2^16 / ring, rounded up: quotients of numbers below 2 kThreads
 };
 // boundary rows: first order, second order, the second order's adjoint
@@ -232,7 +234,9 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
   if ((tid & 31) == 0) atomicMax(&largest, t);
   __syncthreads();
   const int E = (int)(largest >> 20);
-  const bool ok = refs->ok && fixed_ref_ok(E) && fixed_ok(E + Ec);
+  // the power of two that the results are scaled by
+  const int power = MODE == MODE_APPLY && op.sig ? basis_exponent(op.sig[(long long)cols[blockIdx.z] * op.sig_stride]) : 0;
+  const bool ok = refs->ok && fixed_ref_ok(E) && fixed_ok(E + Ec) && fixed_ok(E + Ec + power);
   if (ok) {
     const uint32_t top = largest | 0xfffffu;
     if (mine) {
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
   const int nk = !mine || i >= op.nx ? 0 : IS3D ? (j < op.ny ? op.nz - z0 : 0) : op.ny - j;  // 2D: rows below
   const int gs = IS3D ? sz : h * sy;  // a plane or h rows
   const int p0 = z0 * sz + (j * sy + i);
-  const int e0 = E + Ec + 1 - kFixedScale;  // exponent of a total's unit
+  const int e0 = E + Ec + power + 1 - kFixedScale;  // exponent of a total's unit
   const int4* c = cell + base + (IS3D ? step : 0);
   const double2* bc = b + off;
   double2* yc = y + off;
@@ -311,8 +315,9 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
     const int k = __ffs((int)native) - 1;
     native &= native - 1;
     const int p = p0 + k * gs;
-    const double2 a = IS3D ? native_node<TX, IS3D>(op, diag[p], x + off, i, j, z0 + k)
-                           : native_node<TX, IS3D>(op, diag[p], x + off, i, j + k * h, 0);
+    double2 a = IS3D ? native_node<TX, IS3D>(op, diag[p], x + off, i, j, z0 + k)
+                     : native_node<TX, IS3D>(op, diag[p], x + off, i, j + k * h, 0);
+    if (power) a = cscale<double>(basis_power(power), a);
     yc[p] = result(a, p, MODE == MODE_APPLY ? a : bc[p]);
   }
 }
@@ -391,6 +396,8 @@ void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag
   o.ny = op.g.ny;
   o.nz = op.g.nz;
   o.adj = op.adj;
+  o.sig = op.sig;
+  o.sig_stride = op.sig_stride;
   o.uniform = op.o[0] == op.o[1] && (!is3d || op.o[0] == op.o[2]);
   for (int a = 0; a < 3; ++a) {
     o.o[a] = op.o[a];

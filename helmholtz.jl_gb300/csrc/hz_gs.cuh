@@ -123,8 +123,8 @@ __device__ __forceinline__ void gs_after_dots(const GsColumn& g, int c, int i0, 
   if (want_norm && threadIdx.x == 0) out[K] = mk<double>(tot[2 * K], 0.0);
 }
 
-// Step j of column c is complete: Hessenberg entries of the normalised basis (sig_i sig_j d_i,
-// h_{j+1,j} = sig_j ||w''||), Givens rotations (u, v) -> (conj(c) u + conj(s) v, -s u + c v),
+// Step j of column c is complete: Hessenberg entries of the normalised basis (sig_i tau_j d_i,
+// h_{j+1,j} = tau_j ||w''||), Givens rotations (u, v) -> (conj(c) u + conj(s) v, -s u + c v),
 // residual estimate (to the device and to pinned host memory) and the next scale.
 // Called by one warp.
 __device__ __forceinline__ void gs_finish(const GsColumn& g, int c, int j, bool second, double n2) {
@@ -132,7 +132,7 @@ __device__ __forceinline__ void gs_finish(const GsColumn& g, int c, int j, bool 
   const double* sc = g.sig + (long long)c * g.sstride;
   double2* H = g.Hh + (long long)c * (m + 1) * m + (long long)j * (m + 1);
   const double2 *csc = g.cs + (long long)c * m, *snc = g.sn + (long long)c * m;
-  const double sj = sc[j];
+  const double sj = basis_tau(sc[j]);  // the candidate's scale
   for (int i = lane; i <= j; i += 32) {
     double2 v = g.hA[(long long)c * g.hstride + i];
     const double f = sc[i] * sj;

@@ -122,11 +122,16 @@ template <typename T> __device__ __forceinline__ void add_norm(T (&v)[kNV], int 
   v[i] = fma(w.x, w.x, fma(w.y, w.y, v[i]));
 }
 
-// coefficient a / n (0 for n = 0) in the vectors' precision
-template <typename T> __device__ __forceinline__ cplx<T> ratio(double2 a, double n) {
-  return n > 0.0 ? mk<T>((T)(a.x / n), (T)(a.y / n)) : mk<T>(0, 0);
+// coefficient in the vectors' precision; 0 unless finite: a step whose squares leave the range of
+// FP32 (vectors beyond 1e19) corrects nothing
+template <typename T> __device__ __forceinline__ cplx<T> narrow(double2 a) {
+  const T x = (T)a.x, y = (T)a.y;
+  return isfinite(x) && isfinite(y) ? mk<T>(x, y) : mk<T>(0, 0);
 }
-template <typename T> __device__ __forceinline__ cplx<T> narrow(double2 a) { return mk<T>((T)a.x, (T)a.y); }
+// a / n (0 for n = 0)
+template <typename T> __device__ __forceinline__ cplx<T> ratio(double2 a, double n) {
+  return n > 0.0 ? narrow<T>(make_double2(a.x / n, a.y / n)) : mk<T>(0, 0);
+}
 
 // Two-step least squares from the sums: the 3 x 2 problem min || beta e0 - H y || by two
 // complex Givens rotations, H = [[h00, h01], [h10, h11], [0, h21]] of the normalised
@@ -165,8 +170,9 @@ template <typename T> __device__ void least_squares(const double2* s, double n2,
       if (rn1 > 0.0) y1 = make_double2(y1.x / rn1, y1.y / rn1);
     }
   }
-  kt[6] = narrow<T>(y0);
-  kt[7] = narrow<T>(y1);
+  const bool ok = isfinite((T)y0.x) && isfinite((T)y0.y) && isfinite((T)y1.x) && isfinite((T)y1.y);
+  kt[6] = ok ? narrow<T>(y0) : mk<T>(0, 0);
+  kt[7] = ok ? narrow<T>(y1) : mk<T>(0, 0);
 }
 
 }  // namespace

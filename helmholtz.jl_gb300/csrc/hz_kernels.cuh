@@ -61,6 +61,9 @@ struct FineOp {
   double b[3];  // BC/h_d^2: boundary-row off-diagonal magnitude per axis
   int adj;      // 1: apply the adjoint (transposed boundary rows, conjugated diagonal)
   int outer = 0;  // 1: the Krylov method's operator H (launch-table names outer_*), 0: a cycle operator
+  // FP64 MODE_APPLY: column c's result times 2^basis_exponent(sig[c * sig_stride]) (null: as it is)
+  const double* sig = nullptr;
+  int sig_stride = 0;
 };
 
 // y = op(x) on nodes of a fine level, for the columns cols[0..ncols) of the

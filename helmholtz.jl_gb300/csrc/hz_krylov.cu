@@ -406,9 +406,11 @@ void launch_reduce(Ctx& ctx, const double2* part, const int* cols, int ncols, in
 // The stored basis vector v_i of column c stands for V_i = sig_i v_i with
 // sig_i = sig[c*sstride + i] > 0, so no pass over the vector is spent on
 // normalising it.  From the stored dots d_i = conj(v_i) . w' of the stored
-// candidate w' (= H Z'_j, Z'_j the cycle applied to v_j): the update uses the
-// coefficients sig_i^2 d_i, the Hessenberg entries are sig_i sig_j d_i and
-// h_{j+1,j} = sig_j ||w''|| (hz_gs.cuh).
+// candidate w' (= 2^k H Z'_j, Z'_j the cycle applied to v_j, tau_j = 2^-k sig_j in [1, 2)): the
+// update uses the coefficients sig_i^2 d_i, the Hessenberg entries are sig_i tau_j d_i,
+// h_{j+1,j} = tau_j ||w''|| and sig_{j+1} = tau_j / h_{j+1,j} (hz_gs.cuh).  Without the power of
+// two the scale is the product of all h: a cycle that amplifies took the FP32 levels' sums of squares
+// out of range within a restart.  It changes no bit inside it.
 __global__ void k_sig_init(const int* __restrict__ cols, int ncols, double* __restrict__ sig, int sstride) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < ncols) sig[(long long)cols[i] * sstride] = 1.0;

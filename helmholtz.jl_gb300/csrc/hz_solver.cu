@@ -1109,13 +1109,15 @@ void precondition(hz_handle* h, Hierarchy& H, const double2* vj, void* zj, const
 }
 
 // y = H x (outer operator, FP64 accuracy) for the active columns.  native: in the FP64
-// pipe's own steps.
+// pipe's own steps.  sig: MODE_APPLY's powers of two (FineOp::sig).
 template <typename TX>
 void apply_H(hz_handle* h, int adj, int mode, const cplx<TX>* x, const double2* b, double2* y, const int* cols,
-             int nc, bool native = false) {
+             int nc, bool native = false, const double* sig = nullptr) {
   FineOp fop = h->fop;
   fop.adj = adj;
   fop.outer = 1;
+  fop.sig = sig;
+  fop.sig_stride = h->mcap + 1;
   if (!native && fine_fixed_pays(fop, nc))
     launch_fine_fixed<TX>(h->ctx, mode, fop, h->diagH.as<double2>(), fixed_diag(h, 0), x, b, y, h->g0.N, cols, nc);
   else
@@ -1463,7 +1465,7 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
       // (dots + ||w||^2, update + ||w'||^2) for every column, pass 1 only for the columns
       // whose norm dropped below 1/sqrt(2) of its value (masked on the device); the
       // Hessenberg column, rotation and residual estimate follow in the column's last pass.
-      // v_{j+1} = w'' stays unnormalised: sig_{j+1} = sig_j / h_{j+1,j}.  The estimates
+      // v_{j+1} = w'' stays unnormalised: sig_{j+1} = tau_j / h_{j+1,j}.  The estimates
       // arrive in pinned memory.
       cycle_graph(h, adj, j, nl, df ? 2 : mixed ? 1 : 0, [&] {
         if (df) {
@@ -1471,13 +1473,15 @@ int fgmres(hz_handle* h, int adj, int nrhs) {
           mg_cycle<float, df64_tag>(h, H, 0, Vdj(j), (float2*)Zj(j), dc, nl);
           FineOp fop = h->fop;
           fop.adj = adj;
+          fop.sig = sig + j;
+          fop.sig_stride = SS;
           launch_fine_df64(h->ctx, fop, h->diagHdf.as<float4>(), (const float2*)Zj(j), Vdj(j + 1), N, dc, nl);
         } else {
           precondition(h, H, Vj(j), Zj(j), dc, nl);
           if (mixed)
-            apply_H<float>(h, adj, MODE_APPLY, (const float2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
+            apply_H<float>(h, adj, MODE_APPLY, (const float2*)Zj(j), nullptr, Vj(j + 1), dc, nl, false, sig + j);
           else
-            apply_H<double>(h, adj, MODE_APPLY, (const double2*)Zj(j), nullptr, Vj(j + 1), dc, nl);
+            apply_H<double>(h, adj, MODE_APPLY, (const double2*)Zj(j), nullptr, Vj(j + 1), dc, nl, false, sig + j);
         }
         if (df)
           launch_gs_df(h->ctx, N, Vd, vstride, N, j, dc, nl, gs);

@@ -94,6 +94,8 @@ template <typename T> struct FineOpT {
   long long N;
   T o[3], b[3];
   int adj;
+  const double* sig = nullptr;
+  int sig_stride = 0;
 };
 
 // Off-diagonal magnitudes of the two neighbours of node i on an axis of n
@@ -165,6 +167,8 @@ __global__ void __launch_bounds__(256) k_fine(FineOpT<T> op, const cplx<T>* __re
     // b is read once and y written once: streaming hints keep the cache for the
     // x planes whose neighbours are read again
     if (MODE == MODE_APPLY) {
+      if (std::is_same<T, double>::value && op.sig)
+        ax = cscale<T>((T)basis_power(basis_exponent(op.sig[(long long)cols[ci] * op.sig_stride])), ax);
       __stcs(&y[off + p], ax);
     } else {
       const cplx<TB> bb = __ldcs(&b[off + p]);
@@ -193,6 +197,8 @@ void launch_fine(Ctx& ctx, int mode, const FineOp& op, const cplx<T>* diag, cons
     o.b[d] = (T)op.b[d];
   }
   o.adj = op.adj;
+  o.sig = op.sig;
+  o.sig_stride = op.sig_stride;
   const int TPB = 256;
   long long nbx = (op.g.N + TPB - 1) / TPB;
   int ch = ctx.tune_fine > 0 ? chunks_for(nbx, ncols, ctx.tune_fine) : chunks_for(nbx, ncols);

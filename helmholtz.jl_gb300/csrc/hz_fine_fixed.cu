@@ -15,10 +15,12 @@
 //
 // A value is off by at most 2^-56 of the brick's reference.  A node with no value, its own or a
 // neighbour's, above 2^-5 of it takes the native steps; so do bricks whose exponents are out of
-// range and values that are NaN or Inf.  Against quad precision the product's error is 5.1e-17
-// of its norm on noise (native 7.5e-17), 9.2e-17 on plane waves (5.4e-16) and 6.0e-17 to 7.4e-17
-// on noise that decays or spreads over 2^6 (7.4e-17 to 7.6e-17).  At a single node it is at most
-// 3.8 u of the row's sum of magnitudes, u = 2^-53 (native 1.7 u): a node 2^-5 below its brick.
+// range and values that are NaN or Inf.  Zeros (a brick's, a node's with its neighbours) are not
+// worked on: a sparse column has little else.  Against quad precision the product's error is
+// 5.1e-17 of its norm on noise (native 7.5e-17), 9.2e-17 on plane waves (5.4e-16) and 6.0e-17 to
+// 7.4e-17 on noise that decays or spreads over 2^6 (7.4e-17 to 7.6e-17).  At a single node it is
+// at most 3.8 u of the row's sum of magnitudes, u = 2^-53 (native 1.7 u): a node 2^-5 below its
+// brick.
 //
 // Measured: 157 x 131 x 101 nodes, 13 columns, adjoint: 887 us native, 452; 129^3 nodes, 8 columns of
 // FP32 537 and 355; 1025 x 513 nodes, 16 columns of FP32 176 and 114; the FP64 cycle's residual
@@ -29,6 +31,7 @@
 // bricks per SM, took 326 to 330 instead of 355 in that one case and 2% to 8% longer in the other
 // two; giving every third or fourth brick to the native steps took a quarter longer.
 #include <algorithm>
+#include <cstring>
 #include <stdexcept>
 #include <type_traits>
 
@@ -70,6 +73,7 @@ template <typename TX> struct Raw;
 template <> struct Raw<double> {
   using type = uint4;
   static __device__ __forceinline__ uint4 widen(uint4 r) { return r; }
+  static __device__ __forceinline__ uint32_t any(uint4 r) { return r.x | r.z | (r.y | r.w) << 1; }
 };
 template <> struct Raw<float> {
   using type = uint2;
@@ -79,6 +83,7 @@ template <> struct Raw<float> {
     widen_f32_hilo(r.y, w.w, w.z);
     return w;
   }
+  static __device__ __forceinline__ uint32_t any(uint2 r) { return (r.x | r.y) << 1; }
 };
 
 // |v| in units of 2^(E - 1022 - kBits), truncated; s = E - exponent field (a zero or
@@ -148,6 +153,20 @@ __device__ __forceinline__ double2 native_node(const FixOp& op, double2 d, const
   }
   if (op.adj) d.y = -d.y;
   return cfma<double>(d, ccast<double, TX>(xc[p]), mk<double>(-sr, -si));
+}
+
+// Whether a node and its neighbours are zeros
+template <typename TX, bool IS3D>
+__device__ __forceinline__ bool no_value(const FixOp& op, const cplx<TX>* xc, int i, int j, int k) {
+  const long long sy = op.nx, sz = (long long)op.nx * op.ny;
+  const typename Raw<TX>::type* x = reinterpret_cast<const typename Raw<TX>::type*>(xc) + (i + sy * j + sz * k);
+  const int at[3] = {i, j, k}, n[3] = {op.nx, op.ny, op.nz};
+  const long long st[3] = {1, sy, sz};
+  uint32_t any = Raw<TX>::any(__ldg(x));
+#pragma unroll
+  for (int a = 0; a < (IS3D ? 3 : 2); ++a)
+    any |= Raw<TX>::any(__ldg(x - (at[a] > 0 ? st[a] : 0))) | Raw<TX>::any(__ldg(x + (at[a] < n[a] - 1 ? st[a] : 0)));
+  return any == 0;
 }
 
 struct Acc {
@@ -235,8 +254,19 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
   __syncthreads();
   const int E = (int)(largest >> 20);
   // the power of two that the results are scaled by
-  const int power = MODE == MODE_APPLY && op.sig ? basis_exponent(op.sig[(long long)cols[blockIdx.z] * op.sig_stride]) : 0;
-  const bool ok = refs->ok && fixed_ref_ok(E) && fixed_ok(E + Ec) && fixed_ok(E + Ec + power);
+  const int power =
+      MODE == MODE_APPLY && op.sig ? basis_exponent(op.sig[(long long)cols[blockIdx.z] * op.sig_stride]) : 0;
+  const bool ok = fixed_ref_ok(E) && fixed_ok(E + Ec) && fixed_ok(E + Ec + power);
+  // a brick without a value; its zeros may stand with their powers in E
+  bool empty = false;
+  if (E < kFixedMin) {
+    uint32_t any = 0;
+#pragma unroll
+    for (int q = 0; q < NL; ++q) any |= Raw<double>::any(own[q]);
+#pragma unroll
+    for (int q = 0; q < kHalo; ++q) any |= Raw<double>::any(halo[q]);
+    empty = !__syncthreads_or((int)any);
+  }
   if (ok) {
     const uint32_t top = largest | 0xfffffu;
     if (mine) {
@@ -273,9 +303,13 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
   for (int k = 0; k < kN; ++k) {
     if ((IS3D ? k : k * h) >= nk) break;
     const int p = p0 + k * gs;
-    const int4 d = __ldg(dfix + p);
     double2 bb = mk<double>(0, 0);
     if (MODE != MODE_APPLY) bb = __ldcs(bc + p);
+    if (empty) {
+      __stcs(yc + p, result(mk<double>(0, 0), p, bb));
+      continue;
+    }
+    const int4 d = __ldg(dfix + p);
     const int4* ck = c + k * step;
     const int4 n0 = ck[0], nl = ck[-1], nr = ck[1], nu = ck[-pitch], nd = ck[pitch];
     const int4 zero = make_int4(0, 0, 0, 0);
@@ -307,6 +341,8 @@ __global__ void __launch_bounds__(kThreads, IS3D ? 4 : 5)
       const Assemble out(e0 - pown[k + ZH]);
       const double2 a = mk<double>(out(re.total()), out(im.total()));
       __stcs(yc + p, result(a, p, bb));
+    } else if (ok && no_value<TX, IS3D>(op, x + off, i, IS3D ? j : j + k * h, IS3D ? z0 + k : 0)) {
+      __stcs(yc + p, result(mk<double>(0, 0), p, bb));
     } else {
       native |= 1u << k;
     }
@@ -330,8 +366,6 @@ __global__ void __launch_bounds__(256) k_diag_fixed(long long N, const double2* 
     refs->o[0] = negative(coefficient(o0, E));
     refs->o[1] = negative(coefficient(o1, E));
     refs->o[2] = dim == 3 ? negative(coefficient(o2, E)) : Fixed{0, 0};
-    const double least = min(min(o0, o1), dim == 3 ? o2 : o1);
-    refs->ok = fixed_ref_ok(E) && E - fixed_exponent((uint32_t)__double2hiint(least)) <= kRange;
   }
   if (p >= N) return;
   const double2 v = d[p];
@@ -369,6 +403,19 @@ void choose_tile(FixOp& op, bool is3d) {
 void launch_diag_fixed(Ctx& ctx, const FineOp& op, const double2* d, FixedRefs* refs, int4* out) {
   HZ_LAUNCH(ctx, "fine_setup", (double)op.g.N * 32.0, k_diag_fixed, (unsigned)((op.g.N + 255) / 256), 256, 0, op.g.N, d,
             op.g.nz > 1 ? 3 : 2, op.o[0], op.o[1], op.o[2], refs, out);
+}
+
+// The neighbours' coefficients within kRange exponents of the largest coefficient, the diagonal:
+// 8 to 16 times the smallest of them, as they lie in their binades.  Spacings more unequal (one axis
+// of three stretched by 1.4 to 2.4, one of two by 1.7 to 2.6) and diagonals far above the
+// Laplacian's stay with the native kernel.  157 x 131 x 101 nodes, 13 columns, ratio 4: 890 us
+// there, 1,166 with every node of every brick left to the native steps.
+bool fine_fixed_fits(const FineOp& op, int exponent) {
+  double least = std::min(op.o[0], op.o[1]);
+  if (op.g.nz > 1) least = std::min(least, op.o[2]);
+  uint64_t bits;
+  std::memcpy(&bits, &least, sizeof(bits));
+  return fixed_ref_ok(exponent) && exponent - fixed_exponent((uint32_t)(bits >> 32)) <= kRange;
 }
 
 bool fine_fixed_pays(const FineOp& op, int ncols) {

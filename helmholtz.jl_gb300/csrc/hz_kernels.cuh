@@ -74,19 +74,19 @@ void launch_fine(Ctx& ctx, int mode, const FineOp& op, const cplx<T>* diag, cons
                  const cplx<TB>* b, cplx<T>* y, long long ld, const int* cols, int ncols, double w);
 
 // y = op(x), b - op(x) or x + weight dinv (b - op(x)) in FP64 accuracy on the integer pipe (hz_fine_fixed.cu), where
-// fine_fixed_pays() says so.  Rounds otherwise than launch_fine: not for arithmetic whose
-// bits have to be those of another path.
+// fine_fixed_fits() and fine_fixed_pays() say so.  Rounds otherwise than launch_fine: not for
+// arithmetic whose bits have to be those of another path.
 struct FixedRefs {
   int exponent;  // the largest of the operator's coefficients, from launch_fine_setup
-  int ok;        // whether the rest lie near enough to it; this and below from launch_diag_fixed
-  Fixed o[3];    // minus the neighbours' coefficients per axis
+  Fixed o[3];    // minus the neighbours' coefficients per axis, from launch_diag_fixed
 };
 struct FixedDiag {
   const FixedRefs* refs;
   const int4* d;  // the diagonal's limbs, from launch_diag_fixed
 };
 void launch_diag_fixed(Ctx& ctx, const FineOp& op, const double2* d, FixedRefs* refs, int4* out);
-bool fine_fixed_pays(const FineOp& op, int ncols);
+bool fine_fixed_fits(const FineOp& op, int exponent);  // the operator's coefficients
+bool fine_fixed_pays(const FineOp& op, int ncols);     // the block
 template <typename TX>
 void launch_fine_fixed(Ctx& ctx, int mode, const FineOp& op, const double2* diag, const FixedDiag& fd,
                        const cplx<TX>* x, const double2* b, double2* y, long long ld, const int* cols, int ncols,

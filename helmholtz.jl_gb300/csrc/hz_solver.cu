@@ -146,6 +146,7 @@ struct hz_handle {
   // fine-level diagonals: H, SH (FP64), 1/diag(SH) (FP64), FP32 copies of SH
   DBuf diagH, diagSH, dinvSH, diagSH32, dinvSH32;
   DBuf fixrefs, diagHfix, diagSHfix;  // H and SH for the integer pipe (FixedDiag)
+  bool fix_fits[2] = {false, false};  // whether their coefficients fit it
   DBuf diagHdf;  // diag(H) in df64 (emulated-FP64 outer arithmetic)
   Hierarchy hier[2];
   // FGMRES workspace
@@ -754,6 +755,9 @@ template <> const float2* lev_dinv<float>(Level& L) { return L.dinv32.as<float2>
 FixedDiag fixed_diag(const hz_handle* h, int shifted) {
   return FixedDiag{h->fixrefs.as<FixedRefs>() + shifted, (shifted ? h->diagSHfix : h->diagHfix).as<int4>()};
 }
+bool use_fixed(const hz_handle* h, const FineOp& op, int shifted, int ncols) {
+  return h->fix_fits[shifted] && fine_fixed_pays(op, ncols);
+}
 
 // One level operation in precision T with right-hand side of precision TB.
 template <typename T, typename TB>
@@ -765,7 +769,7 @@ void lev_op(hz_handle* h, Hierarchy& H, int l, int mode, const cplx<T>* x, const
     // FGMRES's FP64 cycle on large blocks (the finest level: a re-discretised one has its own
     // diagonal); BiCGSTAB keeps the native steps' bits
     if constexpr (std::is_same<T, double>::value && std::is_same<TB, double>::value)
-      if (h->opt.krylov == HZ_KRYLOV_FGMRES && L.fd64 == h->diagSH.as<double2>() && fine_fixed_pays(L.fop, nc)) {
+      if (h->opt.krylov == HZ_KRYLOV_FGMRES && L.fd64 == h->diagSH.as<double2>() && use_fixed(h, L.fop, 1, nc)) {
         launch_fine_fixed<double>(h->ctx, mode, L.fop, fine_diag<T>(L), fixed_diag(h, 1), x, b, y, L.ld, cols, nc,
                                   fine_dinv<T>(L), w);
         return;
@@ -1118,7 +1122,7 @@ void apply_H(hz_handle* h, int adj, int mode, const cplx<TX>* x, const double2* 
   fop.outer = 1;
   fop.sig = sig;
   fop.sig_stride = h->mcap + 1;
-  if (!native && fine_fixed_pays(fop, nc))
+  if (!native && use_fixed(h, fop, 0, nc))
     launch_fine_fixed<TX>(h->ctx, mode, fop, h->diagH.as<double2>(), fixed_diag(h, 0), x, b, y, h->g0.N, cols, nc);
   else
     launch_fine<double, TX, double>(h->ctx, mode, fop, h->diagH.as<double2>(), nullptr, x, b, y, h->g0.N, cols, nc,
@@ -1719,7 +1723,10 @@ void init_fine(hz_handle* h) {
                       h->fixrefs.as<FixedRefs>());
     launch_diag_fixed(h->ctx, h->fop, h->diagH.as<double2>(), h->fixrefs.as<FixedRefs>(), h->diagHfix.as<int4>());
     launch_diag_fixed(h->ctx, h->fop, h->diagSH.as<double2>(), h->fixrefs.as<FixedRefs>() + 1, h->diagSHfix.as<int4>());
+    FixedRefs refs[2];
+    ck(cudaMemcpyAsync(refs, h->fixrefs.p, sizeof(refs), cudaMemcpyDeviceToHost, h->ctx.stream), "coefficient exponents");
     sync(h);
+    for (int k = 0; k < 2; ++k) h->fix_fits[k] = fine_fixed_fits(h->fop, refs[k].exponent);
   }
   if (h->opt.precision == HZ_PREC_MIXED && h->opt.outer_arith == HZ_OUTER_EMULATED) {
     h->diagHdf.alloc((size_t)N * 16);
@@ -2049,9 +2056,10 @@ int hz_apply(hz_handle* h, int32_t op, int32_t transpose, const double* X, doubl
     FineOp fop = h->fop;
     fop.adj = transpose ? 1 : 0;
     const double2* diag = (op == HZ_OP_H) ? h->diagH.as<double2>() : h->diagSH.as<double2>();
-    if (fine_fixed_pays(fop, nrhs))
-      launch_fine_fixed<double>(h->ctx, MODE_APPLY, fop, diag, fixed_diag(h, op == HZ_OP_H ? 0 : 1), xd, nullptr,
-                                yd, n, h->apply_cols.as<int>(), nrhs);
+    const int shifted = op == HZ_OP_H ? 0 : 1;
+    if (use_fixed(h, fop, shifted, nrhs))
+      launch_fine_fixed<double>(h->ctx, MODE_APPLY, fop, diag, fixed_diag(h, shifted), xd, nullptr, yd, n,
+                                h->apply_cols.as<int>(), nrhs);
     else
       launch_fine<double, double, double>(h->ctx, MODE_APPLY, fop, diag, nullptr, xd, (const double2*)nullptr, yd, n,
                                           h->apply_cols.as<int>(), nrhs, 0.0);

@@ -14,8 +14,8 @@
 // digit is exact in BF16, a product of two digits is an integer below 2^14, and
 // the FP32 accumulators of the tensor core stay exact integers for kFlush steps
 // (below 2^24); they are then folded into 64-bit integers.  Digit pairs (i, j)
-// with i + j < S are kept.  S = 8 for FP64 columns, S = 6 (48 bits, as the
-// double-float pairs of the emulated mode hold) where b and x are FP32.
+// with i + j < S are kept.  S = 8 (64 bits below the row's and the column's largest), or S = 6
+// (48 bits) in the emulated mode, whose double-float pairs hold no more.
 //
 // Why: GB300 has two FP64 FMA lanes per clock and SM, so a band substitution in
 // FP64 is bound by that pipe and by its chain of grid barriers, two per kl rows.
@@ -650,8 +650,10 @@ template <>
 void launch_coarse<float>(Ctx& ctx, const CoarseOp& op, const float2* b, float2* x, long long ld, const int* cols,
                           int ncols, void* work) {
   if (ncols <= 0) return;
-  if (op.slices != 6) throw std::runtime_error("coarse solve of FP32 columns takes the 6-digit image");
-  coarse_solve<float, 6>(ctx, op, b, x, ld, cols, ncols, work);
+  if (op.slices == 8)
+    coarse_solve<float, 8>(ctx, op, b, x, ld, cols, ncols, work);
+  else
+    coarse_solve<float, 6>(ctx, op, b, x, ld, cols, ncols, work);
 }
 
 }  // namespace hz

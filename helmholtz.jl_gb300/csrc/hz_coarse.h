@@ -12,7 +12,7 @@ static constexpr long long kCoarseDenseMax = 8192;
 
 struct CoarseOp {
   long long N = 0;
-  int slices = 0;             // digits per value: 8 (FP64 columns) or 6 (FP32 columns)
+  int slices = 0;             // digits per value: 8, or 6 (48 bits)
   void* image = nullptr;      // image_bytes(), zero-filled before the setup (padding rows and columns)
   int* rscale = nullptr;      // N row scales (powers of two)
   int steps() const { return (int)((N + 7) / 8); }

@@ -421,7 +421,6 @@ void band_factor_level(hz_handle* h, const Hierarchy& H, const Level& L, std::ve
 bool invert_coarsest(hz_handle* h, Hierarchy& H) {
   Level& L = *H.lv.back();
   const long long N = L.g.N;
-  const bool fp64 = h->opt.precision != HZ_PREC_MIXED;
   // BiCGSTAB's short recurrences carry a rounding difference of the cycle into the
   // iteration count (103 against 112 iterations for one source of a 257 x 129 grid),
   // where FGMRES contracts it: its native-FP64 cycles keep the band substitution
@@ -429,7 +428,8 @@ bool invert_coarsest(hz_handle* h, Hierarchy& H) {
   if (!coarse_supported(L.g)) return false;
   CoarseOp& op = H.coarse;
   op.N = N;
-  op.slices = fp64 ? 8 : 6;
+  // the emulated form holds FP64 data in 48 bits throughout, the others in all of its 53
+  op.slices = h->opt.precision == HZ_PREC_MIXED && h->opt.outer_arith == HZ_OUTER_EMULATED ? 6 : 8;
   const std::vector<std::complex<double>> coef = level_coefficients(h, H, L);
   cudaStream_t st = h->ctx.stream;
   try {

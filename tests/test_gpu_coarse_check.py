@@ -54,3 +54,16 @@ def test_damped_operators_take_the_inverse(hz, cells):
     t = launches(hz, S)
     assert t["coarse_product"][0] > 1 and "band_solve" not in t
 
+
+@pytest.mark.parametrize("precision,outer,digits", [("fp64", "fp64", 8), ("mixed", "fp64", 8), ("mixed", "emulated", 6)])
+def test_digits_of_the_inverse(hz, precision, outer, digits):
+    """The mixed form's coarsest level is FP64 (8 digits of 8 bits; FP32 is what its cycle's vectors
+    are held in); the emulated form's holds the 48 bits of its double-float data.  Bytes charged to a
+    product: 4 per digit and entry of the inverse, and the columns."""
+    P = PB.layered((64, 32), seed=4, pad=4)
+    S = solver(hz, PB.hz_param(hz, P), levels=3, precision=precision, outer=outer, shift=0.5)
+    hz.solveLinearSystem(None, PB.rhs(P["m"].size, 3, seed=1), S)
+    n, by = launches(hz, S)["coarse_product"]
+    N = 17 * 9
+    assert by / n >= 4 * digits * N * N
+    assert by / n < 4 * (digits + 1) * N * N

@@ -767,6 +767,13 @@ bool use_fixed(const hz_handle* h, const FineOp& op, int shifted, int ncols) {
   return h->fix_fits[shifted] && fine_fixed_pays(op, ncols);
 }
 
+// FGMRES's FP64 cycle on large blocks takes the integer pipe on the finest level (a re-discretised
+// one has its own diagonal); BiCGSTAB keeps the native steps' bits.
+template <typename T, typename TB> bool lev_fixed(const hz_handle* h, const Level& L, int nc) {
+  return std::is_same<T, double>::value && std::is_same<TB, double>::value && h->opt.krylov == HZ_KRYLOV_FGMRES &&
+         L.fine && L.fd64 == h->diagSH.as<double2>() && use_fixed(h, L.fop, 1, nc);
+}
+
 // One level operation in precision T with right-hand side of precision TB.
 template <typename T, typename TB>
 void lev_op(hz_handle* h, Hierarchy& H, int l, int mode, const cplx<T>* x, const cplx<TB>* b, cplx<T>* y,
@@ -774,10 +781,8 @@ void lev_op(hz_handle* h, Hierarchy& H, int l, int mode, const cplx<T>* x, const
   Level& L = *H.lv[l];
   const double w = h->opt.relax_param;
   if (L.fine) {
-    // FGMRES's FP64 cycle on large blocks (the finest level: a re-discretised one has its own
-    // diagonal); BiCGSTAB keeps the native steps' bits
     if constexpr (std::is_same<T, double>::value && std::is_same<TB, double>::value)
-      if (h->opt.krylov == HZ_KRYLOV_FGMRES && L.fd64 == h->diagSH.as<double2>() && use_fixed(h, L.fop, 1, nc)) {
+      if (lev_fixed<T, TB>(h, L, nc)) {
         launch_fine_fixed<double>(h->ctx, mode, L.fop, fine_diag<T>(L), fixed_diag(h, 1), x, b, y, L.ld, cols, nc,
                                   fine_dinv<T>(L), w);
         return;
@@ -1278,8 +1283,12 @@ void autotune(hz_handle* h, Hierarchy& H, int nrhs) {
   };
   Level& L0 = *H.lv[0];
   if (H.lv.size() > 1) {
-    // level 0 has two work blocks of its own; the residual goes to the Z workspace
-    pick(c.tune_fine, L0, L0.t.as<cplx<T>>(), L0.r.as<cplx<T>>(), reinterpret_cast<cplx<T>*>(h->Z.p), 0);
+    // level 0 has two work blocks of its own; the residual goes to the Z workspace.  A block that
+    // takes the integer pipe there has nothing to tune: fewer columns later take the default rule
+    if (lev_fixed<T, T>(h, L0, nrhs))
+      c.tune_fine = 0;
+    else
+      pick(c.tune_fine, L0, L0.t.as<cplx<T>>(), L0.r.as<cplx<T>>(), reinterpret_cast<cplx<T>*>(h->Z.p), 0);
     if (H.lv.size() > 2 && !H.lv[1]->fine) {
       Level& L1 = *H.lv[1];
       pick(c.tune_rap, L1, L1.x.as<cplx<T>>(), L1.b.as<cplx<T>>(), L1.r.as<cplx<T>>(), 1);

@@ -760,8 +760,16 @@ template <typename T> const cplx<T>* lev_dinv(Level& L);
 template <> const double2* lev_dinv<double>(Level& L) { return L.dinv64.as<double2>(); }
 template <> const float2* lev_dinv<float>(Level& L) { return L.dinv32.as<float2>(); }
 
-FixedDiag fixed_diag(const hz_handle* h, int shifted) {
-  return FixedDiag{h->fixrefs.as<FixedRefs>() + shifted, (shifted ? h->diagSHfix : h->diagHfix).as<int4>()};
+// H's or SH's words, made at their first use: 16 bytes per node that handles of small blocks, and SH
+// in the mixed form, never need.  (A graph's first application runs eagerly, so none is captured.)
+FixedDiag fixed_diag(hz_handle* h, int shifted) {
+  DBuf& d = shifted ? h->diagSHfix : h->diagHfix;
+  FixedRefs* refs = h->fixrefs.as<FixedRefs>() + shifted;
+  if (!d.p) {
+    d.alloc((size_t)h->g0.N * 16);
+    launch_diag_fixed(h->ctx, h->fop, (shifted ? h->diagSH : h->diagH).as<double2>(), refs, d.as<int4>());
+  }
+  return FixedDiag{refs, d.as<int4>()};
 }
 bool use_fixed(const hz_handle* h, const FineOp& op, int shifted, int ncols) {
   return h->fix_fits[shifted] && fine_fixed_pays(op, ncols);
@@ -1726,8 +1734,6 @@ void init_fine(hz_handle* h) {
   h->diagSH.alloc((size_t)N * 16);
   h->dinvSH.alloc((size_t)N * 16);
   h->fixrefs.alloc(2 * sizeof(FixedRefs));
-  h->diagHfix.alloc((size_t)N * 16);
-  h->diagSHfix.alloc((size_t)N * 16);
   {
     DBuf dm, dg;
     dm.alloc((size_t)N * 8);
@@ -1738,8 +1744,6 @@ void init_fine(hz_handle* h) {
                       p.order_neumann_bc == 1 ? 1.0 : 2.0, p.neumann_on_top, p.sommerfeld, dm.as<double>(),
                       dg.as<double>(), h->diagH.as<double2>(), h->diagSH.as<double2>(), h->dinvSH.as<double2>(),
                       h->fixrefs.as<FixedRefs>());
-    launch_diag_fixed(h->ctx, h->fop, h->diagH.as<double2>(), h->fixrefs.as<FixedRefs>(), h->diagHfix.as<int4>());
-    launch_diag_fixed(h->ctx, h->fop, h->diagSH.as<double2>(), h->fixrefs.as<FixedRefs>() + 1, h->diagSHfix.as<int4>());
     FixedRefs refs[2];
     ck(cudaMemcpyAsync(refs, h->fixrefs.p, sizeof(refs), cudaMemcpyDeviceToHost, h->ctx.stream), "coefficient exponents");
     sync(h);

@@ -30,8 +30,8 @@ def native(hz, A, X):
 
 @pytest.mark.parametrize("adjoint", [False, True])
 @pytest.mark.parametrize("cells,h,zero", [((96, 90, 80), (1, 1, 0.25), False), ((96, 90, 80), (1, 0.3, 0.3), False),
-                                          ((600, 500), (1, 0.25), False), ((96, 90, 80), (1, 1, 1), True),
-                                          ((600, 500), (1, 1), True)])
+                                          ((1500, 1200), (1, 0.25), False), ((96, 90, 80), (1, 1, 1), True),
+                                          ((1500, 1200), (1, 1), True)])
 def test_no_slower_than_the_native_kernel(hz, cells, h, zero, adjoint):
     import torch
     H, n = operator(hz, cells, [0.01 * v for v in h])

@@ -21,7 +21,8 @@
 // FP64 is bound by that pipe and by its chain of grid barriers, two per kl rows.
 // Band substitution -> digits + product, event-timed per solve:
 //   FP64 columns:  289 nodes x 1:  131 -> 7 + 10 us;   2601 x 8: 573 -> 9 + 76 us
-//   FP32 columns: 2145 nodes x 16: 839 -> 10 + 43 us;  4913 x 8: 1425 -> 14 + 136 us
+//   FP32 columns: 2145 nodes x 16: 839 -> 10 + 63 us;  4913 x 8: 1425 -> 14 + 192 us
+// (with 6 digits 43 and 136 us, but then the residual is 1e-12 of the right-hand side, the LU's 1e-16)
 // and against a dense double-float product on the FP32 pipe (861 nodes x 33):
 // 45 -> 8 + 23 us.  The setup (slab elimination on the GPU) takes 10 to 140 ms
 // over those sizes, as the banded LU on the host did.

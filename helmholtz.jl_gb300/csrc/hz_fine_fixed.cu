@@ -18,11 +18,14 @@
 // range and values that are NaN or Inf.  Zeros (a brick's, a node's with its neighbours) are not
 // worked on: a sparse column has little else.  Against quad precision the product's error is
 // 5.1e-17 of its norm on noise (native 7.5e-17), 9.2e-17 on plane waves (5.4e-16) and 6.0e-17 to
-// 7.4e-17 on noise that decays or spreads over 2^6 (7.4e-17 to 7.6e-17).  At a single node it is
-// at most 3.8 u of the row's sum of magnitudes, u = 2^-53 (native 1.7 u): a node 2^-5 below its
-// brick.
+// 7.4e-17 on noise that decays or spreads over 2^6 (7.4e-17 to 7.6e-17).  At a single node, one
+// 2^-5 below its brick, up to 3.8 u of the row's sum of magnitudes was measured on these inputs,
+// u = 2^-53 (native 1.7 u).  The bound is 48 u of the row's sum of coefficients times the largest
+// value around the node (tests/test_gpu_fine_fixed.py): coefficients are rounded relative to the
+// operator's largest, so where the diagonal is far below it and the neighbours are zeros the
+// error can be more of the node's own row.
 //
-// Measured: 157 x 131 x 101 nodes, 13 columns, adjoint: 887 us native, 452; 129^3 nodes, 8 columns of
+// Measured: 157 x 131 x 101 nodes, 13 columns, adjoint: 887 us native, 434; 129^3 nodes, 8 columns of
 // FP32 537 and 355; 1025 x 513 nodes, 16 columns of FP32 176 and 114; the FP64 cycle's residual
 // and Jacobi sweep, 65 x 65 x 33 nodes, 8 columns, 48 and 34, 59 and 49.  What bounds it is
 // instructions (36 per cell converted, 1.75 cells per node in 3D; 106 per sum; 4 additions of the

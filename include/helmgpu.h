@@ -48,7 +48,7 @@ extern "C" {
 
 /* precision of the multigrid preconditioner (the outer FGMRES is always FP64) */
 #define HZ_PREC_FP64 0
-#define HZ_PREC_MIXED 1 /* complex-FP32 V-cycle, FP64 coarsest LU */
+#define HZ_PREC_MIXED 1 /* complex-FP32 cycle, FP64 coarsest solve */
 
 /* outer FGMRES arithmetic: native FP64, or FP64 emulated with pairs of FP32
  * (basis stored as hi+lo, error-free FP32 transformations; ~2^-48 relative),
@@ -169,7 +169,11 @@ int hz_column_stats(const hz_handle* h, double* relres, int32_t* iters, int32_t 
  * replacement of getHelmholtzFun's closure (src/GetHelmholtz.jl:85-95) and of
  * the sparse products H*x the reference tests take.  The apply does not work in
  * place: device X and Y that overlap are rejected with HZ_ERR_ARG.  The column
- * list the kernel reads is kept in the handle and grows only with nrhs. */
+ * list the kernel reads is kept in the handle and grows only with nrhs.
+ * Blocks of 2^17 values (n nrhs) or more are summed on the integer pipe, on meshes
+ * whose spacings are not too unequal: in norm at least as accurate as native FP64, but
+ * rounded otherwise.  So a column's last bits can depend on the width of its block, and
+ * can differ from hz_apply_noalloc's, which always takes the native steps. */
 int hz_apply(hz_handle* h, int32_t op, int32_t transpose, const double* X, double* Y, int64_t n, int32_t nrhs,
              int32_t mem);
 
@@ -218,9 +222,10 @@ int hz_reset_kernel_times(hz_handle* h);
  * persisted there.  Returns HZ_OK once tuned, HZ_NOT_CONVERGED before. */
 int hz_tune_info(const hz_handle* h, int32_t* fine_ctas, int32_t* rap_ctas);
 /* Algorithmic flops of entry idx of the launch table: the tensor-core kernels of
- * the learned correction (BF16) and the native-FP64 kernels of the outer Krylov
- * method (krylov_dots, krylov_update, update_x, outer_apply, outer_resid: the
- * complex arithmetic they do in FP64); 0 for the other, memory-bound kernels. */
+ * the learned correction (BF16) and the outer Krylov method's kernels in FP64
+ * accuracy (krylov_dots, krylov_update, update_x, outer_apply, outer_resid: the
+ * complex arithmetic, on whichever pipe it runs); 0 for the other, memory-bound
+ * kernels. */
 int hz_kernel_flops(hz_handle* h, int32_t idx, double* alg_flops);
 /* Replay the Krylov iterations from CUDA graphs (1) or launch them
  * eagerly (0) from the next application on (options.cuda_graph at create time);
@@ -337,8 +342,8 @@ int hz_learned_stats(const hz_handle* h, int64_t* net_calls, int32_t* fallbacks)
  * coarse level is out of reach) from one cycle on that level followed by
  * sweeps - 1 restarted FP64 two-step
  * FGMRES corrections e += K(r - A e) preconditioned by the level's cycle (which
- * never raise the residual); on the coarsest level the cycle is the band LU and
- * its solve is the target.  In 3D the grid is nx x ny x nz and plain_err
+ * never raise the residual); on the coarsest level the cycle is the direct solve,
+ * whose result is the target.  In 3D the grid is nx x ny x nz and plain_err
  * compares one cycle on that level (what the network stands for) with the target.
  * x_out [max_pairs][N][4] and t_out [max_pairs][N][2] are DEVICE FP32 arrays in
  * the layout above; plain_err (host, may be NULL) gets ||e1 - e|| / ||e|| of one
